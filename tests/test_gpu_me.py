@@ -292,3 +292,48 @@ def test_generic_pus_large_range(gpu, olib):
         assert stats[1] == len(sel)
         exp = _oracle(olib, cur, [ref0, ref1], sel, prm, threads=os.cpu_count() or 1)
         _assert_same(got, exp, sel)
+
+
+@pytest.mark.parametrize("R,w,h,spread,flat", [(64, 200, 136, 10, False), (16, 136, 200, 2, False), (7, 160, 96, 40, False),
+                                                (1, 72, 72, 6, False), (128, 136, 136, 30, False), (24, 192, 128, 3, True)])
+def test_own_centre_partitions(gpu, olib, R, w, h, spread, flat):
+    """PUs with their own predictors: partitions of one CU searched together
+    (predictors `spread` quarter-pels apart around a few motions, so that some
+    fall into one cluster and some stay alone), PUs off the CU grid, limits cut
+    to a few displacements or none, against the oracle.  `flat`: constant
+    areas, where no bound excludes anything and every tie is decided by the
+    visit order."""
+    import xavs2_gb300 as xg
+    rng = np.random.default_rng(R * 7 + w)
+    cur, ref0 = _frames(rng, w, h)
+    _, ref1 = _frames(rng, w, h, shift=(-6, 9))
+    if flat:
+        cur[:, :w // 2] = 90
+        ref0[:, :w // 2 + 20] = 90
+        ref1[:h // 2] = 93
+    pus = xg.frame_pus(w, h, 2)
+    motion = np.array([(0, 0), (37, -21), (-90, 14), (5, 60)])
+    pick = motion[((pus["x"] // 32) * 3 + (pus["y"] // 32)) % 4]
+    pus["mvp_x"] = pick[:, 0] + rng.integers(-spread, spread + 1, len(pus))
+    pus["mvp_y"] = pick[:, 1] + rng.integers(-spread, spread + 1, len(pus))
+    n = 120                                      # off the CU grid, any shape
+    off = np.zeros(n, xg.PU_DTYPE)
+    off["part"] = rng.integers(0, 25, n)
+    off["ref"] = rng.integers(0, 2, n)
+    off["x"] = (rng.random(n) * (w - np.array(xg.PU_W)[off["part"]] + 1)).astype(int)
+    off["y"] = (rng.random(n) * (h - np.array(xg.PU_H)[off["part"]] + 1)).astype(int)
+    off["mvp_x"], off["mvp_y"] = rng.integers(-70, 71, n), rng.integers(-70, 71, n)
+    off = xg.set_limits(off, w, h)
+    keep = 1.0 if R <= 24 else 0.25 if R <= 64 else 0.08
+    pus = pus[rng.random(len(pus)) < keep]
+    tight = rng.random(len(pus)) < 0.1           # limits of a few displacements around a point
+    cx, cy = rng.integers(-20, 21, len(pus)), rng.integers(-20, 21, len(pus))
+    for lo, hi, c in (("min_x", "max_x", cx), ("min_y", "max_y", cy)):
+        a, b = pus[lo].copy(), pus[hi].copy()
+        pus[lo] = np.where(tight, np.clip(c - 3, a, b), a)
+        pus[hi] = np.where(tight, np.clip(c + 2, a, b), b)
+    allp = np.concatenate([pus, off, pus[:40]])
+    prm = xg.MeParams(R, oracle.lambda_factor(30), 1, 0, 0, 0)
+    got, stats = _run(cur, [ref0, ref1], allp, prm)
+    assert stats[1] > 64
+    _assert_same(got, _oracle(olib, cur, [ref0, ref1], allp, prm), allp)

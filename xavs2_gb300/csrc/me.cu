@@ -14,8 +14,10 @@
 // search parts of a window in any order and merge with atomicMin.
 //
 // Kernels: me_init_kernel (candidates), fs_ctu_kernel (shared-window search
-// of all PUs of a 64x64 CTU; fs_ctu.cuh), fs_generic_kernel (one PU per CTA)
-// and refine_kernel.
+// of all PUs of a 64x64 CTU; fs_ctu.cuh), fs_cu_kernel (partitions of one CU
+// with centres close together; fs_cu.cuh), fs_bounded_kernel (one PU per CTA,
+// displacements excluded by a bound; fs_pu.cuh), fs_generic_kernel (one PU per
+// CTA, every displacement) and refine_kernel.
 #include "xavs2gpu_common.cuh"
 
 #include <cudaTypedefs.h>
@@ -63,9 +65,22 @@ struct SessView {
     const uint8_t *pool;
     size_t plane_bytes;
     unsigned *wait_flag;            // set by a kernel that gave up a bounded wait
+    // 4x4 block means of the reference planes (nrefs buffers plane_bytes
+    // apart), written before the per-PU search of each run, or null
+    uint8_t *means;
+    int nrefs;
 };
 constexpr int kSessShift = 24;
 constexpr uint32_t kIdxMask = (1u << kSessShift) - 1;
+
+// 4 bytes at any address, from the aligned words holding them (planes have
+// room behind their last row for the second one)
+__device__ __forceinline__ uint32_t ld4_any(const uint8_t *q)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(q);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    return __funnelshift_r(__ldg(w), __ldg(w + 1), 8 * (int)(a & 3));
+}
 
 __device__ __forceinline__ int sad_block_lane(const uint8_t *a, int sa, const uint8_t *b, int sb, int w, int h, int lane)
 {
@@ -73,6 +88,19 @@ __device__ __forceinline__ int sad_block_lane(const uint8_t *a, int sa, const ui
     for (int i = lane; i < w * h; i += 32) {
         int y = i / w, x = i - y * w;
         s += iabs_d((int)a[y * sa + x] - (int)b[y * sb + x]);
+    }
+    return s;
+}
+
+// the same four pixels per step (w a multiple of 4)
+__device__ __forceinline__ uint32_t sad_block_words(const uint8_t *a, const uint8_t *b, int stride, int w, int h, int lane)
+{
+    const int wq = w >> 2, inv = (65536 + wq - 1) / wq;   // k / wq = k * inv >> 16 for k < 1024
+    uint32_t s = 0;
+    for (int k = lane; k < wq * h; k += 32) {
+        const int y = (k * inv) >> 16;
+        const ptrdiff_t o = (ptrdiff_t)y * stride + 4 * (k - y * wq);
+        s = sad4_acc(ld4_any(a + o), ld4_any(b + o), s);
     }
     return s;
 }
@@ -116,7 +144,7 @@ __device__ __forceinline__ void init_one(int i, int lane, const xavs2gpu_pu_t *_
         int mx = st.cand[c][0], my = st.cand[c][1];
         if (!in_box(p, mx, my)) continue;
         const uint8_t *r = ref + (ptrdiff_t)(p.y + my) * g.stride + p.x + mx;
-        int cost = warp_sum_i(sad_block_lane(o, g.stride, r, g.stride, w, h, lane)) +
+        int cost = (int)__reduce_add_sync(0xffffffffu, sad_block_words(o, r, g.stride, w, h, lane)) +
                    mv_cost_hd(lambda, mx * 4, my * 4, p.mvp_x, p.mvp_y);
         unsigned long long k = ((unsigned long long)(unsigned)cost << 32) | (unsigned)c;
         if (k < best) best = k;
@@ -328,6 +356,12 @@ __device__ __forceinline__ void fs_pu_search(const xavs2gpu_pu_t &p, const PuSta
     }
 }
 
+}  // namespace xg
+
+#include "fs_pu.cuh"
+
+namespace xg {
+
 template <bool WIDE>
 __global__ void __launch_bounds__(kPuThreads) fs_generic_kernel(const uint32_t *__restrict__ list, int n,
                                                                 const SessView *__restrict__ views, int R, int lambda)
@@ -365,6 +399,39 @@ static int fs_generic_launch(const uint32_t *list, int n, const SessView *views,
     count_launch();
     XG_CUDA(cudaGetLastError());
     return XAVS2GPU_OK;
+}
+
+}  // namespace xg
+
+#include "fs_cu.cuh"
+
+namespace xg {
+
+// A list of per-PU searches: n_large and n_small PUs of sessions with a means
+// buffer (bounded search), then n_plain others.
+// With CUs, the list holds what is not a partition of one of them; theirs are
+// grouped on the device (at most cap_large / cap_small of them end up alone).
+struct PerPuList {
+    const uint32_t *list = nullptr;
+    int n_large = 0, n_small = 0, n_plain = 0;
+    const CuRec *cus = nullptr;
+    int n_cus = 0, cap_large = 0, cap_small = 0;
+    CuQueues q{};
+};
+static int per_pu_launch(const PerPuList &l, const SessView *views, int R, int lambda, cudaStream_t st)
+{
+    int rc = XAVS2GPU_OK;
+    if (l.n_cus) {
+        rc = cu_search_launch(l.q, l.cus, l.n_cus, views, R, lambda, st);
+        if (rc == XAVS2GPU_OK)
+            rc = prune_launch_one<64>(l.q.large, l.cap_large, l.q.count + 4, views, R, lambda, st);
+        if (rc == XAVS2GPU_OK)
+            rc = prune_launch_one<kSmallDim>(l.q.small, l.cap_small, l.q.count + 5, views, R, lambda, st);
+    }
+    if (rc == XAVS2GPU_OK) rc = prune_launch(l.list, l.n_large, l.n_small, views, R, lambda, st);
+    if (rc == XAVS2GPU_OK && l.n_plain)
+        rc = fs_generic_launch(l.list + l.n_large + l.n_small, l.n_plain, views, R, lambda, st);
+    return rc;
 }
 
 // ---- 3. sub-pel refinement ------------------------------------------------------------
@@ -1303,7 +1370,7 @@ struct MeSessionImpl {
     unsigned long long *d_keys = nullptr;
     PuState *d_state = nullptr;
     int *d_generic = nullptr;
-    int n_generic = 0;
+    int n_generic = 0, n_generic_large = 0;   // those with a side above 16 come first
     CtuPlan plan;
     int plan_R = -1;               // search range the plan was built for (-1: stale)
     bool plan_ctu = true;          // whether the plan could use the CTU search
@@ -1324,6 +1391,13 @@ struct MeSessionImpl {
     cudaStream_t own_st = nullptr;   // the stream the session created
     SessView h_view{};
     SessView *d_view = nullptr;      // this session as the kernels see it
+    uint8_t *d_means = nullptr;      // 4x4 block means of the references (per-PU search), made with the plan
+    // CUs whose partitions have their own centres, the queues of their
+    // search, and the per-PU list of the rest (all in d_cu)
+    uint8_t *d_cu = nullptr;
+    size_t cap_cu = 0;
+    bool cu_stale = true;            // the per-PU list changed since they were made
+    PerPuList cu_list;
     std::vector<uint32_t> h_generic, h_small, h_large;
     // CU-grouped refinement: the groups, their members, and the thread /
     // warp lists of the searches no group covers
@@ -1427,6 +1501,8 @@ static void refresh_view(MeSessionImpl &m)
     v.pool = m.d_planes;
     v.plane_bytes = m.plane_bytes;
     v.wait_flag = wait_flag_word();
+    v.means = m.d_means;
+    v.nrefs = m.nrefs;
     m.h_view = v;
     XG_CUDA(cudaMemcpyAsync(m.d_view, &m.h_view, sizeof(SessView), cudaMemcpyHostToDevice, m.st));
 }
@@ -1516,6 +1592,7 @@ extern "C" void xavs2gpu_me_destroy(xavs2gpu_me_session_t *s)
     ctu_plan_free(m.plan);
     cudaFree(m.d_planes); cudaFree(m.d_plane_ptrs); cudaFree(m.d_ref0);
     if (m.d_tmap) cudaFree(m.d_tmap);
+    cudaFree(m.d_means); cudaFree(m.d_cu);
     cudaFreeHost(m.h_stage); cudaFree(m.d_upload);
     cudaFree(m.d_pus); cudaFree(m.d_res); cudaFreeHost(m.h_res); cudaFree(m.d_keys);
     cudaFree(m.d_state); cudaFree(m.d_generic); 
@@ -1614,6 +1691,7 @@ extern "C" int xavs2gpu_me_set_pus(xavs2gpu_me_session_t *s, const xavs2gpu_pu_t
     }
     m.n = n;
     m.h_pus.assign(pus, pus + n);
+    m.cu_stale = true;
     XG_CUDA(cudaStreamSynchronize(m.st));
     if (n) XG_CUDA(cudaMemcpyAsync(m.d_pus, pus, sizeof(xavs2gpu_pu_t) * n, cudaMemcpyHostToDevice, m.st));
     refresh_view(m);
@@ -1713,7 +1791,17 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     std::vector<int> generic;
     ctu_plan_build(m.plan, m.h_pus, m.W, m.H, m.nrefs, R, ctu, generic, m.st);
     m.n_generic = (int)generic.size();
+    // largest first: by area the PUs with a side above 16, then the others
+    auto side = [&](int i) { return std::max(h_pu_w[m.h_pus[i].part], h_pu_h[m.h_pus[i].part]); };
+    auto pixels = [&](int i) { return h_pu_w[m.h_pus[i].part] * h_pu_h[m.h_pus[i].part]; };
+    const auto small_from = std::stable_partition(generic.begin(), generic.end(),
+                                                  [&](int i) { return side(i) > kSmallDim; });
+    m.n_generic_large = (int)(small_from - generic.begin());
+    auto larger = [&](int a, int b) { return pixels(a) > pixels(b); };
+    std::stable_sort(generic.begin(), small_from, larger);
+    std::stable_sort(small_from, generic.end(), larger);
     m.n_ctu_pus = m.n - m.n_generic;
+    m.cu_stale = m.cu_stale || !std::equal(generic.begin(), generic.end(), m.h_generic.begin(), m.h_generic.end());
     m.h_generic.assign(generic.begin(), generic.end());
     if (m.n_generic)
         XG_CUDA(cudaMemcpyAsync(m.d_generic, generic.data(), sizeof(int) * m.n_generic, cudaMemcpyHostToDevice, m.st));
@@ -1764,6 +1852,139 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     m.plan_ctu = ctu;
 }
 
+// Per-PU searches from which a run computes the references' block means (a
+// launch of 3-7 us a plane) and groups CUs (a launch and up to six more for
+// the queues): below it the plain search of that many PUs is shorter than the
+// launches (64 PUs of 16x16 at R = 64 take 8 us on 152 SMs).
+constexpr int kMeansMinPus = 64;
+
+// slot of a PU among the partitions of its CU (side 1 << lg, corner cx, cy),
+// -1 when it is none of them
+static int cu_slot(const xavs2gpu_pu_t &p, int &lg, int &cx, int &cy)
+{
+    const int w = h_pu_w[p.part], h = h_pu_h[p.part], S = std::max(8, std::max(w, h));
+    lg = S == 8 ? 3 : S == 16 ? 4 : S == 32 ? 5 : S == 64 ? 6 : 0;
+    if (!lg) return -1;
+    cx = p.x & ~(S - 1);
+    cy = p.y & ~(S - 1);
+    for (int m = 0; m < (S == 8 ? 9 : 13); m++) {
+        SlotGeom g;
+        if (S == 8) {
+            g = slot_geom(m);   // the CTU's first 8x8 CU
+            g.ox += cx;
+            g.oy += cy;
+        } else {
+            g = cu_mode_geom(S, cx, cy, m);
+        }
+        if (g.part == p.part && g.ox == p.x && g.oy == p.y) return m;
+    }
+    return -1;
+}
+
+// The CU records of the per-PU list and the device memory of their search.
+// Without the memory for it every PU keeps to the per-PU search.
+static void ensure_cu_search(MeSessionImpl &m)
+{
+    if (!m.cu_stale) return;
+    m.cu_stale = false;
+    m.cu_list = PerPuList{};
+    const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
+    m.cu_list.list = gen;
+    m.cu_list.n_large = m.n_generic_large;
+    m.cu_list.n_small = m.n_generic - m.n_generic_large;
+    if (!m.d_means || m.n_generic < kMeansMinPus) return;
+    std::vector<CuRec> recs;
+    std::vector<uint32_t> rest;
+    std::vector<int> at[4];          // record of each CU position, per size
+    int n_rec[4] = {0, 0, 0, 0}, rest_large = 0, cap_large = 0, cap_small = 0;
+    for (int k = 0; k < 4; k++)
+        at[k].assign((size_t)m.nrefs * ((m.W >> (3 + k)) + 1) * ((m.H >> (3 + k)) + 1), -1);
+    for (int q = 0; q < m.n_generic; q++) {
+        const int i = (int)m.h_generic[q];
+        const xavs2gpu_pu_t &p = m.h_pus[i];
+        int lg = 0, cx = 0, cy = 0;
+        const int slot = cu_slot(p, lg, cx, cy);
+        bool in = slot >= 0;
+        if (in) {
+            const int k = lg - 3, cols = (m.W >> lg) + 1, rows = (m.H >> lg) + 1;
+            int &r = at[k][((size_t)p.ref * rows + (cy >> lg)) * cols + (cx >> lg)];
+            if (r < 0) {
+                r = (int)recs.size();
+                CuRec c{};
+                c.x = (int16_t)cx;
+                c.y = (int16_t)cy;
+                c.lg = (uint8_t)lg;
+                c.ref = p.ref;
+                for (int &u : c.pu) u = -1;
+                recs.push_back(c);
+                n_rec[k]++;
+            }
+            int32_t &u = recs[r].pu[slot];
+            in = u < 0;              // a second PU of the same partition searches alone
+            if (in) {
+                u = i;
+                (q < m.n_generic_large ? cap_large : cap_small)++;
+            }
+        }
+        if (!in) {
+            rest.push_back((uint32_t)i);
+            rest_large += q < m.n_generic_large ? 1 : 0;
+        }
+    }
+    if (recs.empty()) return;
+    // records | counters | clusters per size (at least two members each) | lone PUs | rest
+    size_t need = 0, o_work[4];
+    auto take = [&](size_t bytes) { const size_t o = need; need += align_up(bytes); return o; };
+    const size_t o_rec = take(sizeof(CuRec) * recs.size()), o_cnt = take(sizeof(int) * kCuCounters);
+    for (int k = 0; k < 4; k++) o_work[k] = take(sizeof(CuWork) * (kCuMembers / 2) * n_rec[k] + 1);
+    const size_t o_large = take(sizeof(uint32_t) * cap_large + 1), o_small = take(sizeof(uint32_t) * cap_small + 1);
+    const size_t o_rest = take(sizeof(uint32_t) * rest.size() + 1);
+    if (need > m.cap_cu) {
+        cudaFree(m.d_cu);
+        m.cap_cu = 0;
+        if (cudaMalloc((void **)&m.d_cu, need) != cudaSuccess) {
+            cudaGetLastError();
+            m.d_cu = nullptr;
+            return;
+        }
+        m.cap_cu = need;
+    }
+    XG_CUDA(cudaMemcpyAsync(m.d_cu + o_rec, recs.data(), sizeof(CuRec) * recs.size(), cudaMemcpyHostToDevice, m.st));
+    if (!rest.empty())
+        XG_CUDA(cudaMemcpyAsync(m.d_cu + o_rest, rest.data(), sizeof(uint32_t) * rest.size(), cudaMemcpyHostToDevice,
+                                m.st));
+    XG_CUDA(cudaStreamSynchronize(m.st));
+    PerPuList &l = m.cu_list;
+    l.list = reinterpret_cast<const uint32_t *>(m.d_cu + o_rest);
+    l.n_large = rest_large;
+    l.n_small = (int)rest.size() - rest_large;
+    l.cus = reinterpret_cast<const CuRec *>(m.d_cu + o_rec);
+    l.n_cus = (int)recs.size();
+    l.cap_large = cap_large;
+    l.cap_small = cap_small;
+    l.q.count = reinterpret_cast<int *>(m.d_cu + o_cnt);
+    for (int k = 0; k < 4; k++) l.q.work[k] = reinterpret_cast<CuWork *>(m.d_cu + o_work[k]);
+    l.q.large = reinterpret_cast<uint32_t *>(m.d_cu + o_large);
+    l.q.small = reinterpret_cast<uint32_t *>(m.d_cu + o_small);
+}
+
+// The session's means buffer, on the first plan that has use for it (without
+// the memory for it the per-PU search runs unbounded, with the same results),
+// and the CU search of the plan's per-PU list.
+static void ensure_per_pu(MeSessionImpl &m)
+{
+    if (m.n_generic < kMeansMinPus) return;
+    if (!m.d_means) {
+        if (cudaMalloc((void **)&m.d_means, m.plane_bytes * m.nrefs + 256) != cudaSuccess) {
+            cudaGetLastError();
+            m.d_means = nullptr;
+            return;
+        }
+        refresh_view(m);
+    }
+    ensure_cu_search(m);
+}
+
 extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm)
 {
     if (!s || !prm || prm->search_range < 1 || prm->search_range > 128 || prm->fractional_me < 0 ||
@@ -1776,18 +1997,23 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     XG_CUDA(cudaSetDevice(m.device));
     const int R = prm->search_range, lam = prm->lambda_factor;
     ensure_plan(m, R, lam);
+    ensure_per_pu(m);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[0], m.st));
     XG_CUDA(cudaMemsetAsync(m.d_keys, 0xff, sizeof(unsigned long long) * m.n, m.st));
     const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
+    PerPuList per_pu{gen, 0, 0, m.n_generic};
+    const bool bounded = m.n_generic >= kMeansMinPus && m.d_means && prune_ok(lam);
+    if (bounded) per_pu = m.cu_list;
     if (m.n_generic) {
         me_init_list_kernel<<<(m.n_generic * 32 + 127) / 128, 128, 0, m.st>>>(gen, m.n_generic, m.d_view, lam);
         count_launch();
+        if (bounded) mean_planes_run(m.d_view, 1, m.nrefs, m.st);
     }
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[1], m.st));
     CtuSide *gside = nullptr;
     const cudaStream_t gst = search_fork(m.st, !m.profiling && m.n_generic && m.plan.n_jobs, gside);
     if (gside && m.n_generic) {
-        const int rc = fs_generic_launch(gen, m.n_generic, m.d_view, R, lam, gst);
+        const int rc = per_pu_launch(per_pu, m.d_view, R, lam, gst);
         if (rc != XAVS2GPU_OK) {
             refine_join(m.st, gside);
             return rc;
@@ -1796,7 +2022,7 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     ctu_jobs_run(m.plan.d_jobs, m.plan.n_jobs, m.plan.n_border, m.d_view, *prm, m.st);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[2], m.st));
     if (!gside && m.n_generic) {
-        const int rc = fs_generic_launch(gen, m.n_generic, m.d_view, R, lam, m.st);
+        const int rc = per_pu_launch(per_pu, m.d_view, R, lam, m.st);
         if (rc != XAVS2GPU_OK) return rc;
     }
     refine_join(m.st, gside);
@@ -1926,6 +2152,7 @@ extern "C" int xavs2gpu_me_prepare(xavs2gpu_me_session_t *s, const xavs2gpu_me_p
     }
     XG_CUDA(cudaSetDevice(s->impl.device));
     ensure_plan(s->impl, prm->search_range, prm->lambda_factor);
+    ensure_per_pu(s->impl);
     ctu_prime(prm->search_range);   // nothing created inside a capture that follows
     return XAVS2GPU_OK;
 }
@@ -2055,7 +2282,8 @@ struct BatchBuf {
     uint32_t *d_lists = nullptr;    // generic | small | large | group members
     SessView *d_views = nullptr;
     RefineGroup *d_groups = nullptr;
-    size_t cap_jobs = 0, cap_lists = 0, cap_views = 0, cap_groups = 0;
+    uint8_t *d_means = nullptr;     // block means of the sessions with per-PU searches
+    size_t cap_jobs = 0, cap_lists = 0, cap_views = 0, cap_groups = 0, cap_means = 0;
     uint8_t *h_stage = nullptr;     // pinned: jobs | lists | views (uploads without a stream wait)
     size_t cap_stage = 0;
     cudaEvent_t done = nullptr;
@@ -2090,7 +2318,8 @@ extern "C" void xavs2gpu_me_batch_destroy(xavs2gpu_me_batch_t *b)
     for (auto &x : b->buf) {
         if (x.used) cudaEventSynchronize(x.done);
         cudaEventDestroy(x.done);
-        cudaFree(x.d_jobs); cudaFree(x.d_lists); cudaFree(x.d_views); cudaFree(x.d_groups); cudaFreeHost(x.h_stage);
+        cudaFree(x.d_jobs); cudaFree(x.d_lists); cudaFree(x.d_views); cudaFree(x.d_groups);
+        cudaFree(x.d_means); cudaFreeHost(x.h_stage);
     }
     delete b;
 }
@@ -2105,6 +2334,24 @@ static void grow(T *&p, size_t &cap, size_t need, cudaStream_t st)
     if (p) XG_CUDA(cudaFreeAsync(p, st));
     cap = need + need / 2 + 64;
     XG_CUDA(cudaMallocAsync((void **)&p, sizeof(T) * cap, st));
+}
+
+// The same for a buffer the launch can do without: false (and no buffer)
+// when the memory is not there.
+template <typename T>
+static bool grow_if_room(T *&p, size_t &cap, size_t need, cudaStream_t st)
+{
+    if (need <= cap) return need != 0;
+    if (p) XG_CUDA(cudaFreeAsync(p, st));
+    p = nullptr;
+    cap = 0;
+    if (cudaMallocAsync((void **)&p, sizeof(T) * need, st) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        return false;
+    }
+    cap = need;
+    return true;
 }
 
 extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session_t *const *sessions, int n,
@@ -2122,7 +2369,9 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     // pass 1: plans and sizes
     const bool grouped = !prm->enable_pmvr && use_groups();
     size_t nj = 0, ng = 0, ns = 0, nl = 0, nm = 0, nheavy = 0, ngr = 0;
-    int nborder = 0;
+    size_t nmeans = 0, ngl = 0, ngs = 0;   // means bytes, per-PU searches of bounded sessions
+    auto bounded = [&](const MeSessionImpl &m) { return prune_ok(lam) && m.n_generic >= kMeansMinPus; };
+    int nborder = 0, max_refs = 0;
     int block = 128;
     for (int k = 0; k < n; k++) {
         MeSessionImpl &m = sessions[k]->impl;
@@ -2135,6 +2384,12 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         nj += m.plan.h_jobs.size();
         nborder += m.plan.n_border;
         ng += m.h_generic.size();
+        if (bounded(m)) {
+            nmeans += m.plane_bytes * m.nrefs + 256;
+            max_refs = std::max(max_refs, m.nrefs);
+            ngl += m.n_generic_large;
+            ngs += m.n_generic - m.n_generic_large;
+        }
         ns += g ? m.h_small_g.size() : m.h_small.size();
         nl += g ? m.h_large_g.size() : m.h_large.size();
         if (g) {
@@ -2152,6 +2407,8 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     grow(bb.d_lists, bb.cap_lists, nlist, st);
     grow(bb.d_views, bb.cap_views, (size_t)n, st);
     grow(bb.d_groups, bb.cap_groups, ngr, st);
+    if (!grow_if_room(bb.d_means, bb.cap_means, nmeans, st)) nmeans = ngl = ngs = 0;
+    size_t means_at = 0;
     const size_t bj = sizeof(CtuJob) * nj, bl = sizeof(uint32_t) * nlist;
     const size_t bv = sizeof(SessView) * n, bg = sizeof(RefineGroup) * ngr;
     const size_t oj = 0, ol = align_up(bj), ov = ol + align_up(bl), og = ov + align_up(bv), need = og + align_up(bg);
@@ -2164,27 +2421,38 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     // tagged with their session's index in this launch; groups of 32x32 and
     // 64x64 CUs first (longest work first)
     CtuJob *J = reinterpret_cast<CtuJob *>(bb.h_stage + oj);
-    uint32_t *Lg = reinterpret_cast<uint32_t *>(bb.h_stage + ol), *Ls = Lg + ng, *Ll = Ls + ns, *Lm = Ll + nl;
+    uint32_t *Lgl = reinterpret_cast<uint32_t *>(bb.h_stage + ol), *Lgs = Lgl + ngl, *Lgp = Lgs + ngs;
+    uint32_t *Ls = Lgl + ng, *Ll = Ls + ns, *Lm = Ll + nl;
     SessView *V = reinterpret_cast<SessView *>(bb.h_stage + ov);
     RefineGroup *Gh = reinterpret_cast<RefineGroup *>(bb.h_stage + og), *Gl = Gh + nheavy;
     uint32_t mbase = 0;
-    auto put = [](uint32_t *&dst, const std::vector<uint32_t> &src, uint32_t tag) {
-        const uint32_t *p = src.data();
-        const size_t c = src.size();
+    auto put_n = [](uint32_t *&dst, const uint32_t *p, size_t c, uint32_t tag) {
         for (size_t i = 0; i < c; i++) dst[i] = tag | p[i];
         dst += c;
+    };
+    auto put = [&](uint32_t *&dst, const std::vector<uint32_t> &src, uint32_t tag) {
+        put_n(dst, src.data(), src.size(), tag);
     };
     for (int k = 0; k < n; k++) {
         MeSessionImpl &m = sessions[k]->impl;
         const bool g = grouped && m.cu_groups;
         const uint32_t tag = (uint32_t)k << kSessShift;
         V[k] = m.h_view;
+        V[k].means = nullptr;
+        const uint32_t *gen = m.h_generic.data();
+        if (nmeans && bounded(m)) {
+            V[k].means = bb.d_means + means_at;
+            means_at += m.plane_bytes * m.nrefs + 256;
+            put_n(Lgl, gen, m.n_generic_large, tag);
+            put_n(Lgs, gen + m.n_generic_large, m.n_generic - m.n_generic_large, tag);
+        } else {
+            put_n(Lgp, gen, m.n_generic, tag);
+        }
         for (const CtuJob &j0 : m.plan.h_jobs) {
             *J = j0;
             J->sess = (uint8_t)k;
             J++;
         }
-        put(Lg, m.h_generic, tag);
         put(Ls, g ? m.h_small_g : m.h_small, tag);
         put(Ll, g ? m.h_large_g : m.h_large, tag);
         if (g) {
@@ -2208,11 +2476,13 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     if (ng) {
         me_init_list_kernel<<<(unsigned)((ng * 32 + 127) / 128), 128, 0, st>>>(d_gen, (int)ng, bb.d_views, lam);
         count_launch();
+        if (nmeans) mean_planes_run(bb.d_views, n, max_refs, st);
     }
+    const PerPuList per_pu{d_gen, (int)ngl, (int)ngs, (int)(ng - ngl - ngs)};
     CtuSide *gside = nullptr;
     const cudaStream_t gst = search_fork(st, ng && nj, gside);
     if (gside) {
-        const int rc = fs_generic_launch(d_gen, (int)ng, bb.d_views, R, lam, gst);
+        const int rc = per_pu_launch(per_pu, bb.d_views, R, lam, gst);
         if (rc != XAVS2GPU_OK) {
             refine_join(st, gside);
             return rc;
@@ -2220,7 +2490,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     }
     ctu_jobs_run(bb.d_jobs, (int)nj, nborder, bb.d_views, *prm, st);
     if (!gside && ng) {
-        const int rc = fs_generic_launch(d_gen, (int)ng, bb.d_views, R, lam, st);
+        const int rc = per_pu_launch(per_pu, bb.d_views, R, lam, st);
         if (rc != XAVS2GPU_OK) return rc;
     }
     refine_join(st, gside);
@@ -2303,6 +2573,8 @@ __global__ void noalloc_prepare_kernel(const xavs2gpu_pu_t *__restrict__ in, int
         v.pool = nullptr;
         v.plane_bytes = 0;
         v.wait_flag = nullptr;
+        v.means = nullptr;   // no memory for block means: the plain per-PU search
+        v.nrefs = nrefs;
         s->view = v;
     }
     if (i >= n) return;
