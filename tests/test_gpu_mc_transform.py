@@ -357,3 +357,59 @@ def test_tq_batch_host(gpu, pinned, chunks):
         assert np.array_equal(hc.numpy().view(np.int16)[own_c], want_c)
         assert np.array_equal(hrec.numpy().view(np.int16)[own_r], want_r)
     assert (hn.numpy().view(np.int32)[::97] == -1).all()
+
+
+@pytest.mark.parametrize("n", [1, 2, 2560, 2561, 5000])
+def test_tq_batch_forms(gpu, olib, n):
+    """Batches on both sides of the direct form's limit (2560 TUs in
+    descriptor order, a CTA each; longer ones ordered by shape): every shape,
+    residuals over the whole int16 range and at its ends, all-zero blocks,
+    offsets of every alignment, invalid descriptors -- against the oracle for
+    a batch's first 250 blocks, and the repeats of those blocks further on
+    against the first."""
+    rng = np.random.default_rng(n)
+    m = min(n, 250)
+    base = np.zeros(m, np.dtype([("offset", "<i8"), ("coef_offset", "<i8"), ("part", "<i4"), ("qp", "<i4"),
+                                 ("flags", "<i4"), ("pad_", "<i4")]))
+    chunks, off, coff = [], 0, 0
+    for i in range(m):
+        p = TU_PARTS[(i + n) % len(TU_PARTS)]
+        k = PU_W[p] * PU_H[p]
+        gap = int(rng.integers(0, 9)) if i % 3 else 0
+        blk = [rng.integers(-32768, 32768, k), np.where(rng.random(k) < 0.5, -32768, 32767), np.zeros(k),
+               np.round(rng.laplace(0, 12, k)).clip(-255, 255), rng.integers(-300, 301, k)][i % 5]
+        chunks += [np.zeros(gap, np.int16), blk.astype(np.int16)]
+        off += gap
+        base[i] = (off, coff, p, int(rng.integers(0, 80)), int(rng.integers(0, 4 if p == 0 else 2)), 0)
+        off += k
+        coff += k // 4 if max(PU_W[p], PU_H[p]) == 64 else k
+    if m > 20:
+        base["part"][7], base["qp"][11] = 9, -1
+    one = np.concatenate(chunks)
+    reps = (n + m - 1) // m
+    off += 8 - off % 8 if off % 8 else 0         # the repeats keep the alignments
+    one = np.pad(one, (0, off - len(one)))
+    blocks = np.tile(base, reps)[:n]
+    rep = np.arange(n) // m
+    blocks["offset"] += rep * off
+    blocks["coef_offset"] += rep * coff
+    coef, rec, nnz = _run_tq_batch(blocks, np.tile(one, reps), off * reps, coff * reps)
+    for i, b in enumerate(base):
+        p, o, co = int(b["part"]), int(b["offset"]), int(b["coef_offset"])
+        if p not in TU_PARTS or not 0 <= b["qp"] <= 79:
+            assert nnz[i] == -1
+            continue
+        k = PU_W[p] * PU_H[p]
+        nc = k // 4 if max(PU_W[p], PU_H[p]) == 64 else k
+        blk, cf = one[o:o + k].copy(), np.zeros(k, np.int16)
+        nz = olib.xo_tq_chain(p, oracle.ptr(blk), oracle.ptr(cf), int(b["qp"]), int(b["flags"]) & 1,
+                              (int(b["flags"]) >> 1) & 1)
+        assert nnz[i] == nz, (i, p)
+        assert np.array_equal(coef[co:co + nc], cf[:nc]), (i, p)
+        assert np.array_equal(rec[o:o + k], blk), (i, p)
+        for r in range(1, reps):
+            if r * m + i >= n:
+                break
+            assert nnz[r * m + i] == nz
+            assert np.array_equal(coef[r * coff + co:r * coff + co + nc], cf[:nc]), (i, p, r)
+            assert np.array_equal(rec[r * off + o:r * off + o + k], blk), (i, p, r)

@@ -4,7 +4,8 @@
 // reference's TU reconstruction (rdo.c:1333-1370, 876-947) with the
 // transforms of transform.c:1123-1587 and the quantiser of quant.c:108-184.
 //
-// Three launches per batch:
+// Small batches take one launch (tq_direct_kernel below).  Three launches per
+// larger batch:
 //   1. count the blocks of every TU shape (invalid descriptors get nnz = -1);
 //   2. scatter the block indices into one list grouped by shape, largest
 //      shapes first, so that at any moment the warps of the persistent
@@ -717,6 +718,290 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) tq_chain_kernel(Ctx cx, cons
     }
 }
 
+// ---- small batches -------------------------------------------------------------
+// A batch of up to a few TUs per SM is bound by the latency of its longest TU
+// (a 64x64 TU is about 6,000 instructions of one warp, 20 us), not by the
+// work: ordering it by shape (three more stream operations before the first
+// TU starts) and one warp per TU only lengthen it.  tq_direct_kernel takes it
+// in descriptor order in one launch, a CTA of 4 warps per TU: the warps share
+// the TU's lines and each computes a quarter of every line's outputs (the
+// shapes whose larger side is below 32 take one warp as in the batch form).
+constexpr int kTuWarps = 4;
+
+// fwd_folded and inv_split, one warp's share of a line's outputs
+template <int N, typename Out>
+__device__ __forceinline__ void fwd_folded_part(const uint32_t (&ep)[N / 4], const uint32_t (&op)[N / 4], int part, Out out)
+{
+    const uint32_t *fe = &c_fwd.w[tab_off(N / 2)], *fo = &c_fwd.w[odd_off(N)];
+#pragma unroll 2
+    for (int k = part; k < N / 2; k += kTuWarps) {
+        out(2 * k, dot_row<N / 2>(ep, fe + k * (N / 8)));
+        out(2 * k + 1, dot_row<N / 2>(op, fo + k * (N / 8)));
+    }
+}
+template <int N, typename Out>
+__device__ __forceinline__ void inv_split_part(const uint32_t (&cp)[N / 2], int part, Out out)
+{
+    uint32_t ce[N / 4], co[N / 4];
+#pragma unroll
+    for (int m = 0; m < N / 4; m++) {
+        ce[m] = __byte_perm(cp[2 * m], cp[2 * m + 1], 0x5410);
+        co[m] = __byte_perm(cp[2 * m], cp[2 * m + 1], 0x7632);
+    }
+    const uint32_t *ie = &c_inv.w[tab_off(N / 2)], *io = &c_inv.w[odd_off(N)];
+#pragma unroll 2
+    for (int n = part; n < N / 2; n += kTuWarps) {
+        const int e = dot_row<N / 2>(ce, ie + n * (N / 8));
+        const int o = dot_row<N / 2>(co, io + n * (N / 8));
+        out(n, e + o);
+        out(N - 1 - n, e - o);
+    }
+}
+// forward transform of a line held by lane l of every warp: by the fold, or
+// in full when a warp's fold overflows 16 bits (the same sums either way)
+template <int N, typename Out>
+__device__ __forceinline__ void fwd_line_part(const uint32_t (&xp)[N / 2], int part, Out out)
+{
+    uint32_t ep[N / 4], op[N / 4];
+    bool bad = false;
+    fold_line<N>(xp, ep, op, bad);
+    if (!__any_sync(__activemask(), bad)) {
+        fwd_folded_part<N>(ep, op, part, out);
+        return;
+    }
+    const uint32_t *rows = &c_fwd.w[tab_off(N)];
+#pragma unroll 2
+    for (int k = part; k < N; k += kTuWarps) out(k, dot_row<N>(xp, rows + k * (N / 4)));
+}
+
+// One TU of a shape with a 32-sample side (or the wavelet around one) by the
+// CTA.  Shared memory: a (wavelet rows, pitch 66; or the two transposes), b
+// (the low band, pitch TW + 2; or the output's staging).
+template <int PART>
+__device__ __noinline__ void tu_cta(const Ctx &cx, int idx, int tid, uint8_t *smem, int *s_nz)
+{
+    using S = Shape<PART>;
+    constexpr int IW = S::IW, IH = S::IH, TW = S::TW, TH = S::TH, kThreads = 32 * kTuWarps;
+    constexpr int P1 = TH + 2, P2 = TW + 2, PS = TW + 2;
+    constexpr int F = S::WAV ? 1 : 0;
+    constexpr int LEVEL = (ilog2c(IW) + ilog2c(IH)) >> 1;
+    const int l = tid & 31, part = tid >> 5;
+    const xavs2gpu_tq_block_t b = cx.blocks[idx];
+    int16_t *tA = reinterpret_cast<int16_t *>(smem), *tB = reinterpret_cast<int16_t *>(smem + kRegionA);
+    const int16_t *src = cx.residual + b.offset;
+    const bool al_in = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+    if (tid == 0) *s_nz = 0;
+    uint32_t xp[TW / 2];
+    if constexpr (S::WAV) {
+        constexpr int PX = 66, PL = TW + 2;
+        if (al_in) {
+            constexpr int NV = IW * IH / 8 / kThreads;
+            uint4 v[NV];
+#pragma unroll
+            for (int k = 0; k < NV; k++) v[k] = __ldg(reinterpret_cast<const uint4 *>(src) + tid + kThreads * k);
+#pragma unroll
+            for (int k = 0; k < NV; k++) {
+                const int e = tid + kThreads * k;
+                uint32_t *d = reinterpret_cast<uint32_t *>(tA + ((e * 8) / IW) * PX + (e * 8) % IW);
+                d[0] = v[k].x; d[1] = v[k].y; d[2] = v[k].z; d[3] = v[k].w;
+            }
+        } else {
+            for (int e = tid; e < IW * IH; e += kThreads) tA[(e / IW) * PX + e % IW] = src[e];
+        }
+        __syncthreads();
+        // horizontal lifting (see tu_group): a thread per row and share of 8
+        // words, its words and the neighbours' odd samples read before any
+        // low-band word is written over the row's first half
+        constexpr int NW = IW / 2, SH = NW / 8;   // shares per row
+        constexpr int IT = (IH * SH + kThreads - 1) / kThreads;
+        uint32_t hw[IT][4];
+#pragma unroll
+        for (int it = 0; it < IT; it++) {
+            const int u = tid + kThreads * it, r = u / SH, c = 8 * (u % SH);
+            if (u < IH * SH) {
+                const uint32_t *pw = reinterpret_cast<const uint32_t *>(tA + r * PX);
+                uint32_t w[9];
+#pragma unroll
+                for (int k = 0; k < 8; k++) w[k] = pw[c + k];
+                w[8] = c + 8 < NW ? pw[c + 8] : w[7];   // p[IW] mirrors to p[IW-2]
+                int pe = (int)(int16_t)(w[0] & 0xFFFFu), prev = 0, hl = 0;
+                if (c > 0) {   // odd[c - 1]
+                    const uint32_t v = pw[c - 1];
+                    prev = (int16_t)(((int)v >> 16) - (((int)(int16_t)(v & 0xFFFFu) + pe) >> 1));
+                }
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int po = (int)w[k] >> 16, pn = (int)(int16_t)(w[k + 1] & 0xFFFFu);
+                    const int odd = (int16_t)(po - ((pe + pn) >> 1));
+                    if (c + k == 0) prev = odd;
+                    const int h = (int16_t)(pe + ((prev + odd + 2) >> 2));
+                    prev = odd;
+                    pe = pn;
+                    if (k & 1) hw[it][k >> 1] = pack16(hl, h);
+                    else hl = h;
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int it = 0; it < IT; it++) {
+            const int u = tid + kThreads * it, r = u / SH, c = 8 * (u % SH);
+            if (u < IH * SH)
+#pragma unroll
+                for (int k = 0; k < 4; k++) reinterpret_cast<uint32_t *>(tA + r * PX)[c / 2 + k] = hw[it][k];
+        }
+        __syncthreads();
+        // vertical lifting: lane j a low-band row, each warp its words
+        if (l < TH) {
+            const int j = l;
+            const int rm2 = j == 0 ? 2 : 2 * j - 2, rm1 = j == 0 ? 1 : 2 * j - 1;
+            const int rp1 = 2 * j + 1, rp2 = j == TH - 1 ? 2 * j : 2 * j + 2;
+            const uint32_t *qa = reinterpret_cast<const uint32_t *>(tA + rm2 * PX);
+            const uint32_t *qb = reinterpret_cast<const uint32_t *>(tA + rm1 * PX);
+            const uint32_t *qc = reinterpret_cast<const uint32_t *>(tA + 2 * j * PX);
+            const uint32_t *qd = reinterpret_cast<const uint32_t *>(tA + rp1 * PX);
+            const uint32_t *qe = reinterpret_cast<const uint32_t *>(tA + rp2 * PX);
+            uint32_t *ow = reinterpret_cast<uint32_t *>(tB + j * PL);
+            auto ll = [](int a, int b, int c, int d, int e) {
+                const int oa = (int16_t)(b - ((a + c) >> 1));
+                const int ob = (int16_t)(d - ((c + e) >> 1));
+                return (int16_t)((c << 1) + ((oa + ob + 1) >> 1));
+            };
+            auto lo = [](uint32_t v) { return (int)(int16_t)(v & 0xFFFFu); };
+            auto hi = [](uint32_t v) { return (int)v >> 16; };
+#pragma unroll 4
+            for (int i = part; i < TW / 2; i += kTuWarps) {
+                const uint32_t a = qa[i], bb = qb[i], c = qc[i], d = qd[i], e = qe[i];
+                ow[i] = pack16(ll(lo(a), lo(bb), lo(c), lo(d), lo(e)), ll(hi(a), hi(bb), hi(c), hi(d), hi(e)));
+            }
+        }
+        __syncthreads();
+        if (l < TH) load_pairs<TW>(tB + l * PL, xp);
+    } else {
+        if (l < TH) load_pairs_global<TW>(src + l * TW, al_in, xp);
+        __syncthreads();   // s_nz
+    }
+    // forward rows -> T1[k][j]
+    if (l < TH)
+        fwd_line_part<TW>(xp, part, [&](int k, int v) {
+            tA[k * P1 + l] = (int16_t)((v + ((1 << S::S1) >> 1)) >> S::S1);
+        });
+    __syncthreads();
+    // forward columns + quant; the dequantised levels go back into T1 once
+    // every warp has read its lines
+    const int qshift = 22 - LEVEL;
+    const int qadd = (int)(((int64_t)1 << (qshift + (b.flags & 1))) * 5 / 31);
+    const int qscale = c_q_scale[b.qp & 127];
+    const int dqshift = iq_shift_of(b.qp) + 9 + LEVEL - 16;
+    const int dqscale = c_iq_scale[b.qp & 127];
+    int nz = 0;
+    uint32_t cp[TH / 2];
+    if (l < TW) load_pairs<TH>(tA + l * P1, cp);
+    __syncthreads();
+    if (l < TW) {
+        int16_t *co = cx.coef + b.coef_offset + l;
+        fwd_line_part<TH>(cp, part, [&](int m, int s) {
+            const int y = (int)(int16_t)((s + ((1 << S::S2) >> 1)) >> S::S2);
+            const int a = (y < 0 ? -y : y) * qscale + qadd;
+            const int q = y < 0 ? -(a >> qshift) : (a >> qshift);
+            co[m * TW] = (int16_t)q;
+            nz += q != 0;
+            tA[l * P1 + m] = (int16_t)clipb((q * dqscale + (1 << (dqshift - 1))) >> dqshift, 16);
+        });
+    }
+    nz = __reduce_add_sync(0xffffffffu, nz);
+    if (l == 0 && nz) atomicAdd(s_nz, nz);
+    __syncthreads();
+    nz = *s_nz;
+    if (tid == 0) cx.nnz[idx] = nz;
+    int16_t *dst = cx.recon + b.offset;
+    const bool al_out = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+    if (nz == 0) {
+        if (al_out)
+            for (int i = tid; i < IW * IH / 8; i += kThreads) reinterpret_cast<uint4 *>(dst)[i] = make_uint4(0, 0, 0, 0);
+        else
+            for (int i = tid; i < IW * IH; i += kThreads) dst[i] = 0;
+        return;
+    }
+    // inverse columns -> T2[n][l]
+    int16_t *t2 = tA + TW * P1;
+    if (l < TW) {
+        load_pairs<TH>(tA + l * P1, cp);
+        inv_split_part<TH>(cp, part, [&](int n, int v) { t2[n * P2 + l] = (int16_t)clipb((v + 16) >> 5, 16); });
+    }
+    __syncthreads();
+    // inverse rows, staged in b
+    if (l < TH) {
+        uint32_t vp[TW / 2];
+        load_pairs<TW>(t2 + l * P2, vp);
+        constexpr int sh = 12 - F, bits = 9 + F;
+        int16_t *o = tB + l * PS;
+        inv_split_part<TW>(vp, part, [&](int x, int v) { o[x] = (int16_t)clipb((v + (1 << (sh - 1))) >> sh, bits); });
+    }
+    __syncthreads();
+    uint32_t *dw = reinterpret_cast<uint32_t *>(dst);
+    auto store = [&](int e, uint32_t v) {   // output word e
+        if (al_out) {
+            dw[e] = v;
+        } else {
+            dst[2 * e] = (int16_t)(v & 0xFFFF);
+            dst[2 * e + 1] = (int16_t)(v >> 16);
+        }
+    };
+    if constexpr (!S::WAV) {
+        for (int e = tid; e < TW * TH / 2; e += kThreads)
+            store(e, *reinterpret_cast<const uint32_t *>(tB + (e / (TW / 2)) * PS + 2 * (e % (TW / 2))));
+    } else {
+        // upsampling (see tu_group): a warp takes a run of low-band rows
+        constexpr int RW = TH / kTuWarps;
+        if (l < TW) {
+            const int i = l, in1 = i + 1 < TW ? i + 1 : i, y0 = part * RW;
+            int h0 = tB[y0 * PS + i] >> 1, h1 = tB[y0 * PS + in1] >> 1;
+#pragma unroll 2
+            for (int y = y0; y < y0 + RW; y++) {
+                const int yn = y + 1 < TH ? y + 1 : TH - 1;
+                const int n0 = tB[yn * PS + i] >> 1, n1 = tB[yn * PS + in1] >> 1;
+                const int v0 = (h0 + n0) >> 1, v1 = (h1 + n1) >> 1;
+                store(2 * y * TW + i, pack16(h0, (h0 + h1) >> 1));
+                store((2 * y + 1) * TW + i, pack16(v0, (v0 + v1) >> 1));
+                h0 = n0;
+                h1 = n1;
+            }
+        }
+    }
+}
+
+template <int RS, int MINB>
+__global__ void __launch_bounds__(32 * kTuWarps, MINB) tq_direct_kernel(Ctx cx, int n)
+{
+    __shared__ __align__(16) uint8_t smem[kRegionA + kRegionB];
+    __shared__ int s_nz;
+    const int tid = threadIdx.x, idx = blockIdx.x;
+    const xavs2gpu_tq_block_t b = cx.blocks[idx];
+    const int c = (b.qp >= 0 && b.qp <= 79) ? class_of(b.part) : -1;
+    if (c < 0) {
+        if (tid == 0) cx.nnz[idx] = -1;
+        return;
+    }
+    switch (b.part) {
+    case 4: tu_cta<4>(cx, idx, tid, smem, &s_nz); return;
+    case 23: tu_cta<23>(cx, idx, tid, smem, &s_nz); return;
+    case 24: tu_cta<24>(cx, idx, tid, smem, &s_nz); return;
+    case 3: tu_cta<3>(cx, idx, tid, smem, &s_nz); return;
+    case 19: tu_cta<19>(cx, idx, tid, smem, &s_nz); return;
+    case 20: tu_cta<20>(cx, idx, tid, smem, &s_nz); return;
+    }
+    if (tid >= 32) return;
+    const int one = tid < 32 / class_g(c) ? idx : -1;   // one TU: the first of the group's sub-warps
+    switch (b.part) {
+    case 2: tu_group<2, RS>(cx, one, tid, smem); break;
+    case 15: tu_group<15, RS>(cx, one, tid, smem); break;
+    case 16: tu_group<16, RS>(cx, one, tid, smem); break;
+    case 1: tu_group<1, RS>(cx, one, tid, smem); break;
+    default: tu_group<0, RS>(cx, one, tid, smem); break;
+    }
+}
+
 }  // namespace tqw
 
 // Region A of the non-wavelet classes: the 32x32 TU's two transposes and its
@@ -762,6 +1047,54 @@ static void tq_run(const tqw::Ctx &cx, const int *counts, const int *sorted, lon
     tqw::tq_chain_kernel<WARPS, C0, C1, RA, MINB><<<(int)grid, WARPS * 32, smem, st>>>(cx, counts, sorted);
 }
 
+// Batches up to this many TUs take the direct form.  Measured (us per batch,
+// direct / ordered): all 11 shapes 777 TUs 14.4 / 36.6, 2000 24.7 / 37.6, 3000
+// 36.3 / 37.5, 4000 47.4 / 37.6; squares 4000 28.8 / 39.7; sides up to 32 4000
+// 22.6 / 26.6.  (A warp per TU in descriptor order: 23.8 at 777, 30.9 at 3000.)
+#ifndef XG_TQ_DIRECT
+#define XG_TQ_DIRECT 2560
+#endif
+constexpr int kDirectMinB = 5;   // CTAs of 4 warps per SM: 96 registers (8 measured the same)
+
+// The two launches of the ordered form beside each other up to this many TUs:
+// the second on a side stream forked from the caller's and joined back (per
+// host thread and device; none is made during a stream capture).  Their tails
+// then overlap (us, forked / in turn: 6000 TUs of all shapes 33.8 / 43.7, 16000
+// 58 / 66, 64000 201 / 207); larger batches fill the GPU with either launch and
+// lose by sharing it (200,000 644 / 602, 10^6 squares 2.61 / 2.55 ms).
+#ifndef XG_TQ_FORK
+#define XG_TQ_FORK 65536
+#endif
+struct TqSide {
+    cudaStream_t st = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    ~TqSide()
+    {
+        if (join) cudaEventDestroy(join);
+        if (fork) cudaEventDestroy(fork);
+        if (st) cudaStreamDestroy(st);
+    }
+};
+static TqSide *tq_side(int dev, cudaStream_t stream)
+{
+    thread_local TqSide side[64];
+    TqSide &s = side[dev];
+    if (!s.st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+    }
+    return &s;
+}
+
 template <int WARPS>
 static int tq_launch_w(const xavs2gpu_tq_block_t *blocks, int n, const int16_t *residual, int16_t *coef,
                        int16_t *recon, int32_t *nnz, cudaStream_t stream)
@@ -793,9 +1126,20 @@ static int tq_launch_w(const xavs2gpu_tq_block_t *blocks, int n, const int16_t *
     tqw::Ctx cx{blocks, residual, coef, recon, nnz};
     const long long ctas_needed = ((long long)n + WARPS - 1) / WARPS;
 #if XG_TQ_SPLIT
+    TqSide *side = n <= XG_TQ_FORK ? tq_side(dev, stream) : nullptr;
+    cudaStream_t st2 = stream;
+    if (side) {
+        XG_CUDA(cudaEventRecord(side->fork, stream));
+        XG_CUDA(cudaStreamWaitEvent(side->st, side->fork, 0));
+        st2 = side->st;
+    }
     tq_run<WARPS, 0, 3, tqw::kRegionA, XG_TQ_BIG_MINB * 4 / WARPS>(cx, counts, sorted, ctas_needed, dev, stream);
     tq_run<WARPS, 3, tqw::kNumClasses, kRegionSmall, XG_TQ_SMALL_MINB * 4 / WARPS>(cx, counts, sorted, ctas_needed, dev,
-                                                                                   stream);
+                                                                                   st2);
+    if (side) {
+        XG_CUDA(cudaEventRecord(side->join, side->st));
+        XG_CUDA(cudaStreamWaitEvent(stream, side->join, 0));
+    }
     count_launch(4);
 #else
     // 16 warps per SM (128 registers)
@@ -816,6 +1160,13 @@ int tq_batch_launch(const xavs2gpu_tq_block_t *blocks, int n, const int16_t *res
         return XAVS2GPU_ERR_ARG;
     }
     if (n == 0) return XAVS2GPU_OK;
+    if (n <= XG_TQ_DIRECT) {
+        tqw::tq_direct_kernel<kRegionSmall, kDirectMinB><<<n, 32 * tqw::kTuWarps, 0, stream>>>(
+            tqw::Ctx{blocks, residual, coef, recon, nnz}, n);
+        count_launch();
+        XG_CUDA(cudaGetLastError());
+        return XAVS2GPU_OK;
+    }
     if (warps == 8) return tq_launch_w<8>(blocks, n, residual, coef, recon, nnz, stream);
     return tq_launch_w<4>(blocks, n, residual, coef, recon, nnz, stream);
 }
