@@ -47,9 +47,15 @@ __device__ void fwd_pass_d(const int8_t (*B)[32], const int16_t *in, int in_stri
     const int add = (1 << shift) >> 1;
     for (int i = threadIdx.x; i < N * lines; i += blockDim.x) {
         int k = i / lines, j = i - k * lines;
-        const int16_t *v = in + j * in_stride;
+        // four products a step: pairs of samples against the basis row's bytes
+        // (rows of an even stride, N a multiple of 4)
+        const uint32_t *v = reinterpret_cast<const uint32_t *>(in + j * in_stride);
+        const uint32_t *row = reinterpret_cast<const uint32_t *>(B[k * (32 / N)]);
         int s = 0;
-        for (int n = 0; n < N; n++) s += basis_d(B, N, k, n) * v[n];
+        for (int n = 0; n < N / 4; n++) {
+            s = __dp2a_lo((int)v[2 * n], (int)row[n], s);
+            s = __dp2a_hi((int)v[2 * n + 1], (int)row[n], s);
+        }
         out[i] = (int16_t)((s + add) >> shift);
     }
 }
@@ -165,7 +171,7 @@ __device__ __forceinline__ void sec_dirs_d(int mode, bool &vt, bool &ht)
 
 // Shared-memory workspace of one TU (largest case: 64x64 input).
 struct TuSmem {
-    int8_t basis[32][32];
+    __align__(16) int8_t basis[32][32];
     int16_t a[64 * 64];
     int16_t b[64 * 64];
     int red[32];
@@ -173,7 +179,8 @@ struct TuSmem {
 
 __device__ void load_basis(TuSmem &s)
 {
-    for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) (&s.basis[0][0])[i] = (&c_basis.v[0][0])[i];
+    for (int i = threadIdx.x; i < 32 * 32 / 4; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(&s.basis[0][0])[i] = __ldg(reinterpret_cast<const uint32_t *>(&d_basis.v[0][0]) + i);
 }
 
 // Forward transform of the block in s.a (iw x ih, stride iw).  Result:
@@ -247,7 +254,9 @@ __global__ void __launch_bounds__(256) tu_percall_kernel(int op, int part, int f
     tu_geom(part, flag, g);
     load_basis(s);
     const int n_in = op == 1 ? g.w * g.h : g.iw * g.ih;
-    for (int i = threadIdx.x; i < n_in; i += blockDim.x) s.a[i] = in[i];
+    // (host memory: as many reads in flight as there are words)
+    for (int i = threadIdx.x; i < n_in / 2; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(s.a)[i] = reinterpret_cast<const uint32_t *>(in)[i];
     __syncthreads();
     if (op == 1) {
         tu_inverse_d(s, g, flag);
@@ -292,22 +301,26 @@ __global__ void __launch_bounds__(256) quant_percall_kernel(int op, int16_t *c, 
     __shared__ int red[32];
     int nz = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        int v = c[i];
+        // c and aux are host memory: each read once
+        const int v = c[i];
+        int16_t r;
         switch (op) {
-        case 0: c[i] = quant1(v, scale, shift, add); nz += c[i] != 0; break;
-        case 1: c[i] = dequant1(v, scale, shift); break;
+        case 0: r = quant1(v, scale, shift, add); nz += r != 0; break;
+        case 1: r = dequant1(v, scale, shift); break;
         case 2: {
             int a = (iabs_d(v) * ls[i] + (1 << 18)) >> 19;
             int q = (a * scale + add) >> shift;
-            c[i] = (int16_t)(v < 0 ? -q : q);
-            nz += c[i] != 0;
+            r = (int16_t)(v < 0 ? -q : q);
+            nz += r != 0;
         } break;
-        case 3: c[i] = (int16_t)iabs_d(aux[i]); break;
-        default:
-            c[i] = (int16_t)(v > 0 ? aux[i] : -aux[i]);
-            nz += aux[i] != 0;
-            break;
+        case 3: r = (int16_t)iabs_d(aux[i]); break;
+        default: {
+            const int16_t x = aux[i];
+            r = (int16_t)(v > 0 ? x : -x);
+            nz += x != 0;
+        } break;
         }
+        c[i] = r;
     }
     nz = block_sum(nz, red);
     if (threadIdx.x == 0) result[0] = nz;
@@ -335,11 +348,11 @@ static void tu_call(int op, int part, const int16_t *src, int16_t *dst, int stri
     CallCtx &c = call_ctx(o_out + align_up((size_t)out_w * out_h * 2));
     if (op == 1) memcpy(c.h_stage + o_in, src, (size_t)in_w * in_h * 2);     // coefficients are contiguous
     else pack_rows(c.h_stage + o_in, src, (intptr_t)st * 2, in_w * 2, in_h);
-    XG_CUDA(cudaMemcpyAsync(c.d_stage + o_in, c.h_stage + o_in, (size_t)in_w * in_h * 2, cudaMemcpyHostToDevice, c.stream));
-    tu_percall_kernel<<<1, 256, sizeof(TuSmem), c.stream>>>(op, part, flag, (const int16_t *)(c.d_stage + o_in),
-                                                           (int16_t *)(c.d_stage + o_out));
+    // the kernel reads the block and writes its result once each, in the
+    // page-locked buffer itself: no copies
+    tu_percall_kernel<<<1, 256, sizeof(TuSmem), c.stream>>>(op, part, flag, (const int16_t *)(c.h_stage + o_in),
+                                                           (int16_t *)(c.h_stage + o_out));
     count_launch();
-    XG_CUDA(cudaMemcpyAsync(c.h_stage + o_out, c.d_stage + o_out, (size_t)out_w * out_h * 2, cudaMemcpyDeviceToHost, c.stream));
     XG_CUDA(cudaStreamSynchronize(c.stream));
     if (op == 1) unpack_rows(dst, (intptr_t)st * 2, c.h_stage + o_out, out_w * 2, out_h);
     else memcpy(dst, c.h_stage + o_out, (size_t)out_w * out_h * 2);
@@ -398,12 +411,10 @@ static int quant_call(int op, int16_t *coef, const int16_t *aux, const int *ls, 
     memcpy(c.h_stage + o_c, coef, (size_t)n * 2);
     if (aux) memcpy(c.h_stage + o_aux, aux, (size_t)n * 2);
     if (ls) memcpy(c.h_stage + o_ls, ls, (size_t)n * 4);
-    XG_CUDA(cudaMemcpyAsync(c.d_stage, c.h_stage, o_res, cudaMemcpyHostToDevice, c.stream));
-    quant_percall_kernel<<<1, 256, 0, c.stream>>>(op, (int16_t *)(c.d_stage + o_c), (const int16_t *)(c.d_stage + o_aux),
-                                                 (const int *)(c.d_stage + o_ls), n, scale, shift, add,
-                                                 (int *)(c.d_stage + o_res));
+    quant_percall_kernel<<<1, 256, 0, c.stream>>>(op, (int16_t *)(c.h_stage + o_c), (const int16_t *)(c.h_stage + o_aux),
+                                                 (const int *)(c.h_stage + o_ls), n, scale, shift, add,
+                                                 (int *)(c.h_stage + o_res));
     count_launch();
-    XG_CUDA(cudaMemcpyAsync(c.h_stage, c.d_stage, o_res + 4, cudaMemcpyDeviceToHost, c.stream));
     XG_CUDA(cudaStreamSynchronize(c.stream));
     memcpy(coef, c.h_stage + o_c, (size_t)n * 2);
     return *(int *)(c.h_stage + o_res);

@@ -27,7 +27,9 @@ static constexpr Basis32 make_basis()
     return b;
 }
 
-static __constant__ Basis32 c_basis = make_basis();
+// in global memory: its readers load it whole, each thread another word (the
+// constant bank serves one address per request)
+static __device__ __align__(16) const Basis32 d_basis = make_basis();
 
 // Secondary transform matrices (transform.c:140-155), fixed by the standard.
 static __constant__ int16_t c_sec_mode[16] = {123, -35, -8, -3, -32, -120, 30, 10, 14, 25, 123, -22, 8, 13, 19, 126};

@@ -76,6 +76,22 @@ __device__ __forceinline__ uint32_t sad4_acc(uint32_t a, uint32_t b, uint32_t c)
 __device__ __forceinline__ int clip3_d(int lo, int hi, int v) { return min(max(v, lo), hi); }
 __device__ __forceinline__ uint8_t clip_pel_d(int v) { return (uint8_t)min(max(v, 0), 255); }
 
+// The 4 bytes at any address from the aligned word or two words that hold
+// them (no word without one of the bytes is read: a block may end at the end
+// of its allocation).
+__device__ __forceinline__ uint32_t ld4_in(const uint8_t *p)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    const uint32_t lo = w[0];
+    return a & 3 ? __funnelshift_r(lo, w[1], 8 * (int)(a & 3)) : lo;
+}
+// byte k of a minus byte k of b
+__device__ __forceinline__ int byte_diff(uint32_t a, uint32_t b, int k)
+{
+    return (int)__byte_perm(a, 0, 0x4440 + k) - (int)__byte_perm(b, 0, 0x4440 + k);
+}
+
 // 4-point Walsh-Hadamard butterfly (unnormalised)
 __device__ __forceinline__ void fwht4_d(int &a, int &b, int &c, int &d)
 {
@@ -89,8 +105,8 @@ __device__ __forceinline__ int hsum4_d(const uint8_t *p1, intptr_t s1, const uin
     int m[4][4];
 #pragma unroll
     for (int y = 0; y < 4; y++) {
-        int a = p1[y * s1 + 0] - p2[y * s2 + 0], b = p1[y * s1 + 1] - p2[y * s2 + 1];
-        int c = p1[y * s1 + 2] - p2[y * s2 + 2], d = p1[y * s1 + 3] - p2[y * s2 + 3];
+        const uint32_t u = ld4_in(p1 + y * s1), v = ld4_in(p2 + y * s2);
+        int a = byte_diff(u, v, 0), b = byte_diff(u, v, 1), c = byte_diff(u, v, 2), d = byte_diff(u, v, 3);
         fwht4_d(a, b, c, d);
         m[y][0] = a; m[y][1] = b; m[y][2] = c; m[y][3] = d;
     }
@@ -112,7 +128,11 @@ __device__ __forceinline__ int hsum8_d(const uint8_t *p1, intptr_t s1, const uin
     for (int y = 0; y < 8; y++) {
         int v[8];
 #pragma unroll
-        for (int x = 0; x < 8; x++) v[x] = p1[y * s1 + x] - p2[y * s2 + x];
+        for (int q = 0; q < 2; q++) {
+            const uint32_t a = ld4_in(p1 + y * s1 + 4 * q), b = ld4_in(p2 + y * s2 + 4 * q);
+#pragma unroll
+            for (int x = 0; x < 4; x++) v[4 * q + x] = byte_diff(a, b, x);
+        }
         int t[8];
 #pragma unroll
         for (int i = 0; i < 4; i++) { t[i] = v[i] + v[i + 4]; t[i + 4] = v[i] - v[i + 4]; }
