@@ -178,6 +178,28 @@ def test_intra_rmd_every_shape(gpu, olib):
         assert np.array_equal(got["cand_mode"], modes) and np.array_equal(got["num_for_rdo"], nrdo)
 
 
+@pytest.mark.parametrize("hadamard", [1, 0])
+def test_intra_rmd_extreme_samples(gpu, olib, hadamard):
+    """Edges and source of 0 and 255 alone: the largest differences and
+    Hadamard sums of every shape."""
+    import xavs2_gb300 as xg
+    import xavs2_gb300.synth as synth
+    rng = np.random.default_rng(77)
+    yy, xx = np.mgrid[0:128, 0:128]
+    src = ((xx ^ yy) & 1).astype(np.uint8) * 255
+    src[:64, :64] = 255
+    src[:64, 64:] = rng.integers(0, 2, (64, 64)) * 255
+    rects = [(x, y, 4 << a, 4 << b) for a in range(5) for b in range(5) if abs(a - b) <= 2
+             for x, y in ((0, 0), (64, 0), (64, 64))]
+    blocks, edges = synth.intra_pack(rects, 255 - src, rng, xg.INTRA_BLOCK_DTYPE)
+    edges[:] = np.where(edges > 127, 255, 0)
+    prm = xg.IntraParams(7.25, hadamard, 1, 4, 2)
+    got = _rmd_gpu(gpu, blocks, edges, src, prm)
+    cost, modes, ccost, nrdo = _rmd_expected(olib, blocks, edges, src, prm)
+    assert np.array_equal(got["cost"], cost)
+    assert np.array_equal(got["cand_mode"], modes) and np.array_equal(got["num_for_rdo"], nrdo)
+
+
 def _fill_gpu(gpu, jobs, pic, size, width=None, height=None, prefill=0):
     import torch
     dev = torch.device("cuda:0")

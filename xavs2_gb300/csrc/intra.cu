@@ -12,6 +12,7 @@
 // predicts a block into shared memory and scores it in the same pass.
 #include "xavs2gpu_common.cuh"
 
+#include <cstddef>
 #include <cstring>
 
 namespace xg {
@@ -207,7 +208,10 @@ __global__ void __launch_bounds__(256) pred_block_kernel(int mode, const uint8_t
 // 4-sample window of the edge array (in ascending address order for all
 // directions) taken with a funnel shift and weighted with one dp4a.
 constexpr int kN = 9;             // INTRA_MODE_NUM_FOR_RDO (defines.h:290)
-constexpr int kTW = 11;           // warps per CTA: 3 modes each
+#ifndef XG_RMD_WARPS
+#define XG_RMD_WARPS 4
+#endif
+constexpr int kTW = XG_RMD_WARPS;   // warps per CTA
 constexpr int kTT = kTW * 32;
 constexpr int kCls = 25;
 // max over classes of G * (align4(edge window) + 4: the window's offset in
@@ -238,10 +242,33 @@ __host__ __device__ __forceinline__ Geo geo_of(int c)
     return g;
 }
 
+// Classes by tile work (G * w * h) descending, ties by class, and blocks per
+// tile: fixed by the geometry, so a table (with every CTA sorting the classes
+// by itself, one thread at a time, the 64x64 blocks of a 1080p picture alone
+// took 107 us against 66).
+struct ClassTab {
+    int8_t order[kCls], G[kCls];
+};
+constexpr ClassTab make_class_tab()
+{
+    ClassTab t{};
+    int work[kCls] = {};
+    for (int c = 0; c < kCls; c++) {
+        const int w = 4 << (c / 5), h = 4 << (c % 5), units = w / (w == 4 ? 4 : 8) * (h >> 2);
+        t.G[c] = (int8_t)(32 / (units < 32 ? units : 32));
+        work[c] = t.G[c] * w * h;
+        int j = c;
+        for (; j > 0 && work[(int)t.order[j - 1]] < work[c]; j--) t.order[j] = t.order[j - 1];
+        t.order[j] = (int8_t)c;
+    }
+    return t;
+}
+static __constant__ ClassTab c_classes = make_class_tab();
+
 // Two tile buffers: the next tile is copied in (cp.async) while the warps
 // score the current one.
 struct TileBuf {
-    uint8_t edge[kEdgeArea];          // block b: the words holding edge samples -lo..hi at b * (R + 4)
+    __align__(16) uint8_t edge[kEdgeArea];   // block b: the words holding edge samples -lo..hi at b * (R + 4)
     uint8_t fenc[4096 + 64];          // block b: w x h source samples at b * (w * h + 4)
     int64_t eoff[32], foff[32];
     int idx[32], dc_avail[32], mpm[32][2];
@@ -271,148 +298,200 @@ struct LaneConst {
     int dc, pa, pb, pc, bt;
 };
 
-// 4 edge samples p[0..3] as one word (any byte alignment)
-__device__ __forceinline__ uint32_t win4(const uint8_t *p)
+// Twice the weights of a 4-sample window for fraction f (0..31), first sample
+// lowest: (32 - f, 64 - f, 32 + f, f) = kUp + f kStep, its mirror kDown - f
+// kStep; no byte borrows.  Twice, so that the prediction is the second byte of
+// the weighted sum (which with its rounding stays below 2^16).
+constexpr uint32_t kWtsUp = 0x00408040u, kWtsDown = 0x40804000u, kWtsStep = 0x0201FDFEu;
+
+// 8 (12) bytes at byte offset `o` of the edge words (shared memory addressed
+// by index: a pointer cut to its word would be a generic 64-bit one)
+__device__ __forceinline__ void win8(const uint32_t *e, int o, uint32_t &b0, uint32_t &b1)
 {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    return __funnelshift_r(w[0], w[1], (unsigned)(a & 3) * 8u);
+    const int i = o >> 2, sh = (o & 3) * 8;
+    const uint32_t w0 = e[i], w1 = e[i + 1], w2 = e[i + 2];
+    b0 = __funnelshift_r(w0, w1, sh);
+    b1 = __funnelshift_r(w1, w2, sh);
 }
-__device__ __forceinline__ uint32_t wts(int b0, int b1, int b2, int b3)
+__device__ __forceinline__ void win12(const uint32_t *e, int o, uint32_t &b0, uint32_t &b1, uint32_t &b2)
 {
-    return (uint32_t)b0 | ((uint32_t)b1 << 8) | ((uint32_t)b2 << 16) | ((uint32_t)b3 << 24);
+    const int i = o >> 2, sh = (o & 3) * 8;
+    const uint32_t w0 = e[i], w1 = e[i + 1], w2 = e[i + 2], w3 = e[i + 3];
+    b0 = __funnelshift_r(w0, w1, sh);
+    b1 = __funnelshift_r(w1, w2, sh);
+    b2 = __funnelshift_r(w2, w3, sh);
 }
-__device__ __forceinline__ int tap(const uint8_t *ep, int s, uint32_t w)
+// bytes k .. k + 3 of the 8 bytes (a, b), k = 0..3
+__device__ __forceinline__ uint32_t bytes_at(uint32_t a, uint32_t b, int k)
 {
-    return (int)(__dp4a(win4(ep + s), w, 64u) >> 7);
+    return k == 0 ? a : __byte_perm(a, b, k == 1 ? 0x4321 : k == 2 ? 0x5432 : 0x6543);
 }
 
-// Hadamard sum of a 4x4 difference block held in registers
-__device__ __forceinline__ int hsum4_reg(int (&d)[4][4])
+// ---- one SATD unit: 4 rows of 8 samples (WIDE) or of 4 ---------------------------
+// Samples are kept as 16-bit pairs: column c in the low half, column c + 4 in
+// the high half (0 in units of 4 columns), so one packed add or subtract is a
+// butterfly of both 4x4 blocks.
+
+// A row's samples: column x reads the 4 edge bytes from o + x on.
+template <bool WIDE>
+__device__ __forceinline__ void row_pairs(const uint32_t *e, int o, uint32_t w, uint32_t (&p)[4])
 {
+    if (WIDE) {
+        uint32_t b0, b1, b2;
+        win12(e, o, b0, b1, b2);
 #pragma unroll
-    for (int r = 0; r < 4; r++) fwht4_d(d[r][0], d[r][1], d[r][2], d[r][3]);
-    int s = 0;
+        for (int c = 0; c < 4; c++)
+            p[c] = __byte_perm(__dp4a(bytes_at(b0, b1, c), w, 128u), __dp4a(bytes_at(b1, b2, c), w, 128u), 0x7531);
+    } else {
+        uint32_t b0, b1;
+        win8(e, o, b0, b1);
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        fwht4_d(d[0][c], d[1][c], d[2][c], d[3][c]);
-        s += iabs_d(d[0][c]) + iabs_d(d[1][c]) + iabs_d(d[2][c]) + iabs_d(d[3][c]);
+        for (int c = 0; c < 4; c++) p[c] = __dp4a(bytes_at(b0, b1, c), w, 128u) >> 8;
     }
-    return s;
+}
+// A column's weighted sums: row r reads the 4 edge bytes from o + 3 - r on.
+__device__ __forceinline__ void col_sums(const uint32_t *e, int o, uint32_t w, uint32_t (&s)[4])
+{
+    uint32_t b0, b1;
+    win8(e, o, b0, b1);
+#pragma unroll
+    for (int r = 0; r < 4; r++) s[r] = __dp4a(bytes_at(b0, b1, 3 - r), w, 128u);
 }
 
-// |H (src - pred) H^T| of the 4x4 sub-block at (x0, y0) of a block in `mode`
-__device__ __forceinline__ int sub4_hsum(int mode, const uint8_t *ep, const uint8_t *fb, int fstride, const Geo &g,
-                                         int x0, int y0, const LaneConst &kc, bool narrow5, bool narrow31)
+// the prediction of the unit at (x0, y0) of a block in `mode`
+template <bool WIDE>
+__device__ __forceinline__ void unit_pred(int mode, const uint32_t *e, int eo, const Geo &g, int x0, int y0,
+                                          const LaneConst &kc, bool narrow5, bool narrow31, uint32_t (&p)[4][4])
 {
-    int p[4][4];
+    const uint8_t *ep = reinterpret_cast<const uint8_t *>(e) + eo;
+    constexpr int kCols = WIDE ? 8 : 4;
+    constexpr uint32_t kBoth = WIDE ? 0x00010001u : 1u;
     if (mode == 0) {
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) p[r][c] = kc.dc;
+            for (int c = 0; c < 4; c++) p[r][c] = (uint32_t)kc.dc * kBoth;
     } else if (mode == 1) {
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) p[r][c] = min(max((kc.pa + kc.pb * (x0 + c) + kc.pc * (y0 + r)) >> 5, 0), 255);
+            for (int c = 0; c < 4; c++) {
+                const int v = kc.pa + kc.pb * (x0 + c) + kc.pc * (y0 + r);
+                p[r][c] = (uint32_t)min(max(v >> 5, 0), 255);
+                if (WIDE) p[r][c] |= (uint32_t)min(max((v + 4 * kc.pb) >> 5, 0), 255) << 16;
+            }
     } else if (mode == 2) {
         const int lx = ilog2d(g.w), ly = ilog2d(g.h), a = ep[g.w], b = ep[-g.h];
 #pragma unroll
         for (int r = 0; r < 4; r++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < kCols; c++) {
                 const int x = x0 + c, y = y0 + r, top = ep[1 + x], left = ep[-1 - y];
                 const int predx = (left << lx) + (x + 1) * (a - left);
                 const int predy = (top << ly) + (y + 1) * (b - top);
                 const int v = ((predx << ly) + (predy << lx) + x * y * kc.bt + (1 << (lx + ly))) >> (lx + ly + 1);
-                p[r][c] = min(max(v, 0), 255);
+                const uint32_t q = (uint32_t)min(max(v, 0), 255);
+                if (c < 4) p[r][c] = q;
+                else p[r][c & 3] |= q << 16;
             }
     } else if (mode == 12) {
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            const int v = ep[1 + x0 + c];
+            const uint32_t v = ep[1 + x0 + c] | (WIDE ? (uint32_t)ep[5 + x0 + c] << 16 : 0u);
 #pragma unroll
             for (int r = 0; r < 4; r++) p[r][c] = v;
         }
     } else if (mode == 24) {
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            const int v = ep[-1 - y0 - r];
+            const uint32_t v = ep[-1 - y0 - r] * kBoth;
 #pragma unroll
             for (int c = 0; c < 4; c++) p[r][c] = v;
         }
     } else if (narrow5 || narrow31) {
         // the reference's tabulated mode-5 / mode-31 variants (intra.c:455-605, 1147-1161)
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                p[r][c] = narrow5 ? mode5_narrow([ep](int i) { return (int)ep[i]; }, x0 + c, y0 + r, g.w)
-                                  : mode5_narrow([ep](int i) { return (int)ep[-i]; }, y0 + r, x0 + c, g.h);
-    } else if (mode < 12) {
-        // from the top row: row y reads ep[ix .. ix + 3], ix = step + x
-#pragma unroll
+#pragma unroll 1
         for (int r = 0; r < 4; r++) {
-            int f;
-            const int ix = ang_step(mode, 0, y0 + r + 1, f) + x0;
-            const uint32_t w = wts(32 - f, 64 - f, 32 + f, f);
+            uint32_t q[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) p[r][c] = tap(ep, ix + c, w);
-        }
-    } else if (mode > 24) {
-        // from the left column: column x reads ep[-iy - 3 .. -iy], iy = y + step
+            for (int c = 0; c < kCols; c++) {
+                const uint32_t v =
+                    (uint32_t)(narrow5 ? mode5_narrow([ep](int i) { return (int)ep[i]; }, x0 + c, y0 + r, g.w)
+                                       : mode5_narrow([ep](int i) { return (int)ep[-i]; }, y0 + r, x0 + c, g.h));
+                if (c < 4) q[c] = v;
+                else q[c & 3] |= v << 16;
+            }
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            int f;
-            const int iy = ang_step(mode, 1, x0 + c + 1, f) + y0;
-            const uint32_t w = wts(f, 32 + f, 64 - f, 32 - f);
+            for (int k = 0; k < 4; k++)
+                if (k == r)
 #pragma unroll
-            for (int r = 0; r < 4; r++) p[r][c] = tap(ep, -iy - r - 3, w);
+                    for (int c = 0; c < 4; c++) p[k][c] = q[c];
         }
     } else {
-        // both edges (intra.c:363-397)
-        int sx[4], sy[4];
-        uint32_t wx[4], wy[4];
+        // one edge (3..11 top, 25..32 left) or both (13..23, intra.c:363-397: the
+        // left column's samples where y - step >= 0); ang_step's step and
+        // fraction of distance d are d * 32 mul >> sh cut at bit 5
+        const bool both = mode < 24 && mode > 12;
+        const int lx0 = eo + x0 - (both ? 1 : 0), ly0 = eo - y0 - (both ? 5 : 6), sgn = both ? -1 : 1;
+        if (mode < 24) {
+            // row y from ep[x + step] (one edge) or ep[x - step - 1]
+            const int mul = 32 * c_ang[0][mode][0], sh = c_ang[0][mode][1];
+            const uint32_t wb = both ? kWtsDown : kWtsUp, wk = both ? 0u - kWtsStep : kWtsStep;
+            // both: rows that the left column serves in every column are skipped
+            const int last = both ? ((x0 + kCols) * 32 * c_ang[1][mode][0]) >> (c_ang[1][mode][1] + 5) : 1 << 20;
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            int f;
-            sx[r] = ang_step(mode, 0, y0 + r + 1, f);
-            wx[r] = wts(f, 32 + f, 64 - f, 32 - f);
+            for (int r = 0; r < 4; r++) {
+                const int q = ((y0 + r + 1) * mul) >> sh;
+                if (y0 + r < last) row_pairs<WIDE>(e, lx0 + sgn * (q >> 5), wb + (uint32_t)(q & 31) * wk, p[r]);
+                else p[r][0] = p[r][1] = p[r][2] = p[r][3] = 0;
+            }
         }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            int f;
-            sy[c] = ang_step(mode, 1, x0 + c + 1, f);
-            wy[c] = wts(32 - f, 64 - f, 32 + f, f);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++)
+        if (mode > 12) {
+            // column x, row y from ep[-(y + step) - 3] (one edge) or ep[step - y - 2]
+            const int mul = 32 * c_ang[1][mode][0], sh = c_ang[1][mode][1];
+            const uint32_t wb = both ? kWtsUp : kWtsDown, wk = both ? kWtsStep : 0u - kWtsStep;
 #pragma unroll
             for (int c = 0; c < 4; c++) {
-                const int x = x0 + c, y = y0 + r, iyy = y - sy[c];
-                p[r][c] = iyy <= -1 ? tap(ep, x - sx[r] - 1, wx[r]) : tap(ep, -iyy - 2, wy[c]);
+                const int q = ((x0 + c + 1) * mul) >> sh, q4 = ((x0 + c + 5) * mul) >> sh;
+                // the unit's rows from these on take the column
+                const int from = both ? (q >> 5) - y0 : 0, from4 = both ? (q4 >> 5) - y0 : 0;
+                if (from >= 4) continue;   // steps grow with the column
+                uint32_t s[4];
+                col_sums(e, ly0 - sgn * (q >> 5), wb + (uint32_t)(q & 31) * wk, s);
+                if (WIDE) {
+                    uint32_t s4[4];
+                    col_sums(e, ly0 - sgn * (q4 >> 5), wb + (uint32_t)(q4 & 31) * wk, s4);
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const uint32_t v = __byte_perm(s[r], s4[r], 0x7531);
+                        p[r][c] = r >= from4 ? v : r >= from ? __byte_perm(v, p[r][c], 0x7610) : p[r][c];
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) p[r][c] = r >= from ? s[r] >> 8 : p[r][c];
+                }
             }
+        }
     }
-    int d[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const uint32_t f = *reinterpret_cast<const uint32_t *>(fb + (y0 + r) * fstride + x0);
-#pragma unroll
-        for (int c = 0; c < 4; c++) d[r][c] = (int)((f >> (8 * c)) & 0xFFu) - p[r][c];
-    }
-    return hsum4_reg(d);
 }
 
-// SAD of the same sub-block (use_hadamard = 0)
-__device__ __forceinline__ int sub4_sad(int mode, const uint8_t *ep, const uint8_t *fb, const Geo &g, int x0, int y0,
-                                        const ModeConst &k)
+// Cost of one unit: SATD, half the Hadamard sum of its one or two 4x4
+// blocks, or SAD.
+template <bool WIDE>
+__device__ __forceinline__ int unit_cost(bool hadamard, int mode, const uint32_t *e, int eo, const uint8_t *fb,
+                                         const Geo &g, int x0, int y0, const LaneConst &kc, bool narrow5, bool narrow31)
 {
-    int s = 0;
-    for (int r = 0; r < 4; r++)
-        for (int c = 0; c < 4; c++)
-            s += iabs_d((int)fb[(y0 + r) * g.w + x0 + c] - pred_sample(mode, ep, x0 + c, y0 + r, g.w, g.h, k));
-    return s;
+    uint32_t d[4][4];
+    unit_pred<WIDE>(mode, e, eo, g, x0, y0, kc, narrow5, narrow31, d);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const uint8_t *q = fb + (y0 + r) * g.w + x0;
+        const uint32_t f0 = *reinterpret_cast<const uint32_t *>(q);
+        const uint32_t f1 = WIDE ? *reinterpret_cast<const uint32_t *>(q + 4) : 0u;
+#pragma unroll
+        for (int c = 0; c < 4; c++) d[r][c] = (__byte_perm(f0, f1, 0x4400 + 0x1111 * c) & 0x00FF00FFu) - d[r][c];
+    }
+    return hadamard ? satd_pairs(d) : sad_pairs(d);
 }
 
 // update_candidate_list (md_intra.c:195-210): insertion into the 9-entry
@@ -555,8 +634,13 @@ __global__ void rmd_scatter_kernel(const xavs2gpu_intra_block_t *__restrict__ bl
 }
 
 // 3. the tiles, persistent; classes with the most work per tile first
+// Warps per CTA and resident CTAs per SM (registers): a CTA's 33 modes go round
+// its warps, so few warps leave fewer idle in the last round and the CTAs hide
+// the tile loads of one another.  The whole decision of a 1080p picture took,
+// in us: 11 x 2 938, 8 x 3 899, 6 x 5 884, 3 x 9 864, 4 x 8 838 (spills),
+// 4 x 6 829, 4 x 7 814.
 #ifndef XG_RMD_MINB
-#define XG_RMD_MINB 3
+#define XG_RMD_MINB 7
 #endif
 __global__ void __launch_bounds__(kTT, XG_RMD_MINB) rmd_tile_kernel(const xavs2gpu_intra_block_t *__restrict__ blocks,
                                                         const int *__restrict__ counts, const int *__restrict__ sorted,
@@ -576,25 +660,11 @@ __global__ void __launch_bounds__(kTT, XG_RMD_MINB) rmd_tile_kernel(const xavs2g
             s.start[c] = acc;
             acc += s.count[c];
         }
-        // order: tile work (G * w * h) descending, ties by class
-        for (int c = 0; c < kCls; c++) s.order[c] = c;
-        for (int i = 1; i < kCls; i++) {
-            const int c = s.order[i];
-            const Geo gc = geo_of(c);
-            const int wc = gc.G * gc.w * gc.h;
-            int j = i;
-            while (j > 0) {
-                const Geo gp = geo_of(s.order[j - 1]);
-                if (gp.G * gp.w * gp.h >= wc) break;
-                s.order[j] = s.order[j - 1];
-                j--;
-            }
-            s.order[j] = c;
-        }
         s.tile_base[0] = 0;
         for (int k = 0; k < kCls; k++) {
-            const Geo g = geo_of(s.order[k]);
-            s.tile_base[k + 1] = s.tile_base[k] + (s.count[s.order[k]] + g.G - 1) / g.G;
+            const int c = c_classes.order[k], G = c_classes.G[c];   // G a power of two
+            s.order[k] = c;
+            s.tile_base[k + 1] = s.tile_base[k] + ((s.count[c] + G - 1) >> ilog2d(G));
         }
     }
     __syncthreads();
@@ -687,9 +757,11 @@ __global__ void __launch_bounds__(kTT, XG_RMD_MINB) rmd_tile_kernel(const xavs2g
             const int b = lane / g.lanes, u0 = lane - b * g.lanes;
             const bool live = b < nb;
             const int bb = live ? b : 0;
-            const uint8_t *ep = B.edge + bb * (g.R + 4) + B.emis[bb] + g.lo;
+            const uint32_t *ew = reinterpret_cast<const uint32_t *>(B.edge);
+            const int eo = bb * (g.R + 4) + B.emis[bb] + g.lo;   // the block's sample ep[0]
+            const uint8_t *ep = B.edge + eo;
             const uint8_t *fb = B.fenc + bb * fpitch;
-            const int lx = ilog2d(g.w), ly = ilog2d(g.h);
+            const int lx = ilog2d(g.w), ly = ilog2d(g.h), lnux = ilog2d(g.nux);
             int mi = 0;
             if (lane == 0) mi = atomicAdd(&s.next_mode, 1);
             mi = __shfl_sync(0xffffffffu, mi, 0);
@@ -732,22 +804,10 @@ __global__ void __launch_bounds__(kTT, XG_RMD_MINB) rmd_tile_kernel(const xavs2g
                 int acc = 0;
                 if (live) {
                     for (int it = 0; it < g.iters; it++) {
-                        const int u = u0 + it * g.lanes, uq = u / g.nux;
-                        const int uy = uq * 4, ux = (u - uq * g.nux) * g.uw;
-                        int hs = 0;
-                        if (prm.use_hadamard) {
-#pragma unroll 1
-                            for (int x0 = ux; x0 < ux + g.uw; x0 += 4)
-                                hs += sub4_hsum(mode, ep, fb, g.w, g, x0, uy, kc, n5, n31);
-                            acc += hs >> 1;
-                        } else {
-                            ModeConst k{};
-                            k.dc = kc.dc; k.pa = kc.pa; k.pb = kc.pb; k.pc = kc.pc; k.bt = kc.bt;
-                            k.ba = ep[g.w]; k.bb = ep[-g.h]; k.lx = lx; k.ly = ly;
-                            for (int r = 0; r < 4; r++)
-                                for (int x = ux; x < ux + g.uw; x++)
-                                    acc += iabs_d((int)fb[(uy + r) * g.w + x] - pred_sample(mode, ep, x, uy + r, g.w, g.h, k));
-                        }
+                        const int u = u0 + it * g.lanes, uq = u >> lnux;
+                        const int uy = uq * 4, ux = (u - (uq << lnux)) * g.uw;
+                        acc += g.uw == 8 ? unit_cost<true>(prm.use_hadamard != 0, mode, ew, eo, fb, g, ux, uy, kc, n5, n31)
+                                         : unit_cost<false>(prm.use_hadamard != 0, mode, ew, eo, fb, g, ux, uy, kc, n5, n31);
                     }
                 }
                 for (int o = g.lanes >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -768,21 +828,35 @@ __global__ void __launch_bounds__(kTT, XG_RMD_MINB) rmd_tile_kernel(const xavs2g
     }
 }
 
-// 4. the candidate lists, a thread per block
-__global__ void __launch_bounds__(128) rmd_cand_kernel(const xavs2gpu_intra_block_t *__restrict__ blocks, int n,
-                                                        xavs2gpu_intra_params_t prm,
-                                                        xavs2gpu_intra_result_t *__restrict__ out)
+// 4. the candidate lists, a thread per block.  The CTA's costs (the first 264
+// of a record's 376 bytes) come through shared memory: read as consecutive
+// words instead of one 8-byte access per thread and record, and the replay
+// reads the ones it visits from there.
+constexpr int kCandThreads = 64;
+constexpr int kRecWords = (int)sizeof(xavs2gpu_intra_result_t) / 4, kCostWords = 66;
+static_assert(sizeof(xavs2gpu_intra_result_t) % 8 == 0 && offsetof(xavs2gpu_intra_result_t, cand_cost) == 4 * kCostWords,
+              "a result record: 33 costs, then the candidates");
+
+__global__ void __launch_bounds__(kCandThreads) rmd_cand_kernel(const xavs2gpu_intra_block_t *__restrict__ blocks, int n,
+                                                                 xavs2gpu_intra_params_t prm,
+                                                                 xavs2gpu_intra_result_t *__restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const xavs2gpu_intra_block_t b = blocks[i];
+    __shared__ __align__(8) uint32_t cost[kCandThreads * kCostWords];
+    const int i0 = blockIdx.x * kCandThreads, tid = threadIdx.x, nb = min(kCandThreads, n - i0);
+    const uint32_t *g = reinterpret_cast<const uint32_t *>(out + i0);
+#pragma unroll 6
+    for (int e = tid; e < nb * kCostWords; e += kCandThreads) {
+        const int r = e / kCostWords;
+        cost[e] = g[r * kRecWords + e - r * kCostWords];
+    }
+    __syncthreads();
+    if (tid >= nb) return;
+    const xavs2gpu_intra_block_t b = blocks[i0 + tid];
     if (block_class(b) < 0) return;
-    xavs2gpu_intra_result_t &r = out[i];
-    long long key[33];
-#pragma unroll
-    for (int m = 0; m < 33; m++) key[m] = __double_as_longlong(r.cost[m]);
     CandList L;
-    const int nr = candidates(key, prm.rough, prm.dist2, prm.dist1, b.num_for_rdo, b.mpm[0], b.mpm[1], L);
+    const int nr = candidates(reinterpret_cast<const long long *>(cost + tid * kCostWords), prm.rough, prm.dist2,
+                              prm.dist1, b.num_for_rdo, b.mpm[0], b.mpm[1], L);
+    xavs2gpu_intra_result_t &r = out[i0 + tid];
     r.num_for_rdo = nr;
 #pragma unroll
     for (int k = 0; k < kN; k++) {
@@ -809,7 +883,10 @@ __device__ __forceinline__ int usable_sides(int avail, int x, int y, int bsx, in
     return avail & ok;
 }
 
-// A warp per block writes ep[-edge_below .. edge_above]: the top row and
+constexpr int kFillLanes = 16;
+// A half-warp per block (a small block's window is three steps of 16 samples,
+// and a warp repeats the block's setup for fewer: 64 us for a 1080p picture's
+// blocks, 42 with half-warps) writes ep[-edge_below .. edge_above]: the top row and
 // top-right run (the last top sample repeated when the top-right is
 // missing), the left column and left-down run likewise, 128 for a missing
 // side, the corner from the top-left, else the first top, else the first
@@ -819,7 +896,7 @@ __global__ void __launch_bounds__(256) fill_edges_kernel(const xavs2gpu_intra_ed
                                                          const uint8_t *__restrict__ pic, int stride, int width,
                                                          int height, uint8_t *__restrict__ edges, long long edges_size)
 {
-    const int w = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int w = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) / kFillLanes), lane = threadIdx.x % kFillLanes;
     if (w >= n) return;
     const xavs2gpu_intra_edge_job_t j = jobs[w];
     const int bsx = j.width, bsy = j.height, a = side_log(bsx), c = side_log(bsy);
@@ -830,29 +907,16 @@ __global__ void __launch_bounds__(256) fill_edges_kernel(const xavs2gpu_intra_ed
     const bool L = av & 1, T = av & 2, LD = av & 4, TR = av & 8, TL = av & 16;
     const long long row = (long long)(j.y - 1) * stride + j.x - 1;   // the corner's position
     uint8_t *ep = edges + j.edge_offset;
-    for (int k = -lo + lane; k <= hi; k += 32) {
+    for (int k = -lo + lane; k <= hi; k += kFillLanes) {
+        // a side's sample o away from the corner: past the first run the next
+        // one's, or the first run's last again; past both the last
+        const int bs = k > 0 ? bsx : bsy;
+        const bool first = k > 0 ? T : L, second = k > 0 ? TR : LD;
+        int o = min(abs(k), 2 * bs);
+        if (o > bs && !second) o = bs;
         int v = 128;
-        if (k > 0) {
-            const int kk = min(k, 2 * bsx);
-            if (kk <= bsx) {
-                if (T) v = pic[row + kk];
-            } else if (TR) {
-                v = pic[row + kk];
-            } else if (T) {
-                v = pic[row + bsx];
-            }
-        } else if (k < 0) {
-            const int jj = min(-k, 2 * bsy);
-            if (jj <= bsy) {
-                if (L) v = pic[row + (long long)jj * stride];
-            } else if (LD) {
-                v = pic[row + (long long)jj * stride];
-            } else if (L) {
-                v = pic[row + (long long)bsy * stride];
-            }
-        } else {
-            v = TL ? pic[row] : T ? pic[row + 1] : L ? pic[row + stride] : 128;
-        }
+        if (k == 0) v = TL ? pic[row] : T ? pic[row + 1] : L ? pic[row + stride] : 128;
+        else if (o > bs || first) v = pic[row + (k > 0 ? (long long)o : (long long)o * stride)];
         ep[k] = (uint8_t)v;
     }
 }
@@ -870,8 +934,9 @@ extern "C" int xavs2gpu_intra_fill_edges(const xavs2gpu_intra_edge_job_t *jobs, 
         return XAVS2GPU_ERR_ARG;
     }
     if (n == 0) return XAVS2GPU_OK;
-    intra::fill_edges_kernel<<<(unsigned)((n + 7) / 8), 256, 0, (cudaStream_t)stream>>>(jobs, n, pic, stride, width,
-                                                                                         height, edges, edges_size);
+    const unsigned per_cta = 256 / intra::kFillLanes;
+    intra::fill_edges_kernel<<<((unsigned)n + per_cta - 1) / per_cta, 256, 0, (cudaStream_t)stream>>>(
+        jobs, n, pic, stride, width, height, edges, edges_size);
     count_launch();
     XG_CUDA(cudaGetLastError());
     return XAVS2GPU_OK;
@@ -983,7 +1048,7 @@ extern "C" int xavs2gpu_intra_rmd_batch(const xavs2gpu_intra_block_t *blocks, in
     if (grid > n) grid = n;
     intra::rmd_tile_kernel<<<(int)grid, intra::kTT, smem, stream>>>(blocks, counts, sorted, edges, fenc, fenc_stride,
                                                                      *prm, out);
-    intra::rmd_cand_kernel<<<(n + 127) / 128, 128, 0, stream>>>(blocks, n, *prm, out);
+    intra::rmd_cand_kernel<<<(n + intra::kCandThreads - 1) / intra::kCandThreads, intra::kCandThreads, 0, stream>>>(blocks, n, *prm, out);
     count_launch(4);
     XG_CUDA(cudaFreeAsync(scratch, stream));
     XG_CUDA(cudaGetLastError());

@@ -99,6 +99,50 @@ __device__ __forceinline__ void fwht4_d(int &a, int &b, int &c, int &d)
     a = s0 + s1; b = d0 + d1; c = s0 - s1; d = d0 - d1;
 }
 
+// ---- two 4x4 blocks side by side ---------------------------------------------
+// Differences of two 4x4 blocks in one integer each, hi * 2^16 + lo with both
+// signed: plain 32-bit adds and subtracts are exact butterflies of both blocks
+// at 123 lanes a clock per SM, where __vadd2 / __vsub2 run at 60 and __vabsss2
+// at 12 (measured; 128 is full issue).  The Hadamard sum's last butterflies
+// |a + b| + |a - b| are 2 max(|a|, |b|); with a and b (|a|, |b| <= 2040) biased
+// by 2^11 their halves are unsigned 16-bit values and
+//     max(|a|, |b|) = max(max(a', b'), 2^12 - min(a', b')) - 2^11,
+// three native packed instructions and a subtraction.
+constexpr uint32_t kPairBias = 0x08000800u;
+__device__ __forceinline__ uint32_t max_abs_pair(uint32_t a, uint32_t b)   // a, b and the result biased
+{
+    return __vmaxu2(__vmaxu2(a, b), 0x10001000u - __vminu2(a, b));
+}
+// half the sum of |H D H^T| over both blocks (the sum is even)
+__device__ __forceinline__ int satd_pairs(uint32_t (&d)[4][4])
+{
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        const uint32_t s0 = d[r][0] + d[r][1], e0 = d[r][0] - d[r][1];
+        const uint32_t s1 = d[r][2] + d[r][3], e1 = d[r][2] - d[r][3];
+        d[r][0] = s0 + s1;
+        d[r][1] = e0 + e1;
+        d[r][2] = s0 - s1;
+        d[r][3] = e0 - e1;
+    }
+    uint32_t s = 0;
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        s += max_abs_pair(d[0][c] + d[1][c] + kPairBias, d[2][c] + d[3][c] + kPairBias) +
+             max_abs_pair(d[0][c] - d[1][c] + kPairBias, d[2][c] - d[3][c] + kPairBias);
+    return (int)(s & 0xFFFFu) + (int)(s >> 16) - 2 * 8 * 2048;
+}
+// sum of |d| over both blocks (|d| <= 255)
+__device__ __forceinline__ int sad_pairs(uint32_t (&d)[4][4])
+{
+    uint32_t s = 0;
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) s += max_abs_pair(d[r][c] + kPairBias, d[r][c] + kPairBias);
+    return (int)(s & 0xFFFFu) + (int)(s >> 16) - 2 * 16 * 2048;
+}
+
 // sum of |H D H^T| over the 4x4 difference block at (p1, p2)
 __device__ __forceinline__ int hsum4_d(const uint8_t *p1, intptr_t s1, const uint8_t *p2, intptr_t s2)
 {
