@@ -201,6 +201,26 @@ def test_cu_partition_refinement(gpu, olib, had, frac, fast, pmvr):
     _assert_same(got, exp, allp)
 
 
+@pytest.mark.parametrize("had", [1, 0])
+def test_refinement_extreme_samples(gpu, olib, had):
+    """Pictures of 0 and 255 alone (checkerboard, flat, random): the largest
+    differences and Hadamard sums of the refinement's units."""
+    import xavs2_gb300 as xg
+    rng = np.random.default_rng(61)
+    w, h = 128, 128
+    yy, xx = np.mgrid[0:h, 0:w]
+    cur = ((xx ^ yy) & 1).astype(np.uint8) * 255
+    cur[:64, :64] = 255
+    cur[:64, 64:] = rng.integers(0, 2, (64, 64)) * 255
+    refs = [255 - cur, np.zeros_like(cur)]
+    ctu = xg.frame_pus(w, h, 2)
+    cus, _ = xg.cu_pus(xg.split_map_cus(w, h, 5), w, h, 2)
+    prm = xg.MeParams(4, oracle.lambda_factor(27), had, 2)
+    for pus in (ctu, cus):
+        got, _ = _run(cur, refs, pus, prm)
+        _assert_same(got, _oracle(olib, cur, refs, pus, prm), pus)
+
+
 def test_tuning_cu_groups(gpu, olib):
     """The CU-grouped refinement on and off (xavs2gpu_me_set_tuning) give the
     same results; bad tuning values are refused."""

@@ -549,11 +549,8 @@ __global__ void __launch_bounds__(128) refine_kernel(const xavs2gpu_pu_t *__rest
 // The refinement's unit costs (SATD with one rounding per 4x4 or 8x4 unit,
 // pixel.c:321, 347, or SAD) on packed 16-bit pairs: a pair holds column k of
 // the unit's left 4x4 block and column k of its right one (zero for a 4x4
-// unit), so each vadd2 / vsub2 takes one butterfly of both blocks.  The
-// differences (|d| <= 255) grow to at most 16 x 255 = 4080 through the two
-// 4-point passes, well inside 16 bits, so every value equals the 32-bit
-// form's; the absolute values are summed by dp2a.  Build option
-// XG_REFINE_PACKED=0 keeps the 32-bit form.
+// unit); one 32-bit add or subtract takes one butterfly of both blocks
+// (satd_pairs).  Build option XG_REFINE_PACKED=0 keeps the 32-bit form.
 #ifndef XG_REFINE_PACKED
 #define XG_REFINE_PACKED 1
 #endif
@@ -600,12 +597,6 @@ __device__ __forceinline__ void load_unit(const uint8_t *o, int stride, UnitCur 
     }
 }
 
-// |x| summed over the two halves of v, plus acc
-__device__ __forceinline__ int abs_pair_acc(uint32_t v, int acc)
-{
-    return __dp2a_lo((int)__vabsss2(v), 0x0101, acc);
-}
-
 template <bool U4>
 __device__ __forceinline__ int unit_cost_pre(bool had, const UnitCur &c, const uint8_t *r, int stride)
 {
@@ -626,26 +617,10 @@ __device__ __forceinline__ int unit_cost_pre(bool had, const UnitCur &c, const u
         uint32_t lo, hi, q[4];
         load8u(r + y * stride, lo, hi);
         row_pairs(lo, U4 ? 0u : hi, q);
-        // differences, then the 4-point transform of the row in both blocks
-        const uint32_t d0 = __vsub2(c.q[y][0], q[0]), d1 = __vsub2(c.q[y][1], q[1]);
-        const uint32_t d2 = __vsub2(c.q[y][2], q[2]), d3 = __vsub2(c.q[y][3], q[3]);
-        const uint32_t s0 = __vadd2(d0, d1), e0 = __vsub2(d0, d1), s1 = __vadd2(d2, d3), e1 = __vsub2(d2, d3);
-        d[y][0] = __vadd2(s0, s1);
-        d[y][1] = __vadd2(e0, e1);
-        d[y][2] = __vsub2(s0, s1);
-        d[y][3] = __vsub2(e0, e1);
-    }
-    int s = 0;
 #pragma unroll
-    for (int x = 0; x < 4; x++) {
-        const uint32_t s0 = __vadd2(d[0][x], d[1][x]), e0 = __vsub2(d[0][x], d[1][x]);
-        const uint32_t s1 = __vadd2(d[2][x], d[3][x]), e1 = __vsub2(d[2][x], d[3][x]);
-        s = abs_pair_acc(__vadd2(s0, s1), s);
-        s = abs_pair_acc(__vadd2(e0, e1), s);
-        s = abs_pair_acc(__vsub2(s0, s1), s);
-        s = abs_pair_acc(__vsub2(e0, e1), s);
+        for (int x = 0; x < 4; x++) d[y][x] = c.q[y][x] - q[x];
     }
-    return s >> 1;
+    return satd_pairs(d);
 }
 
 #if XG_REFINE_PACKED
@@ -760,25 +735,10 @@ __device__ __forceinline__ int unit_cost_pre_rt(bool had, bool u4, const UnitCur
         uint32_t lo, hi, q[4];
         load8u(r + y * stride, lo, hi);
         row_pairs(lo, u4 ? 0u : hi, q);
-        const uint32_t d0 = __vsub2(c.q[y][0], q[0]), d1 = __vsub2(c.q[y][1], q[1]);
-        const uint32_t d2 = __vsub2(c.q[y][2], q[2]), d3 = __vsub2(c.q[y][3], q[3]);
-        const uint32_t s0 = __vadd2(d0, d1), e0 = __vsub2(d0, d1), s1 = __vadd2(d2, d3), e1 = __vsub2(d2, d3);
-        d[y][0] = __vadd2(s0, s1);
-        d[y][1] = __vadd2(e0, e1);
-        d[y][2] = __vsub2(s0, s1);
-        d[y][3] = __vsub2(e0, e1);
-    }
-    int s = 0;
 #pragma unroll
-    for (int x = 0; x < 4; x++) {
-        const uint32_t s0 = __vadd2(d[0][x], d[1][x]), e0 = __vsub2(d[0][x], d[1][x]);
-        const uint32_t s1 = __vadd2(d[2][x], d[3][x]), e1 = __vsub2(d[2][x], d[3][x]);
-        s = abs_pair_acc(__vadd2(s0, s1), s);
-        s = abs_pair_acc(__vadd2(e0, e1), s);
-        s = abs_pair_acc(__vsub2(s0, s1), s);
-        s = abs_pair_acc(__vsub2(e0, e1), s);
+        for (int x = 0; x < 4; x++) d[y][x] = c.q[y][x] - q[x];
     }
-    return s >> 1;
+    return satd_pairs(d);
 }
 #endif
 
