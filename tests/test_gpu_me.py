@@ -77,6 +77,28 @@ def test_ctu_layout_all_pus(gpu, olib, R, w, h):
     _assert_same(got, exp, pus)
 
 
+@pytest.mark.parametrize("R,w,h,nrefs,extra", [(16, 2040, 1016, 2, 300), (16, 2040, 1016, 1, 300), (64, 760, 632, 1, 60),
+                                               (128, 200, 136, 1, 0), (2, 72, 72, 1, 200)])
+def test_ctu_rows_per_cta(gpu, olib, R, w, h, nrefs, extra):
+    """The shared-window search at each chunk height (8, 4 and 2 rows per
+    warp: many jobs, a middle number, the largest range and few jobs), sizes
+    that are no multiple of 64: one PU per CTU and reference and some more."""
+    import xavs2_gb300 as xg
+    rng = np.random.default_rng(R + w + nrefs)
+    cur, ref0 = _frames(rng, w, h)
+    _, ref1 = _frames(rng, w, h, shift=(-3, 4))
+    pus = xg.frame_pus(w, h, nrefs)
+    order = rng.permutation(len(pus))
+    ctu = (pus["ref"].astype(np.int64) << 32) + ((pus["y"].astype(np.int64) >> 6) << 16) + (pus["x"] >> 6)
+    _, first = np.unique(ctu[order], return_index=True)
+    pus = pus[np.concatenate([order[first], order[:extra]])]
+    pus = pus[np.unique(np.stack([pus["x"], pus["y"], pus["part"], pus["ref"]], 1), axis=0, return_index=True)[1]]
+    prm = xg.MeParams(R, oracle.lambda_factor(32), 1, 0, 0, 0)
+    got, stats = _run(cur, [ref0, ref1][:nrefs], pus, prm)
+    assert stats[0] == len(pus) and stats[1] == 0, stats
+    _assert_same(got, _oracle(olib, cur, [ref0, ref1][:nrefs], pus, prm), pus)
+
+
 @pytest.mark.parametrize("lam,on_ctu", [(1 << 25, True), (1 << 27, False)])
 def test_large_lambda(gpu, olib, lam, on_ctu):
     """Large MV costs: lambda 2^25 keeps the CTU search (its 32-bit keys hold

@@ -10,20 +10,30 @@
 // block SADs of the CTU once per displacement and derives all 849 PU costs
 // from them (sums in registers, warp shuffles across regions).
 //
-// Warp layout: lane = ry*8 + rx*2 + half.  (rx, ry) is one of the 16 16x16
+// Warp layout: a lane is (rx, ry, half): (rx, ry) is one of the 16 16x16
 // regions of the CTU, half selects its top or bottom 8 rows.  A lane owns the
 // 8 4x4 SADs of its half-region, the 18 PUs of its two 8x8 CUs and 6-7 PUs of
 // its 16x16 CU; the 52 PUs of the 32x32 CUs and the 13 of the 64x64 CU are
 // spread over the lanes (2 + 1 per lane at most).
 //
-// A CTA of 4 warps handles one (CTU, reference) and a chunk of 32 search rows
-// (8 per warp) over the whole horizontal range; its reference window lives in
-// shared memory.  Each warp keeps, per PU, the minimum of a 32-bit key
-// (cost << 11 | row-in-warp << 8 | dx+R) for PUs up to 16x16 and per-row keys
-// for the larger ones (the same form in interior jobs, cost << 8 | dx+R in
-// border jobs, whose poisoned sums need the room), and merges them into the
-// global 64-bit (cost, visit order) keys with atomicMin.  For ranges of 32
-// and up a warp takes two search rows per pass over the window.
+// A CTA of 4 warps handles one (CTU, reference) and a chunk of 8, 16 or 32
+// search rows (2, 4 or 8 per warp) over the whole horizontal range; its
+// reference window lives in shared memory.  Each warp keeps, per PU, the
+// minimum of a 32-bit key (cost << 11 | row-in-warp << 8 | dx+R) and merges it
+// into the global 64-bit (cost, visit order) keys with atomicMin.  A warp takes
+// two search rows per pass over the window.
+//
+// The search is bound by instruction issue and, within it, by the pipe that
+// byte SADs share with permutes, selects and minima (half rate).  So the window
+// holds every 4-sample word at its four byte alignments, as two planes of
+// 8-byte entries (row, k): {w(4k), w(4k+1)} and {w(4k+2), w(4k+3)}, w(i) the
+// samples i .. i+3.  An 8-byte load then serves two displacements of two rows,
+// where a row's four words took five word loads and twelve byte permutes.  A
+// pass covers two rows and two displacements: 32 accumulators and no spill at
+// 168 registers, so three CTAs share an SM (16-byte entries of all four
+// alignments need 64 accumulators, spill at 255 registers and wait on their
+// loads).  1080p, one reference, R = 64: 1677 us with the permutes (two CTAs per
+// SM), 1354 now, where 16-byte entries took 2119 and passes of four rows 1493.
 //
 // Search limits: a PU is valid at a displacement iff the referenced block
 // lies within [-58, W+58) x [-58, H+58) -- the limits pred_inter_search_single
@@ -36,9 +46,10 @@
 namespace xg {
 
 constexpr int kSlots = 849;
-constexpr int kDyChunk = 32;            // search rows per CTA
-constexpr int kDyWarp = 8;              // search rows per warp
-constexpr int kCtuThreads = 128;
+constexpr int kCtuWarps = 4;
+constexpr int kCtuThreads = 32 * kCtuWarps;
+constexpr int kDyWarpMax = 8;           // search rows per warp: 8, 4 or 2 (3 key bits)
+constexpr int kDyChunkMax = kCtuWarps * kDyWarpMax;
 constexpr uint32_t kPoisonSmall = 126976u;     // > any valid cost of a PU up to 16x16
 constexpr uint32_t kPoisonLarge = 1u << 22;    // replaces a 4x4 SAD outside the limits
 constexpr uint32_t kCapLarge = 2000000u;       // > any valid cost of a 64x64 PU
@@ -136,31 +147,29 @@ struct SlotTable {
 
 // ---- device helpers ------------------------------------------------------------------
 
-// bytes o..o+3 of the 8-byte little-endian pair (lo, hi), o = 1..3
-#ifndef XG_CTU_PRMT
-#define XG_CTU_PRMT 1
-#endif
-__device__ __forceinline__ uint32_t align_bytes(uint32_t lo, uint32_t hi, int o)
-{
-#if XG_CTU_PRMT
-    return __byte_perm(lo, hi, o == 1 ? 0x4321 : o == 2 ? 0x5432 : 0x6543);
-#else
-    return __funnelshift_r(lo, hi, 8 * o);
-#endif
-}
-
 __device__ __forceinline__ uint32_t addmin(uint32_t a, uint32_t b, uint32_t c)
 {
     return __viaddmin_u32(a, b, c);   // min(a + b, c)
 }
 
-// Window row layout: rows are ww bytes apart (ww a multiple of 128, i.e. each
-// row starts on bank 0) and row i is shifted right by swz(i) words.  In one
-// shared load the 32 lanes read rows 8q + t (q = 2*ry + half, t common) at
-// word 4*rx + k + t'; swz maps the eight q to {0,1,2,3,16,17,18,19}, so with
-// the 4*rx offsets the lanes hit 32 distinct banks.
-__host__ __device__ __forceinline__ int swz(int row) { return ((row >> 3) & 3) + 16 * ((row >> 5) & 1); }
-constexpr int kSwzMax = 19;   // words
+// Window layout in 8-byte entries: a row is ctu_pitch(R) entries (15 + R/2:
+// word 4*rx + c + (displacement >> 2) of rx, c <= 3), one entry is skipped
+// after every 8 rows, and the second plane follows the first.  An 8-byte shared
+// load serves 16 lanes at a time; lane bits 0-3 are half, rx bit 0, ry bit 0 and
+// rx bit 1, so these read rows 8q + t of four consecutive q = 2*ry + half
+// (skewed by 0..3 entries) at entries 4*rx: 16 distinct pairs of banks.
+__host__ __device__ __forceinline__ int ctu_pitch(int R) { return 15 + (R >> 1); }
+__host__ __device__ __forceinline__ int ctu_entry(int row, int pitch) { return row * pitch + (row >> 3); }
+
+// bytes of a chunk's MV-cost keys and of its window (multiples of 128), and
+// the distance of the window's planes in entries
+__host__ __device__ __forceinline__ uint32_t ctu_key_bytes(int R, int dyw) { return 4u * (uint32_t)(kCtuWarps * dyw * 2 * R); }
+__host__ __device__ __forceinline__ uint32_t ctu_win_bytes(int R, int dyw)
+{
+    const int rows = 64 + kCtuWarps * dyw - 1;   // two planes of 8-byte entries
+    return (uint32_t)(ctu_entry(rows - 1, ctu_pitch(R)) + ctu_pitch(R) + 7) / 8 * 128;
+}
+__host__ __device__ __forceinline__ int ctu_plane(int R, int dyw) { return (int)(ctu_win_bytes(R, dyw) >> 4); }
 
 // slot of small key k (0..24) of a lane
 __device__ __forceinline__ int small_slot(int rx, int ry, int half, int k)
@@ -173,25 +182,25 @@ __device__ __forceinline__ int small_slot(int rx, int ry, int half, int k)
     // 16-CU keys 18..24 -> modes (half 0 / half 1)
     const int i = k - 18;
     const int m0[7] = {0, 1, 3, 5, 6, 9, 10};
-    const int m1[7] = {4, 2, 2, 8, 7, 12, 11};
+    const int m1[7] = {4, 2, 3, 8, 7, 12, 11};
     return 576 + (ry * 4 + rx) * 13 + (half ? m1[i] : m0[i]);
 }
 
-// 32-CU key modes per (half, qx, qy) (-1: none); keys A and B
+// 32-CU key modes per (half, qx, qy) (-1: none); keys A and B.  A lane's own
+// pair of regions sums to X1, its outer-half part (top 8 rows or left 8 columns
+// of the pair) to X2, the CU's other pair to X3: A = a X1 + b X2, B = c X1 +
+// d X2 + X3.
 __constant__ int8_t c_m32[2][2][2][2] = {
     // half 0: [qx][qy] -> {A, B}
-    {{{1, 0}, {2, 8}}, {{5, 6}, {7, -1}}},
+    {{{1, 0}, {2, 7}}, {{5, 6}, {8, -1}}},
     // half 1
-    {{{3, 9}, {10, 11}}, {{4, 12}, {-1, -1}}}};
-// coefficients over (X1, X2, X3, X4) for the modes above
-__constant__ int8_t c_c32[2][2][2][2][4] = {
-    {{{{1, 0, 0, 0}, {1, 0, 1, 0}}, {{1, 0, 0, 0}, {1, -1, 0, 0}}},
-     {{{0, 1, 0, 0}, {1, -1, 1, 0}}, {{0, 1, 1, 0}, {0, 0, 0, 0}}}},
-    {{{{1, 0, 0, 0}, {0, 1, 0, 0}}, {{1, -1, 1, 0}, {1, 0, 0, 1}}},
-     {{{1, 0, 0, 0}, {1, -1, 0, 0}}, {{0, 0, 0, 0}, {0, 0, 0, 0}}}}};
-// 64-CU key per lane (lane = ry*8 + rx*2 + half): mode (-1 none) and
-// coefficients over (TOT, P, RS) -- half-0 lanes hold row quantities (RS =
-// sum of a row of regions, P = pair of rows), half-1 lanes the column ones.
+    {{{3, 10}, {9, -1}}, {{4, 11}, {12, -1}}}};
+__constant__ int8_t c_c32[2][2][2][4] = {   // a, b, c, d
+    {{{1, 0, 1, 0}, {1, 0, 0, 1}}, {{0, 1, 1, -1}, {1, -1, 0, 0}}},
+    {{{1, 0, 1, -1}, {0, 1, 0, 0}}, {{1, 0, 0, 1}, {1, -1, 0, 0}}}};
+// 64-CU key per ry*8 + rx*2 + half: mode (-1 none) and
+// coefficients over (TOT, P, RS) -- half-0 entries hold row quantities (RS =
+// sum of a row of regions, P = pair of rows), half-1 entries the column ones.
 __constant__ int8_t c_m64[32] = {0, 3, 1, -1, 5, 4, 6, 11, -1, 9, -1, -1, -1, -1, -1, 12,
                                  2, 10, -1, -1, -1, -1, -1, -1, 7, -1, 8, -1, -1, -1, -1, -1};
 __constant__ int8_t c_c64[32][3] = {
@@ -203,24 +212,23 @@ __constant__ int8_t c_c64[32][3] = {
 // Per-lane constants of the warp layout.
 struct LaneRole {
     int half, rx, ry;
+    int nh;                         // -half
     int pr1, pr2, pr3, pr4, pr5;    // shuffle partners (see below)
-    int c32a[4], c32b[4], c64[3];   // coefficient sets of the 32-CU / 64-CU keys
+    int c32[4], c64[3];             // coefficients of the 32-CU / 64-CU keys
     int bx0, by0;                   // picture position of the half-region
 };
 
 // Folds the costs of one displacement into the lane's keys.  `raw` are the
-// lane's eight 4x4 SADs; `mks` = (mvc << 11) | (row << 8) | dx+R for the
-// small keys, `mkl` = (mvc << 8) | dx+R for the large ones.
+// lane's eight 4x4 SADs; `mks` = (mvc << 11) | (row << 8) | dx+R.
 // LV (a compile-time set of CU sizes, as CtuJob::levels) drops the key
 // updates of the CU sizes a job has no PU of.  BORDER poisons the blocks
-// outside the limits; BJ marks a border job, whose large keys are
-// (cost << 8) | dx+R (poisoned sums need the room).  An interior job keeps its
-// large keys in the small-key form (cost << 11 | row << 8 | dx+R: a 64x64
-// cost plus its MV cost stays below 2^21), with no shifts.
-template <bool BORDER, int LV, bool BJ = BORDER>
-__device__ __forceinline__ void fold_displacement(const LaneRole &LR, uint32_t (&raw)[2][4], uint32_t mks,
-                                                  uint32_t mkl, int dx, bool brow0, bool brow1, const Geometry &g,
-                                                  uint32_t (&ks)[25], uint32_t (&rowl)[3])
+// outside the limits; the poisoned sums of the large PUs are formed unshifted
+// and capped before they become keys (a valid cost, and the cap, plus an MV
+// cost stay below 2^21).
+template <bool BORDER, int LV>
+__device__ __forceinline__ void fold_displacement(const LaneRole &LR, uint32_t (&raw)[2][4], uint32_t mks, int dx,
+                                                  bool brow0, bool brow1, const Geometry &g, uint32_t (&ks)[25],
+                                                  uint32_t (&kl)[3])
 {
     const int half = LR.half;
     if (BORDER) {
@@ -272,16 +280,16 @@ __device__ __forceinline__ void fold_displacement(const LaneRole &LR, uint32_t (
     const uint32_t F = Fh + Fh_o, L = Lh + Lh_o;
     const uint32_t cc = (half ? c3h : c0h) + xs_o;          // col 3 (half 1) / col 0 (half 0)
     if (LV & 2) {
-        ks[18] = addmin(F - (half ? L : 0u), mks, ks[18]);     // 16x16 | 8x16 right
+        ks[18] = addmin(F + L * (uint32_t)LR.nh, mks, ks[18]); // 16x16 | 8x16 right
         ks[19] = addmin(Fh, mks, ks[19]);                      // 16x8 top | bottom
-        ks[20] = addmin(half ? Fh : L, mks, ks[20]);           // 8x16 left | (dup)
+        ks[20] = addmin(L, mks, ks[20]);                       // 8x16 left (both halves)
         ks[21] = addmin(rr_, mks, ks[21]);                     // 16x4 y0 | y12
         ks[22] = addmin(F - rr_, mks, ks[22]);                 // 16x12 y4 | y0
         ks[23] = addmin(cc, mks, ks[23]);                      // 4x16 x0 | x12
         ks[24] = addmin(F - cc, mks, ks[24]);                  // 12x16 x4 | x0
     }
-    // large PUs in the raw domain
-    uint32_t Fr, Tr, Lr;
+    // large PUs: the region's sum and its top (half 0) or left (half 1) part
+    uint32_t Fr = F, a1 = half ? L : Fh;
     if (BORDER) {
         uint32_t fh = 0, lh = 0;
 #pragma unroll
@@ -291,67 +299,44 @@ __device__ __forceinline__ void fold_displacement(const LaneRole &LR, uint32_t (
                 fh += raw[br][c];
                 if (c < 2) lh += raw[br][c];
             }
-        const uint32_t fh_o = __shfl_xor_sync(0xffffffffu, fh, 1);
         const uint32_t lh_o = __shfl_xor_sync(0xffffffffu, lh, 1);
-        Fr = fh + fh_o;
-        Tr = half ? fh_o : fh;
-        Lr = lh + lh_o;
-    } else if (BJ) {
-        Fr = F >> 11;
-        Tr = (half ? Fh_o : Fh) >> 11;
-        Lr = L >> 11;
-    } else {
-        Fr = F;
-        Tr = half ? Fh_o : Fh;
-        Lr = L;
+        Fr = fh + __shfl_xor_sync(0xffffffffu, fh, 1);
+        a1 = half ? lh + lh_o : fh;
     }
     // 32x32 CUs
-    const uint32_t a1 = half ? Lr : Tr;
     const uint32_t F_p = __shfl_xor_sync(0xffffffffu, Fr, LR.pr1);
     const uint32_t a_p = __shfl_xor_sync(0xffffffffu, a1, LR.pr1);
     const uint32_t X1 = Fr + F_p, X2 = a1 + a_p;           // FH, TH  |  FV, LV
     const uint32_t X3 = __shfl_xor_sync(0xffffffffu, X1, LR.pr2);
-    const uint32_t X4 = __shfl_xor_sync(0xffffffffu, X2, LR.pr2);
-    const int va = LR.c32a[0] * (int)X1 + LR.c32a[1] * (int)X2 + LR.c32a[2] * (int)X3 + LR.c32a[3] * (int)X4;
-    const int vb = LR.c32b[0] * (int)X1 + LR.c32b[1] * (int)X2 + LR.c32b[2] * (int)X3 + LR.c32b[3] * (int)X4;
+    const int va = LR.c32[0] * (int)X1 + LR.c32[1] * (int)X2;
+    const int vb = LR.c32[2] * (int)X1 + LR.c32[3] * (int)X2 + (int)X3;
     // 64x64 CU
     const uint32_t RS = X1 + __shfl_xor_sync(0xffffffffu, X1, LR.pr3);     // row | column sums
     const uint32_t P = RS + __shfl_xor_sync(0xffffffffu, RS, LR.pr4);      // row | column pairs
     const uint32_t TOT = P + __shfl_xor_sync(0xffffffffu, P, LR.pr5);
     const int v64 = LR.c64[0] * (int)TOT + LR.c64[1] * (int)P + LR.c64[2] * (int)RS;
-    // without poisoned blocks a 64x64 cost stays below kCapLarge (1,044,480 <
-    // 2,000,000) and a lane without a key has all-zero coefficients
-    if (!BJ) {
-        if (LV & 4) {
-            rowl[0] = addmin((uint32_t)va, mks, rowl[0]);
-            rowl[1] = addmin((uint32_t)vb, mks, rowl[1]);
-        }
-        if (LV & 8) rowl[2] = addmin((uint32_t)v64, mks, rowl[2]);
-        return;
-    }
+    auto key = [](int v) { return BORDER ? min((uint32_t)v, kCapLarge) << 11 : (uint32_t)v; };
     if (LV & 4) {
-        rowl[0] = addmin((BORDER ? min((uint32_t)va, kCapLarge) : (uint32_t)va) << 8, mkl, rowl[0]);
-        rowl[1] = addmin((BORDER ? min((uint32_t)vb, kCapLarge) : (uint32_t)vb) << 8, mkl, rowl[1]);
+        kl[0] = addmin(key(va), mks, kl[0]);
+        kl[1] = addmin(key(vb), mks, kl[1]);
     }
-    if (LV & 8) rowl[2] = addmin((BORDER ? min((uint32_t)v64, kCapLarge) : (uint32_t)v64) << 8, mkl, rowl[2]);
+    if (LV & 8) kl[2] = addmin(key(v64), mks, kl[2]);
 }
 
-// 4x4 SADs of the lane's half-region against window rows wrow0.. at byte
-// offset j (any alignment).
-__device__ __forceinline__ void sad_at(const uint8_t *win, int ww, int wrow0, int rx, int j, const uint32_t (&cw)[8][4],
+// 4x4 SADs of the lane's half-region at the first displacement of an entry:
+// row0 = its first window row, k the entry of its first word
+__device__ __forceinline__ void sad_at(const uint2 *win, int pitch, int row0, int k, const uint32_t (&cw)[8][4],
                                        uint32_t (&raw)[2][4])
 {
-    const int j0 = j & ~3, o = j & 3;
 #pragma unroll
     for (int br = 0; br < 2; br++)
 #pragma unroll
         for (int c = 0; c < 4; c++) raw[br][c] = 0;
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-        const int wr = wrow0 + r;
-        const uint32_t *wp = reinterpret_cast<const uint32_t *>(win + wr * ww + 4 * swz(wr) + 16 * rx + j0);
+        const uint2 *wp = win + ctu_entry(row0 + r, pitch) + k;
 #pragma unroll
-        for (int c = 0; c < 4; c++) raw[r >> 2][c] = sad4_acc(cw[r][c], __funnelshift_r(wp[c], wp[c + 1], 8 * o), raw[r >> 2][c]);
+        for (int c = 0; c < 4; c++) raw[r >> 2][c] = sad4_acc(cw[r][c], wp[c].x, raw[r >> 2][c]);
     }
 }
 
@@ -360,24 +345,17 @@ __device__ __forceinline__ void sad_at(const uint8_t *win, int ww, int wrow0, in
 #define XG_CTU_SAFE_SPLIT 1
 #endif
 
-// window fill with 16-byte loads when the window lies inside the padded plane
-#ifndef XG_CTU_VEC_FILL
-#define XG_CTU_VEC_FILL 1
-#endif
-
 // Window fill by the tensor memory accelerator: where the session has a
 // tensor map over its plane pool (3-D: column, row, plane; box 64 columns x
-// 95 rows) and the window qualifies for the 16-byte fill, one thread issues
+// 95 rows) and the window lies inside the padded plane at 16-byte alignment, one thread issues
 // the window as 64-column boxes into a dense staging area before the CTA
-// computes its MV-cost keys, so the copy overlaps that work.  The search's
-// row layout shifts rows by 1-3 words (the bank spread above), which no
-// 16-byte-aligned TMA destination can hold, so a shared-to-shared pass then
-// places the rows.
+// computes its MV-cost keys, so the copy overlaps that work; a
+// shared-to-shared pass then forms the window's entries.
 #ifndef XG_CTU_TMA
 #define XG_CTU_TMA 1
 #endif
 constexpr int kTmaBoxCols = 64;
-constexpr int kTmaBoxRows = 64 + kDyChunk - 1;
+constexpr int kTmaBoxRows = 64 + kDyChunkMax - 1;
 constexpr int kTmaPieceBytes = (kTmaBoxCols * kTmaBoxRows + 127) / 128 * 128;   // 6144
 constexpr int kWaitLimit = 1 << 20;   // mbarrier polls before a CTA gives up its window
 
@@ -399,7 +377,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// Thread 0 only: the window rows [y, y + 95) of plane z, columns x .. x + 64*np
+// Thread 0 only: rows [y, y + 95) of plane z (a smaller chunk's window is the
+// first of them; rows outside the plane are filled with zeros), columns x .. x + 64*np
 // (x a multiple of 16), as np boxes into stage (128-byte aligned), counted
 // on the barrier at bar.
 __device__ __forceinline__ void tma_window_issue(const void *tmap, uint32_t stage, uint32_t bar, int x, int y, int z,
@@ -418,82 +397,38 @@ __device__ __forceinline__ void tma_window_issue(const void *tmap, uint32_t stag
                      : "memory");
 }
 
-// resident CTAs per SM the register budget is sized for (3: up to 168
-// registers; measured faster than 4 CTAs of 128 registers and than 2)
+// resident CTAs per SM the register budget is sized for (3: 168 registers; 2
+// measured 2 % slower at R = 64)
 #ifndef XG_CTU_MINB
 #define XG_CTU_MINB 3
 #endif
-// the same for the two-row form (2: up to 255 registers)
-#ifndef XG_CTU_PAIR_MINB
-#define XG_CTU_PAIR_MINB 2
-#endif
 
-// Ranges from which the search takes two displacement rows per window pass
-// (see ctu_search): the pair form needs about 240 registers (2 CTAs per SM
-// instead of 3) and measured 8 % faster at R = 64 (3.39 against 3.68 ms per
-// 1080p picture), 9 % slower at R = 16 (0.269 against 0.247 ms), where the
-// per-CTA setup of the 32-row chunk weighs more.
-#ifndef XG_CTU_PAIR_MIN_R
-#define XG_CTU_PAIR_MIN_R 32
-#endif
-
-// Folds the 4 displacements j0 .. j0 + 3 of one search row (SADs s[o]) into
-// the lane's keys.
+// Folds the displacements d0 and d0 + 1 of one search row (SADs s[o], key
+// parts mk) into the lane's keys.
 template <bool BORDER, int LV>
-__device__ __forceinline__ void fold_four(const LaneRole &L, uint32_t (&s)[4][2][4], const uint32_t *mrow, int nd, int j0,
-                                          int R, bool brow0, bool brow1, bool row_safe, const CtuJob &job,
-                                          const Geometry &g, uint32_t (&ks)[25], uint32_t (&rowl)[3])
+__device__ __forceinline__ void fold_group(const LaneRole &L, uint32_t (&s)[2][2][4], uint2 mk, int d0, int R, int dy,
+                                           const CtuJob &job, const Geometry &g, uint32_t (&ks)[25],
+                                           uint32_t (&kl)[3])
 {
-#if XG_CTU_SAFE_SPLIT
+    const uint32_t m[2] = {mk.x, mk.y};
     // in a border job, displacements whose every block stays inside the
     // limits take the interior fold (same keys: nothing to poison)
-    const bool safe = !BORDER || (row_safe && job.x0 + j0 - R >= -kLimitMargin &&
-                                  job.x0 + 64 + j0 + 3 - R <= g.W + kLimitMargin);
-    if (BORDER && !safe) {
+    if (BORDER && !(XG_CTU_SAFE_SPLIT && job.y0 + dy >= -kLimitMargin && job.y0 + 64 + dy <= g.H + kLimitMargin &&
+                    job.x0 + d0 - R >= -kLimitMargin && job.x0 + 65 + d0 - R <= g.W + kLimitMargin)) {
+        const int yb = L.by0 + dy;
+        const bool b0 = yb >= -kLimitMargin && yb + 4 <= g.H + kLimitMargin;
+        const bool b1 = yb + 4 >= -kLimitMargin && yb + 8 <= g.H + kLimitMargin;
 #pragma unroll
-        for (int o = 0; o < 4; o++) {
-            const int dxr = j0 + o;
-            const uint32_t mks = mrow[dxr], mkl = mrow[nd * kDyChunk + dxr];
-            fold_displacement<true, LV, true>(L, s[o], mks, mkl, dxr - R, brow0, brow1, g, ks, rowl);
-        }
+        for (int o = 0; o < 2; o++) fold_displacement<true, LV>(L, s[o], m[o], d0 + o - R, b0, b1, g, ks, kl);
     } else {
 #pragma unroll
-        for (int o = 0; o < 4; o++) {
-            const int dxr = j0 + o;
-            const uint32_t mks = mrow[dxr], mkl = mrow[nd * kDyChunk + dxr];
-            fold_displacement<false, LV, BORDER>(L, s[o], mks, mkl, dxr - R, brow0, brow1, g, ks, rowl);
-        }
-    }
-#else
-    (void)row_safe;
-    (void)job;
-#pragma unroll
-    for (int o = 0; o < 4; o++) {
-        const int dxr = j0 + o;
-        const uint32_t mks = mrow[dxr], mkl = mrow[nd * kDyChunk + dxr];
-        fold_displacement<BORDER, LV>(L, s[o], mks, mkl, dxr - R, brow0, brow1, g, ks, rowl);
-    }
-#endif
-}
-
-// a search row's large-PU minima into the 64-bit (cost, order) keys (cost
-// above the low 8 bits in a border job, above the low 11 in an interior job)
-template <bool BJ>
-__device__ __forceinline__ void merge_rowl(const uint32_t (&rowl)[3], int dy, int R, int nd,
-                                           unsigned long long (&kl)[3])
-{
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const uint32_t cost = rowl[k] >> (BJ ? 8 : 11), dxr = rowl[k] & 0xffu;
-        if (cost >= kCapLarge) continue;
-        const unsigned long long key = ((unsigned long long)cost << 32) | (unsigned)(2 + (dy + R) * nd + (int)dxr);
-        kl[k] = key < kl[k] ? key : kl[k];
+        for (int o = 0; o < 2; o++) fold_displacement<false, LV>(L, s[o], m[o], d0 + o - R, true, true, g, ks, kl);
     }
 }
 
-template <bool BORDER, int LV, bool PAIR>
-__device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, const SessView *__restrict__ views, int R,
-                                           int lambda, int ww, uint8_t *smem)
+template <bool BORDER, int LV>
+__device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw, const SessView *__restrict__ views,
+                                           int R, int lambda, uint8_t *smem)
 {
     const SessView &view = views[job.sess];
     const int32_t *__restrict__ slots = view.slots;
@@ -501,54 +436,46 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, const S
     const uint8_t *const *refs = view.ref0;
     const Geometry g = view.g;
     unsigned long long *__restrict__ keys = view.keys;
-    const int dy0 = -R + chunk * kDyChunk;
-    const int wrows = 64 + kDyChunk - 1;
-    const int nd = 2 * R;
-    // MV-cost keys: small-PU form [kDyChunk][nd], then the large-PU form
-    uint32_t *mvk = reinterpret_cast<uint32_t *>(smem);                 // [2][kDyChunk][nd]
-    uint8_t *win = smem + 2 * sizeof(uint32_t) * kDyChunk * nd;          // [wrows][ww]
+    const int rows = kCtuWarps * dyw;                 // search rows of the chunk
+    const int dy0 = -R + chunk * rows;
+    const int wrows = 64 + rows - 1, pitch = ctu_pitch(R), nd = 2 * R;
+    uint32_t *mvk = reinterpret_cast<uint32_t *>(smem);                      // [rows][nd] MV-cost keys
+    uint2 *win = reinterpret_cast<uint2 *>(smem + ctu_key_bytes(R, dyw));    // the window's entries
+    const int plane = ctu_plane(R, dyw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // reference window: rows y0+dy0 .., columns x0-R .., clamped into the plane
+    // reference window: rows y0+dy0 .., columns x0-R .. (64 + 2R), clamped into the plane
     const uint8_t *ref = refs[job.ref];
     const int wx0 = job.x0 - R, wy0 = job.y0 + dy0;
-    const int rowlen = ww - 4 * kSwzMax - 4;   // bytes of a row that are filled (a multiple of 16)
-    const bool vec_ok = wx0 >= -kPad && wx0 + rowlen <= g.W + kPad && wy0 >= -kPad && wy0 + wrows <= g.H + kPad &&
-                        (g.stride & 15) == 0 &&
-                        ((uintptr_t)(ref + (ptrdiff_t)wy0 * g.stride + wx0) & 15) == 0;
-#if XG_CTU_TMA
+    const bool inside = wx0 >= -kPad && wx0 + 64 + 2 * R <= g.W + kPad && wy0 >= -kPad && wy0 + wrows <= g.H + kPad &&
+                        (g.stride & 15) == 0 && ((uintptr_t)(ref + (ptrdiff_t)wy0 * g.stride + wx0) & 15) == 0;
     // staging area after the window (128-byte aligned when the dynamic shared
-    // memory base is), the barrier after it
-    uint8_t *stage = win + (size_t)wrows * ww;
+    // memory base is), the barrier after it; the launch does not give it
+    // where that would cost a CTA per SM
+    uint8_t *stage = smem + ctu_key_bytes(R, dyw) + ctu_win_bytes(R, dyw);
     const int np = tma_pieces(R);
     const uint32_t stage_s = smem_u32(stage), bar_s = stage_s + (uint32_t)(np * kTmaPieceBytes);
-    int tx = 0, ty = 0, tz = 0;
-    bool use_tma = false;
-    // the launch gave the CTA the staging area (it does not where that would
-    // cost a CTA per SM)
     uint32_t dyn_smem;
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
-    const bool staged = (uint32_t)(stage - smem) + (uint32_t)(np * kTmaPieceBytes) + 16u <= dyn_smem;
-    if (view.tmap != nullptr && staged && vec_ok && (stage_s & 127) == 0) {
+    const bool staged = XG_CTU_TMA && (uint32_t)(stage - smem) + (uint32_t)(np * kTmaPieceBytes) + 16u <= dyn_smem;
+    bool use_tma = false;
+    if (view.tmap != nullptr && staged && inside && (stage_s & 127) == 0) {
         const ptrdiff_t off = (ref + (ptrdiff_t)wy0 * g.stride + wx0) - view.pool;
-        tz = (int)(off / (ptrdiff_t)view.plane_bytes);
+        const int tz = (int)(off / (ptrdiff_t)view.plane_bytes);
         const ptrdiff_t rem = off - (ptrdiff_t)tz * view.plane_bytes;
-        ty = (int)(rem / g.stride);
-        tx = (int)(rem - (ptrdiff_t)ty * g.stride);
+        const int ty = (int)(rem / g.stride);
+        const int tx = (int)(rem - (ptrdiff_t)ty * g.stride);
         use_tma = off >= 0 && (tx & 15) == 0;
+        if (use_tma && tid == 0) tma_window_issue(view.tmap, stage_s, bar_s, tx, ty, tz, np);
     }
-    if (use_tma && tid == 0) tma_window_issue(view.tmap, stage_s, bar_s, tx, ty, tz, np);
     __syncthreads();   // the barrier's initialisation, before any thread polls it
-#endif
 
     // MV cost keys of this chunk's displacements (uniform over the CTU)
-    for (int e = tid; e < kDyChunk * nd; e += kCtuThreads) {
-        const int row = e / nd, dxr = e - row * nd;
-        const int dy = dy0 + row, dx = dxr - R;
-        const uint32_t mvc = (uint32_t)mv_cost_hd(lambda, dx * 4, dy * 4, job.mvp_x, job.mvp_y);
-        mvk[e] = (mvc << 11) | ((uint32_t)(row & (kDyWarp - 1)) << 8) | (uint32_t)dxr;
-        mvk[kDyChunk * nd + e] = (mvc << 8) | (uint32_t)dxr;
-    }
-#if XG_CTU_TMA
+    for (int row = warp; row < rows; row += kCtuWarps)
+        for (int dxr = lane; dxr < nd; dxr += 32) {
+            const uint32_t mvc = (uint32_t)mv_cost_hd(lambda, (dxr - R) * 4, (dy0 + row) * 4, job.mvp_x, job.mvp_y);
+            mvk[row * nd + dxr] = (mvc << 11) | ((uint32_t)(row & (dyw - 1)) << 8) | (uint32_t)dxr;
+        }
+    // the window's entries, a row per warp
     if (use_tma) {
         const bool ok = mbar_wait_bounded(bar_s, 0);
         if (__syncthreads_or(!ok)) {
@@ -558,53 +485,45 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, const S
             mbar_wait_bounded(bar_s, 0);
             return;
         }
-        // staged rows [95][64] per box -> the swizzled window rows; only the
-        // bytes the row layout holds (a multiple of 16, at least 64 + 2R + 8)
-        const int cols = min(np * kTmaBoxCols, rowlen) >> 4;
-        for (int e = tid; e < wrows * cols; e += kCtuThreads) {
-            const int r = e / cols, c = (e - r * cols) << 4;
-            const uint4 v = *reinterpret_cast<const uint4 *>(stage + (c >> 6) * kTmaPieceBytes + r * kTmaBoxCols +
-                                                             (c & (kTmaBoxCols - 1)));
-            uint32_t *d = reinterpret_cast<uint32_t *>(win + r * ww + 4 * swz(r) + c);
-            d[0] = v.x;
-            d[1] = v.y;
-            d[2] = v.z;
-            d[3] = v.w;
+    } else if (staged && !inside) {
+        for (int r = warp; r < wrows; r += kCtuWarps) {
+            const uint8_t *row = ref + (ptrdiff_t)min(max(wy0 + r, -kPad), g.H + kPad - 1) * g.stride;
+            for (int c = lane; c < 64 + 2 * R; c += 32)
+                stage[(c >> 6) * kTmaPieceBytes + r * kTmaBoxCols + (c & (kTmaBoxCols - 1))] =
+                    row[min(max(wx0 + c, -kPad), g.W + kPad - 1)];
         }
-    } else
-#endif
-#if XG_CTU_VEC_FILL
-    if (vec_ok) {
-        // the window lies inside the padded plane and its rows start on
-        // 16-byte boundaries: 16-byte loads, word stores into the swizzled rows
-        const int q = rowlen >> 4;
-        for (int e = tid; e < wrows * q; e += kCtuThreads) {
-            const int r = e / q, c = (e - r * q) << 4;
-            const uint4 v = __ldg(reinterpret_cast<const uint4 *>(ref + (ptrdiff_t)(wy0 + r) * g.stride + wx0 + c));
-            uint32_t *d = reinterpret_cast<uint32_t *>(win + r * ww + 4 * swz(r) + c);
-            d[0] = v.x;
-            d[1] = v.y;
-            d[2] = v.z;
-            d[3] = v.w;
-        }
-    } else
-#endif
-    {
-        for (int e = tid; e < wrows * rowlen; e += kCtuThreads) {
-            const int r = e / rowlen, c = e - r * rowlen;
-            const int y = min(max(wy0 + r, -kPad), g.H + kPad - 1);
-            const int x = min(max(wx0 + c, -kPad), g.W + kPad - 1);
-            win[r * ww + 4 * swz(r) + c] = ref[(ptrdiff_t)y * g.stride + x];
+        __syncthreads();
+    }
+    const bool from_stage = use_tma || (staged && !inside);
+    for (int r = warp; r < wrows; r += kCtuWarps) {
+        const uint8_t *row = ref + (ptrdiff_t)min(max(wy0 + r, -kPad), g.H + kPad - 1) * g.stride;
+        auto word = [&](int k) -> uint32_t {   // samples 4k .. 4k + 3 of the window row
+            if (from_stage)
+                return *reinterpret_cast<const uint32_t *>(stage + (k >> 4) * kTmaPieceBytes + r * kTmaBoxCols +
+                                                           4 * (k & 15));
+            if (inside) return __ldg(reinterpret_cast<const uint32_t *>(row + wx0) + k);
+            uint32_t v = 0;
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                v |= (uint32_t)row[min(max(wx0 + 4 * k + b, -kPad), g.W + kPad - 1)] << (8 * b);
+            return v;
+        };
+        uint2 *d = win + ctu_entry(r, pitch);
+        for (int k = lane; k < pitch; k += 32) {
+            const uint32_t lo = word(k), hi = word(k + 1);
+            d[k] = make_uint2(lo, __byte_perm(lo, hi, 0x4321));
+            d[k + plane] = make_uint2(__byte_perm(lo, hi, 0x5432), __byte_perm(lo, hi, 0x6543));
         }
     }
     __syncthreads();
 
     LaneRole L;
     L.half = lane & 1;
-    L.rx = (lane >> 1) & 3;
-    L.ry = lane >> 3;
+    L.rx = ((lane >> 1) & 1) + 2 * ((lane >> 3) & 1);
+    L.ry = ((lane >> 2) & 1) + 2 * (lane >> 4);
+    L.nh = -L.half;
     const int half = L.half, rx = L.rx, ry = L.ry;
-    const int qx = rx & 1, qy = ry & 1;
+    const int qx = rx & 1, qy = ry & 1, id = ry * 8 + rx * 2 + half;
     // current block: 8 rows x 16 pixels of this half-region
     uint32_t cw[8][4];
     {
@@ -616,180 +535,108 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, const S
         }
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        L.c32a[k] = c_c32[half][qx][qy][0][k];
-        L.c32b[k] = c_c32[half][qx][qy][1][k];
-    }
+    for (int k = 0; k < 4; k++) L.c32[k] = c_c32[half][qx][qy][k];
 #pragma unroll
-    for (int k = 0; k < 3; k++) L.c64[k] = c_c64[lane][k];
-    const int m32a = c_m32[half][qx][qy][0], m32b = c_m32[half][qx][qy][1], m64 = c_m64[lane];
-    // shuffle partners: region pairs along the axis this half works on
-    L.pr1 = half ? 8 : 2;     // 32-CU pair (vertical for half 1, horizontal for half 0)
-    L.pr2 = half ? 2 : 8;     // the other 32-CU row/column
-    L.pr3 = half ? 16 : 4;    // 64-CU row / column sums
-    L.pr4 = half ? 2 : 8;     // 64-CU pairs
-    L.pr5 = half ? 4 : 16;    // 64-CU total
+    for (int k = 0; k < 3; k++) L.c64[k] = c_c64[id][k];
+    // shuffle partners: region pairs along the axis this half works on (lane
+    // bits: 1 rx0, 2 ry0, 3 rx1, 4 ry1)
+    L.pr1 = half ? 4 : 2;     // 32-CU pair (vertical for half 1, horizontal for half 0)
+    L.pr2 = half ? 2 : 4;     // the other 32-CU row/column
+    L.pr3 = half ? 16 : 8;    // 64-CU row / column sums
+    L.pr4 = half ? 2 : 4;     // 64-CU pairs
+    L.pr5 = half ? 8 : 16;    // 64-CU total
     L.bx0 = job.x0 + 16 * rx;
     L.by0 = job.y0 + 16 * ry + 8 * half;
     const int32_t *smap = slots + (size_t)job.slot_base;
     const int cu32 = (ry >> 1) * 2 + (rx >> 1);
-    const int lm[3] = {m32a, m32b, m64};
+    const int lm[3] = {c_m32[half][qx][qy][0], c_m32[half][qx][qy][1], c_m64[id]};
+
+    uint32_t ks[25], kl[3];
+    auto clear = [&]() {
+#pragma unroll
+        for (int k = 0; k < 25; k++) ks[k] = 0xffffffffu;
+#pragma unroll
+        for (int k = 0; k < 3; k++) kl[k] = 0xffffffffu;
+    };
+    // the warp's minima into the global keys; order(row, dxr) is the visit order
+    auto merge = [&](auto order) {
+#pragma unroll
+        for (int k = 0; k < 25; k++) {
+            const uint32_t cost = ks[k] >> 11;
+            if (cost >= kPoisonSmall) continue;
+            const int pu = smap[small_slot(rx, ry, half, k)];
+            if (pu >= 0)
+                atomicMin(&keys[pu], ((unsigned long long)cost << 32) | order((ks[k] >> 8) & 7u, ks[k] & 0xffu));
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const uint32_t cost = kl[k] >> 11;
+            if (lm[k] < 0 || cost >= kCapLarge) continue;
+            const int pu = smap[k < 2 ? 784 + cu32 * 13 + lm[k] : 836 + lm[k]];
+            if (pu >= 0)
+                atomicMin(&keys[pu], ((unsigned long long)cost << 32) | order((kl[k] >> 8) & 7u, kl[k] & 0xffu));
+        }
+    };
+    clear();
+    const int q8 = 16 * ry + 8 * half;   // the half-region's first row
 
     // The search candidate (0,0) is visited before the window (me.c:913-917):
     // its cost enters with visit order 0, so it wins every tie.  The CTA whose
     // rows contain dy = 0 evaluates it (warp 0).
-    if (warp == 0 && dy0 <= 0 && 0 < dy0 + kDyChunk) {
-        uint32_t ks0[25], rowl0[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-#pragma unroll
-        for (int k = 0; k < 25; k++) ks0[k] = 0xffffffffu;
+    if (warp == 0 && dy0 <= 0 && 0 < dy0 + rows) {
         uint32_t raw[2][4];
-        sad_at(win, ww, 16 * ry + 8 * half - dy0, rx, R, cw, raw);
+        sad_at(win + ((R >> 1) & 1) * plane, pitch, q8 - dy0, 4 * rx + (R >> 2), cw, raw);   // R is even
         const uint32_t mvc0 = (uint32_t)mv_cost_hd(lambda, 0, 0, job.mvp_x, job.mvp_y);
         bool b0 = true, b1 = true;
         if (BORDER) {
             b0 = L.by0 >= -kLimitMargin && L.by0 + 4 <= g.H + kLimitMargin;
             b1 = L.by0 + 4 >= -kLimitMargin && L.by0 + 8 <= g.H + kLimitMargin;
         }
-        fold_displacement<BORDER, LV>(L, raw, mvc0 << 11, mvc0 << 8, 0, b0, b1, g, ks0, rowl0);
-#pragma unroll
-        for (int k = 0; k < 25; k++) {
-            const uint32_t cost = ks0[k] >> 11;
-            if (cost >= kPoisonSmall) continue;
-            const int pu = smap[small_slot(rx, ry, half, k)];
-            if (pu >= 0) atomicMin(&keys[pu], (unsigned long long)cost << 32);
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const uint32_t cost = rowl0[k] >> (BORDER ? 8 : 11);
-            if (lm[k] < 0 || cost >= kCapLarge) continue;
-            const int pu = smap[k < 2 ? 784 + cu32 * 13 + lm[k] : 836 + lm[k]];
-            if (pu >= 0) atomicMin(&keys[pu], (unsigned long long)cost << 32);
-        }
+        fold_displacement<BORDER, LV>(L, raw, mvc0 << 11, 0, b0, b1, g, ks, kl);
+        merge([](uint32_t, uint32_t) { return 0u; });
+        clear();
     }
 
-    uint32_t ks[25];
-    unsigned long long kl[3] = {~0ull, ~0ull, ~0ull};
-#pragma unroll
-    for (int k = 0; k < 25; k++) ks[k] = 0xffffffffu;
-
-    if constexpr (PAIR) {
-    // two displacement rows per pass: window rows wrow0 .. wrow0 + 8 are
-    // loaded and aligned once; row r serves block row r of the first
-    // displacement row and block row r - 1 of the second
-    for (int rr = 0; rr < kDyWarp; rr += 2) {
-        const int row = warp * kDyWarp + rr;
+    // two displacement rows per pass: window rows q8 + row .. + 8 are read
+    // once; row r serves block row r of the first displacement row and block
+    // row r - 1 of the second
+    const int dyw0 = dy0 + warp * dyw;
+    for (int rr = 0; rr < dyw; rr += 2) {
+        const int row = warp * dyw + rr;
         const int dy = dy0 + row;
-        if (dy >= R) break;     // 2R and kDyWarp are even: a pair is all in or all out
-        const int wrow0 = 16 * ry + 8 * half + row;
-        const uint32_t *mrowA = mvk + row * nd, *mrowB = mrowA + nd;
-        uint32_t rowlA[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, rowlB[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-        bool bA0 = true, bA1 = true, bB0 = true, bB1 = true;
-        if (BORDER) {
-            const int yb = L.by0 + dy;
-            bA0 = yb >= -kLimitMargin && yb + 4 <= g.H + kLimitMargin;
-            bA1 = yb + 4 >= -kLimitMargin && yb + 8 <= g.H + kLimitMargin;
-            bB0 = yb + 1 >= -kLimitMargin && yb + 5 <= g.H + kLimitMargin;
-            bB1 = yb + 5 >= -kLimitMargin && yb + 9 <= g.H + kLimitMargin;
-        }
-        const bool safeA = job.y0 + dy >= -kLimitMargin && job.y0 + 64 + dy <= g.H + kLimitMargin;
-        const bool safeB = job.y0 + dy + 1 >= -kLimitMargin && job.y0 + 65 + dy <= g.H + kLimitMargin;
-        for (int j0 = 0; j0 < nd; j0 += 4) {
-            uint32_t sA[4][2][4], sB[4][2][4];
+        if (dy >= R) break;     // 2R and dyw are even: a pair is all in or all out
+        uint32_t rp[9];   // the window rows' shared-memory addresses
 #pragma unroll
-            for (int o = 0; o < 4; o++)
+        for (int r = 0; r < 9; r++) rp[r] = smem_u32(win + ctu_entry(q8 + row + r, pitch) + 4 * rx);
+        const uint2 *mk = reinterpret_cast<const uint2 *>(mvk + row * nd);
+#pragma unroll 1
+        for (uint32_t j = 0, step = 8u * plane; j < (uint32_t)R; j++) {   // displacements 2j and 2j + 1
+            uint32_t s[2][2][2][4];     // [displacement row][displacement][block row][block column]
 #pragma unroll
-                for (int br = 0; br < 2; br++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) sA[o][br][c] = sB[o][br][c] = 0;
+            for (int k = 0; k < 32; k++) s[k >> 4][(k >> 3) & 1][(k >> 2) & 1][k & 3] = 0;
 #pragma unroll
             for (int r = 0; r < 9; r++) {
-                const int wr = wrow0 + r;
-                const uint32_t *wp = reinterpret_cast<const uint32_t *>(win + wr * ww + 4 * swz(wr) + 16 * rx + j0);
-                uint32_t w5[5];
 #pragma unroll
-                for (int k = 0; k < 5; k++) w5[k] = wp[k];
+                for (int c = 0; c < 4; c++) {
+                    uint2 v;
+                    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(rp[r] + 8 * c));
 #pragma unroll
-                for (int o = 0; o < 4; o++) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const uint32_t a = o ? align_bytes(w5[c], w5[c + 1], o) : w5[c];
-                        if (r < 8) sA[o][r >> 2][c] = sad4_acc(cw[r][c], a, sA[o][r >> 2][c]);
-                        if (r >= 1) sB[o][(r - 1) >> 2][c] = sad4_acc(cw[r - 1][c], a, sB[o][(r - 1) >> 2][c]);
+                    for (int i = 0; i < 2; i++) {
+                        const int b = r - i;
+                        if (b < 0 || b > 7) continue;
+                        s[i][0][b >> 2][c] = sad4_acc(cw[b][c], v.x, s[i][0][b >> 2][c]);
+                        s[i][1][b >> 2][c] = sad4_acc(cw[b][c], v.y, s[i][1][b >> 2][c]);
                     }
                 }
+                rp[r] += step;
             }
-            fold_four<BORDER, LV>(L, sA, mrowA, nd, j0, R, bA0, bA1, safeA, job, g, ks, rowlA);
-            fold_four<BORDER, LV>(L, sB, mrowB, nd, j0, R, bB0, bB1, safeB, job, g, ks, rowlB);
+            step = 8u - step;   // to the other plane and back one entry further
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                fold_group<BORDER, LV>(L, s[i], mk[i * R + j], 2 * j, R, dy + i, job, g, ks, kl);
         }
-        merge_rowl<BORDER>(rowlA, dy, R, nd, kl);
-        merge_rowl<BORDER>(rowlB, dy + 1, R, nd, kl);
     }
-    } else {
-    for (int rr = 0; rr < kDyWarp; rr++) {
-        const int row = warp * kDyWarp + rr;
-        const int dy = dy0 + row;
-        if (dy >= R) break;
-        const int wrow0 = 16 * ry + 8 * half + row;
-        const uint32_t *mrow = mvk + row * nd;
-        uint32_t rowl[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-        bool brow0 = true, brow1 = true;
-        if (BORDER) {
-            const int yb = L.by0 + dy;
-            brow0 = yb >= -kLimitMargin && yb + 4 <= g.H + kLimitMargin;
-            brow1 = yb + 4 >= -kLimitMargin && yb + 8 <= g.H + kLimitMargin;
-        }
-        // every block of the CTU inside the vertical limits at this dy
-        const bool row_safe = job.y0 + dy >= -kLimitMargin && job.y0 + 64 + dy <= g.H + kLimitMargin;
-        for (int j0 = 0; j0 < nd; j0 += 4) {
-            uint32_t s[4][2][4];
-#pragma unroll
-            for (int o = 0; o < 4; o++)
-#pragma unroll
-                for (int br = 0; br < 2; br++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) s[o][br][c] = 0;
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const int wr = wrow0 + r;
-                const uint32_t *wp = reinterpret_cast<const uint32_t *>(win + wr * ww + 4 * swz(wr) + 16 * rx + j0);
-                uint32_t w5[5];
-#pragma unroll
-                for (int k = 0; k < 5; k++) w5[k] = wp[k];
-#pragma unroll
-                for (int o = 0; o < 4; o++) {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        // the 4 bytes at byte offset o: a byte permute with a
-                        // constant selector (4321, 5432, 6543)
-                        const uint32_t a = o ? align_bytes(w5[c], w5[c + 1], o) : w5[c];
-                        s[o][r >> 2][c] = sad4_acc(cw[r][c], a, s[o][r >> 2][c]);
-                    }
-                }
-            }
-            fold_four<BORDER, LV>(L, s, mrow, nd, j0, R, brow0, brow1, row_safe, job, g, ks, rowl);
-        }
-        merge_rowl<BORDER>(rowl, dy, R, nd, kl);
-    }
-    }
-    // merge into the global keys
-    const int dyw = dy0 + warp * kDyWarp;
-#pragma unroll
-    for (int k = 0; k < 25; k++) {
-        const uint32_t key = ks[k];
-        const uint32_t cost = key >> 11;
-        if (cost >= kPoisonSmall) continue;
-        const int pu = smap[small_slot(rx, ry, half, k)];
-        if (pu < 0) continue;
-        const int dy = dyw + (int)((key >> 8) & 7), dxr = (int)(key & 0xffu);
-        atomicMin(&keys[pu], ((unsigned long long)cost << 32) | (unsigned)(2 + (dy + R) * nd + dxr));
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        if (lm[k] < 0 || kl[k] == ~0ull) continue;
-        const int slot = k < 2 ? 784 + cu32 * 13 + lm[k] : 836 + lm[k];
-        const int pu = smap[slot];
-        if (pu >= 0) atomicMin(&keys[pu], kl[k]);
-    }
+    merge([&](uint32_t row, uint32_t dxr) { return (uint32_t)(2 + (dyw0 + (int)row + R) * nd + (int)dxr); });
 }
 
 // CU sizes with separate compiled folds (serving's leaf CUs often have no
@@ -798,21 +645,21 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, const S
 #define XG_CTU_LEVELS 1
 #endif
 
-template <bool BORDER, bool PAIR>
-__global__ void __launch_bounds__(kCtuThreads, PAIR ? XG_CTU_PAIR_MINB : XG_CTU_MINB)
-    fs_ctu_kernel(const CtuJob *__restrict__ jobs, int nchunks, const SessView *__restrict__ views, int R, int lambda,
-                  int ww)
+template <bool BORDER>
+__global__ void __launch_bounds__(kCtuThreads, XG_CTU_MINB)
+    fs_ctu_kernel(const CtuJob *__restrict__ jobs, int nchunks, int dyw, const SessView *__restrict__ views, int R,
+                  int lambda)
 {
     extern __shared__ __align__(16) uint8_t smem[];
     const int job_idx = blockIdx.x / nchunks, chunk = blockIdx.x % nchunks;
     const CtuJob job = jobs[job_idx];
     if (BORDER != (job.border != 0)) return;
 #if XG_CTU_LEVELS
-    if (job.levels & 1) ctu_search<BORDER, 15, PAIR>(job, chunk, views, R, lambda, ww, smem);
-    else if (job.levels & 2) ctu_search<BORDER, 14, PAIR>(job, chunk, views, R, lambda, ww, smem);
-    else ctu_search<BORDER, 12, PAIR>(job, chunk, views, R, lambda, ww, smem);
+    if (job.levels & 1) ctu_search<BORDER, 15>(job, chunk, dyw, views, R, lambda, smem);
+    else if (job.levels & 2) ctu_search<BORDER, 14>(job, chunk, dyw, views, R, lambda, smem);
+    else ctu_search<BORDER, 12>(job, chunk, dyw, views, R, lambda, smem);
 #else
-    ctu_search<BORDER, 15, PAIR>(job, chunk, views, R, lambda, ww, smem);
+    ctu_search<BORDER, 15>(job, chunk, dyw, views, R, lambda, smem);
 #endif
 }
 
@@ -898,14 +745,11 @@ static void ctu_plan_build(CtuPlan &p, const std::vector<xavs2gpu_pu_t> &pus, in
     }
 }
 
-// ww: row pitch of the window (bytes), a multiple of 128 that holds the
-// 64 + 2R + 8 bytes a row needs after its swizzle shift.
-static inline size_t ctu_smem_bytes(int R, int &ww, bool staging)
+constexpr int kCtuSmemMax = 227 * 1024;
+static inline size_t ctu_smem_bytes(int R, int dyw, bool staging)
 {
-    ww = (int)align_up((size_t)64 + 2 * R + 8 + 4 * kSwzMax + 4, 128);
-    const size_t keys_win = 2 * sizeof(uint32_t) * kDyChunk * 2 * R + (size_t)(64 + kDyChunk - 1) * ww;
-    // the TMA staging boxes and their barrier
-    return staging ? keys_win + (size_t)tma_pieces(R) * kTmaPieceBytes + 16 : keys_win;
+    const size_t b = (size_t)ctu_key_bytes(R, dyw) + ctu_win_bytes(R, dyw);
+    return staging ? b + (size_t)tma_pieces(R) * kTmaPieceBytes + 16 : b;   // the boxes and their barrier
 }
 
 // The kernels' dynamic shared-memory limit (the largest range's need), once
@@ -914,45 +758,71 @@ static void ctu_attrs(int dev)
 {
     static std::atomic<bool> done[64];
     if (dev < 0 || dev >= 64 || done[dev].load(std::memory_order_acquire)) return;
-    int ww_max;
-    const int maxb = (int)ctu_smem_bytes(128, ww_max, XG_CTU_TMA != 0);
-    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
-    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
-    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
-    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+    const int maxb = kCtuSmemMax;
+    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
+    XG_CUDA(cudaFuncSetAttribute(fs_ctu_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxb));
     done[dev].store(true, std::memory_order_release);
 }
 
-// Dynamic shared memory of a launch of variant (border, pair) at range R:
-// with the TMA staging area where it costs no CTA per SM (it would from
-// R = 96 on in the two-row form), else without (the CTAs then fill their
-// windows with 16-byte loads).  Cached per device, variant and range.
-template <bool BORDER, bool PAIR>
-static size_t ctu_launch_smem(int dev, int R, int &ww)
+// What a launch at range R with dyw search rows per warp runs with: its
+// dynamic shared memory (the TMA staging area included where it costs no CTA
+// per SM; the CTAs fill their windows with word loads without it) and the
+// CTAs an SM holds.  Kept per device and range.
+struct CtuFit {
+    int smem = 0, ctas = 0;
+};
+static CtuFit ctu_fit(int dev, int R, int dyw)
 {
-    static std::atomic<int> choice[64][129];   // 0 unknown, 1 without, 2 with (threads agree)
-    const size_t base = ctu_smem_bytes(R, ww, false);
-#if XG_CTU_TMA
-    if (dev < 0 || dev >= 64 || R < 1 || R > 128) return base;
-    std::atomic<int> &slot = choice[dev][R];
-    int c = slot.load(std::memory_order_relaxed);
-    if (c == 0) {
-        ctu_attrs(dev);
-        int wwt, nb = 0, nt = 0;
-        const size_t with = ctu_smem_bytes(R, wwt, true);
-        const bool ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fs_ctu_kernel<BORDER, PAIR>, kCtuThreads,
-                                                                      base) == cudaSuccess &&
-                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nt, fs_ctu_kernel<BORDER, PAIR>, kCtuThreads,
-                                                                      with) == cudaSuccess;
-        if (!ok) cudaGetLastError();
-        c = ok && nb > 0 && nt >= nb ? 2 : 1;
-        slot.store(c, std::memory_order_relaxed);
+    static std::atomic<int> known[64][129][3];   // smem << 4 | ctas (threads agree)
+    const int with = (int)ctu_smem_bytes(R, dyw, true), base = (int)ctu_smem_bytes(R, dyw, false);
+    CtuFit f;
+    const bool keep = dev >= 0 && dev < 64 && R >= 1 && R <= 128;
+    std::atomic<int> *slot = keep ? &known[dev][R][dyw == 8 ? 2 : dyw == 4 ? 1 : 0] : nullptr;
+    const int v = slot ? slot->load(std::memory_order_relaxed) : 0;
+    if (v) {
+        f.smem = v >> 4;
+        f.ctas = v & 15;
+        return f;
     }
-    return c == 2 ? ctu_smem_bytes(R, ww, true) : base;
-#else
-    (void)dev;
-    return base;
+    ctu_attrs(dev);
+    auto resident = [](int bytes) {
+        int a = 0, b = 0;
+        if (bytes > kCtuSmemMax) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, fs_ctu_kernel<false>, kCtuThreads, bytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fs_ctu_kernel<true>, kCtuThreads, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return std::min(std::min(a, b), 15);
+    };
+    const int n0 = resident(base), n1 = XG_CTU_TMA ? resident(with) : 0;
+    f.smem = n1 > 0 && n1 >= n0 ? with : base;
+    f.ctas = std::max(n0, n1);
+    if (slot) slot->store(f.smem << 4 | f.ctas, std::memory_order_relaxed);
+    return f;
+}
+
+// Search rows per warp: 8, 4 or 2 (a CTA's chunk is four times that).  More
+// rows share a window and a final merge; fewer make a smaller window, which
+// lets an SM hold more CTAs (R = 64: 2 at 8 rows, 3 at 4; R = 128: 1, 2 at 2),
+// and more CTAs.  So: the most rows at which an SM holds the most CTAs, halved while
+// the launch is below two rounds of the GPU.  Measured, one reference, us at 8 /
+// 4 / 2 rows: 1080p R = 64 1558 / 1422 / 1473, R = 32 372 / 380 / 399, R = 16
+// 125 / 118 / 138; 720p R = 16 104 / 85 / 82; 416x240 R = 16 51 / 34 / 26,
+// R = 64 223 / 165 / 123; 1080p R = 128 7649 / 7845 / 6241.
+#ifndef XG_CTU_DYW
+#define XG_CTU_DYW 0   // 0: by the rule
 #endif
+static int ctu_rows(int dev, int R, int n_jobs)
+{
+    if (XG_CTU_DYW) return XG_CTU_DYW;
+    int dyw = kDyWarpMax;
+    for (int d = dyw / 2; d >= 2; d /= 2)
+        if (ctu_fit(dev, R, d).ctas > ctu_fit(dev, R, dyw).ctas) dyw = d;
+    const long long slots = (long long)sm_count() * ctu_fit(dev, R, dyw).ctas;
+    auto chunks = [&](int d) { return (2 * R + kCtuWarps * d - 1) / (kCtuWarps * d); };
+    while (dyw > 2 && (long long)n_jobs * chunks(dyw) < 2 * slots) dyw /= 2;
+    return dyw;
 }
 
 // Run the border variant on a side stream forked from the caller's, so its
@@ -997,19 +867,12 @@ static CtuSide *ctu_side(int dev, int k = 0)   // k: 0 the search's own, 1 the p
 static void ctu_prime(int R)
 {
     const int dev = current_device();
-    int ww;
     if (XG_CTU_FORK) {
         ctu_side(dev, 0);
         ctu_side(dev, 1);
     }
     if (R < 1 || R > 128) return;
-    if (R >= XG_CTU_PAIR_MIN_R) {
-        ctu_launch_smem<false, true>(dev, R, ww);
-        ctu_launch_smem<true, true>(dev, R, ww);
-    } else {
-        ctu_launch_smem<false, false>(dev, R, ww);
-        ctu_launch_smem<true, false>(dev, R, ww);
-    }
+    for (int dyw = 2; dyw <= kDyWarpMax; dyw *= 2) ctu_fit(dev, R, dyw);
 }
 
 // One launch of each variant over `n_jobs` jobs (sessions per job.sess).
@@ -1020,12 +883,12 @@ static void ctu_jobs_run(const CtuJob *d_jobs, int n_jobs, int n_border, const S
 {
     if (n_jobs == 0) return;
     const int R = prm.search_range;
-    int ww;
     const int dev = current_device();
     ctu_attrs(dev);
-    const int nchunks = (2 * R + kDyChunk - 1) / kDyChunk;
+    const int dyw = ctu_rows(dev, R, n_jobs), rows = kCtuWarps * dyw;
+    const size_t smem = (size_t)ctu_fit(dev, R, dyw).smem;
+    const int nchunks = (2 * R + rows - 1) / rows;
     const int grid = n_jobs * nchunks;
-    const bool pair = R >= XG_CTU_PAIR_MIN_R;
     const int lam = prm.lambda_factor;
     // the border launch on the side stream when both variants run
     CtuSide *side = XG_CTU_FORK && n_border > 0 && n_border < n_jobs ? ctu_side(dev) : nullptr;
@@ -1036,23 +899,11 @@ static void ctu_jobs_run(const CtuJob *d_jobs, int n_jobs, int n_border, const S
         bst = side->st;
     }
     if (n_border < n_jobs) {
-        if (pair) {
-            const size_t smem = ctu_launch_smem<false, true>(dev, R, ww);
-            fs_ctu_kernel<false, true><<<grid, kCtuThreads, smem, st>>>(d_jobs, nchunks, d_views, R, lam, ww);
-        } else {
-            const size_t smem = ctu_launch_smem<false, false>(dev, R, ww);
-            fs_ctu_kernel<false, false><<<grid, kCtuThreads, smem, st>>>(d_jobs, nchunks, d_views, R, lam, ww);
-        }
+        fs_ctu_kernel<false><<<grid, kCtuThreads, smem, st>>>(d_jobs, nchunks, dyw, d_views, R, lam);
         count_launch();
     }
     if (n_border > 0) {
-        if (pair) {
-            const size_t smem = ctu_launch_smem<true, true>(dev, R, ww);
-            fs_ctu_kernel<true, true><<<grid, kCtuThreads, smem, bst>>>(d_jobs, nchunks, d_views, R, lam, ww);
-        } else {
-            const size_t smem = ctu_launch_smem<true, false>(dev, R, ww);
-            fs_ctu_kernel<true, false><<<grid, kCtuThreads, smem, bst>>>(d_jobs, nchunks, d_views, R, lam, ww);
-        }
+        fs_ctu_kernel<true><<<grid, kCtuThreads, smem, bst>>>(d_jobs, nchunks, dyw, d_views, R, lam);
         count_launch();
     }
     if (side) {
