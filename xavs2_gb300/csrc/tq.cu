@@ -150,19 +150,22 @@ __device__ __forceinline__ void fold_line(const uint32_t (&xp)[N / 2], uint32_t 
 {
 #if XG_TQ_PACKED_FOLD
     // on the packed pairs: (x[2m], x[2m+1]) +- (x[N-1-2m], x[N-2-2m]), the
-    // second the half-swapped pair N/2-1-m; a 16-bit sum is exact iff the
-    // wrapping and the saturating forms agree (the wrapped value of an
-    // overflowing sum of two int16 is never the saturation bound)
+    // second the half-swapped pair N/2-1-m.  A 16-bit sum a + b overflows iff
+    // its sign is neither's and a - b iff the signs differ and the result's is
+    // not a's, so with t = a ^ b both are the sign of a ^ (t ? a - b : a + b):
+    // three logic instructions per pair (the saturating packed forms to
+    // compare with take five instructions each)
     uint32_t ov = 0;
 #pragma unroll
     for (int m = 0; m < N / 4; m++) {
         const uint32_t a = xp[m], b = __byte_perm(xp[N / 2 - 1 - m], 0, 0x1032);
         const uint32_t e = __vadd2(a, b), o = __vsub2(a, b);
-        ov |= (e ^ __vaddss2(a, b)) | (o ^ __vsubss2(a, b));
+        const uint32_t t = a ^ b;
+        ov |= a ^ ((t & o) | (~t & e));
         ep[m] = e;
         op[m] = o;
     }
-    bad |= ov != 0;
+    bad |= (ov & 0x80008000u) != 0;
 #else
     int x[N];
 #pragma unroll
@@ -293,9 +296,12 @@ __device__ __noinline__ void tu_group(const Ctx &cx, int idx, int lane, uint8_t 
     xavs2gpu_tq_block_t b{};
     if (act) b = cx.blocks[idx];
     const bool sec = PART == 0 && (b.flags & 2);
-    static_assert(S::WAV ? RA == kRegionA : RA / 2 / S::G >= 2 * TW * (TH + 2) + TW * TH,
-                  "region A holds the transposes and the staging of every TU of the group");
-    int16_t *tA = reinterpret_cast<int16_t *>(smem) + sub * (RA / 2 / S::G);
+    // A TU's part of region A holds its two transposes and its staged output; a
+    // stride of L words modulo 32 banks puts the rows of the group's TUs on
+    // different banks
+    constexpr int kNeed = (TW * P1 + 2 * TH * P2) / 2, kSub = (kNeed + 31 - L) / 32 * 32 + L;   // words
+    static_assert(S::WAV ? RA == kRegionA : (S::G == 1 ? kNeed : S::G * kSub) * 4 <= RA, "region A holds the group");
+    int16_t *tA = reinterpret_cast<int16_t *>(smem) + sub * 2 * kSub;
     int16_t *tB = reinterpret_cast<int16_t *>(smem + kRegionA);
     const int16_t *src = cx.residual + b.offset;
     const bool al_in = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
@@ -523,9 +529,10 @@ __device__ __noinline__ void tu_group(const Ctx &cx, int idx, int lane, uint8_t 
     __syncwarp();
 
     // ---- inverse rows: lane l < TH; rows staged after T2 (or, for the
-    // wavelet shapes, into region B for the upsampling)
+    // wavelet shapes, into region B for the upsampling) at T2's pitch, which
+    // spreads them over the banks
     int16_t *stage = S::WAV ? tB : t2 + TH * P2;
-    constexpr int PS = S::WAV ? TW + 2 : TW;
+    constexpr int PS = P2;
     if (inv && l < TH) {
         uint32_t vp[TW / 2];
         load_pairs<TW>(t2 + l * P2, vp);
@@ -544,12 +551,13 @@ __device__ __noinline__ void tu_group(const Ctx &cx, int idx, int lane, uint8_t 
     if constexpr (!S::WAV) {
         if (inv) {
             if (al_out) {
-                for (int i = l; i < TW * TH / 8; i += L) {
-                    const uint32_t *w = reinterpret_cast<const uint32_t *>(stage + 8 * i);
-                    reinterpret_cast<uint4 *>(dst)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+                for (int i = l; i < TW * TH / 8; i += L) {   // 8 samples: part of a row, or two rows of 4
+                    const uint32_t *w = reinterpret_cast<const uint32_t *>(stage + 8 * i / TW * PS + 8 * i % TW);
+                    constexpr int h = TW >= 8 ? 2 : PS / 2;
+                    reinterpret_cast<uint4 *>(dst)[i] = make_uint4(w[0], w[1], w[h], w[h + 1]);
                 }
             } else {
-                for (int i = l; i < TW * TH; i += L) dst[i] = stage[i];
+                for (int i = l; i < TW * TH; i += L) dst[i] = stage[i / TW * PS + i % TW];
             }
         }
     } else {
@@ -1005,8 +1013,8 @@ __global__ void __launch_bounds__(32 * kTuWarps, MINB) tq_direct_kernel(Ctx cx, 
 }  // namespace tqw
 
 // Region A of the non-wavelet classes: the 32x32 TU's two transposes and its
-// staging (2 x 32 x 34 + 32 x 32 int16).
-constexpr int kRegionSmall = 6400;
+// staging (3 x 32 x 34 int16).
+constexpr int kRegionSmall = 6528;
 
 // Build option: 1 runs the wavelet classes and the others as two launches,
 // the latter with 6.4 KB of shared memory per warp and a register budget for
