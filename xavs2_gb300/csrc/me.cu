@@ -778,10 +778,10 @@ __device__ __forceinline__ void refine_stage_thread(bool had, bool u4, int nux, 
 }
 
 // resident CTAs per SM the register budget of the per-thread refinement is
-// sized for (4: 128 registers, measured slightly faster than the
-// compiler's 168-register choice)
+// sized for (5: 96 registers; serving mix 17.0 ms at 4, 16.8 at 5 and 6, 17.15
+// at 3; 1080p R = 64 search 3.90 ms at 4 and 5, 3.98 at 6)
 #ifndef XG_REFINE_MINB
-#define XG_REFINE_MINB 4
+#define XG_REFINE_MINB 5
 #endif
 
 // HAD: SATD (1) or SAD (0) unit costs, fixed per launch so that each
@@ -1019,66 +1019,47 @@ constexpr int kGrpU4 = 16;    // 4x4 units of a 16x16 CU (the only size with 4- 
 struct GroupSmem {
     int t8[kGrpU8][kGrpMaxPos];
     int t4[kGrpU4][kGrpMaxPos];
-    int16_t rx[32], ry[32], rw[32], rh[32];
-    int8_t ru4[32];
+    uint32_t mask[32][kGrpU8 / 32];           // a member's units: bit u of the CU's units of its type
+    uint8_t list[kGrpU8];                     // the covered units
     int offx[kGrpMaxPos], offy[kGrpMaxPos];   // the stage's positions relative to the centre
 };
 
 // floor(q / d) for q < 4096, d <= 16, with m = ceil(65536 / d)
 __device__ __forceinline__ int div_small(int q, int m) { return (q * m) >> 16; }
 
-// is unit (x, y, type u4) of the CU inside a member of `grp`?
-__device__ __forceinline__ bool unit_covered(const GroupSmem &S, unsigned grp, int x, int y, int u4)
-{
-    while (grp) {
-        const int m = __ffs(grp) - 1;
-        grp &= grp - 1;
-        if (S.ru4[m] == u4 && x >= S.rx[m] && x < S.rx[m] + S.rw[m] && y >= S.ry[m] && y < S.ry[m] + S.rh[m])
-            return true;
-    }
-    return false;
-}
-
-// Costs of the covered units of one type at the P positions (qpel, absolute)
-// ccx + offx[k], ccy + offy[k].
+// Costs of the units of one type that the members `grp` cover at the P
+// positions (qpel, absolute) ccx + offx[k], ccy + offy[k], into T.  The covered
+// units are listed first; a lane then takes a unit and all positions (its
+// current block loaded once) or, where that leaves more lanes idle, a unit and
+// a position.  Loading the block weighs about a quarter of a position.
 template <bool U4>
 __device__ __forceinline__ void group_table(GroupSmem &S, unsigned grp, bool had, int cs, const uint8_t *o,
                                             const uint8_t *const *planes, int stride, int px, int py, int ccx,
                                             int ccy, int P, int lane)
 {
-    constexpr int UW = U4 ? 4 : 8;
+    constexpr int UW = U4 ? 4 : 8, LUW = U4 ? 2 : 3;
     const int *offx = S.offx, *offy = S.offy;
-    const int cols = cs / UW, nu = cols * (cs >> 2);
-    const int mcols = (65536 + cols - 1) / cols;
+    const int lgc = 31 - __clz(cs) - LUW, cols = 1 << lgc, nw = U4 ? 1 : (cols * (cs >> 2) + 31) >> 5;
     int(*T)[kGrpMaxPos] = U4 ? S.t4 : S.t8;
-    if (nu >= 32) {
-        // a lane per unit, its current block loaded once for all positions
-        for (int u = lane; u < nu; u += 32) {
-            const int uy = div_small(u, mcols), ux = u - uy * cols;
-            if (!unit_covered(S, grp, ux * UW, uy * 4, U4)) continue;
-            UnitC c;
-            const ptrdiff_t off = (ptrdiff_t)uy * 4 * stride + ux * UW;
-            load_unit<U4>(o + off, stride, c);
-            // one copy of the unit's cost code (the kernel stays small in
-            // the instruction cache)
+    int n = 0;
+    for (int w = 0; w < nw; w++) {
+        const unsigned cov = __reduce_or_sync(0xffffffffu, (grp >> lane) & 1 ? S.mask[lane][w] : 0u);
+        if ((cov >> lane) & 1) S.list[n + __popc(cov & ((1u << lane) - 1))] = (uint8_t)(32 * w + lane);
+        n += __popc(cov);
+    }
+    __syncwarp();
+    const bool pairs = ((n * P + 31) >> 5) * 5 < ((n + 31) >> 5) * (1 + 4 * P);
+    const int items = pairs ? n * P : n, mp = P == 9 ? 7282 : P == 8 ? 8192 : P == 5 ? 13108 : 16384;   // 65536 / P
+    for (int e = lane; e < items; e += 32) {
+        const int q = pairs ? div_small(e, mp) : e, k0 = pairs ? e - q * P : 0, k1 = pairs ? k0 + 1 : P;
+        const int u = S.list[q], uy = u >> lgc, ux = u - uy * cols;
+        UnitC c;
+        const ptrdiff_t off = (ptrdiff_t)uy * 4 * stride + ux * UW;
+        load_unit<U4>(o + off, stride, c);
+        // one copy of the unit's cost code (the kernel stays small in the
+        // instruction cache)
 #pragma unroll 1
-            for (int k = 0; k < P; k++) {
-                const int mx = ccx + offx[k], my = ccy + offy[k];
-                const uint8_t *r = planes[((my & 3) << 2) + (mx & 3)] + (ptrdiff_t)(py + (my >> 2)) * stride + px +
-                                   (mx >> 2) + off;
-                T[u][k] = unit_cost_pre<U4>(had, c, r, stride);
-            }
-        }
-    } else {
-        // a lane per (unit, position)
-        const int mp = (65536 + P - 1) / P;
-        for (int e = lane; e < nu * P; e += 32) {
-            const int u = div_small(e, mp), k = e - u * P;
-            const int uy = div_small(u, mcols), ux = u - uy * cols;
-            if (!unit_covered(S, grp, ux * UW, uy * 4, U4)) continue;
-            UnitC c;
-            const ptrdiff_t off = (ptrdiff_t)uy * 4 * stride + ux * UW;
-            load_unit<U4>(o + off, stride, c);
+        for (int k = k0; k < k1; k++) {
             const int mx = ccx + offx[k], my = ccy + offy[k];
             const uint8_t *r = planes[((my & 3) << 2) + (mx & 3)] + (ptrdiff_t)(py + (my >> 2)) * stride + px +
                                (mx >> 2) + off;
@@ -1087,11 +1068,13 @@ __device__ __forceinline__ void group_table(GroupSmem &S, unsigned grp, bool had
     }
 }
 
-// resident CTAs per SM the register budget is sized for (5: 96 registers;
-// measured faster on serving batches than 4 (126) and than the compiler's
-// own choice of 168)
+// Bound by instruction issue at the latency of the plane reads: with a lane per
+// unit and the members' units tested one by one, 19 of 32 lanes were active
+// (1.86 ms of a 2160p picture's chain).  Unit masks and
+// listed units leave few lanes idle, and 72 registers let 7 CTAs share an SM
+// (serving mix of 17.0 ms: 5 CTAs 16.4, 6 16.1, 7 15.9, 8 16.1).
 #ifndef XG_GROUP_MINB
-#define XG_GROUP_MINB 5
+#define XG_GROUP_MINB 7
 #endif
 __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_kernel(const RefineGroup *__restrict__ groups,
                                                                       int ngroups,
@@ -1113,7 +1096,7 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
     const int lam = prm.lambda_factor;
     const bool mem = lane < M;
     int i = 0, pmx = 0, pmy = 0, bx = 0, by = 0, best = 0;
-    bool valid = false;
+    bool valid = false, u4 = false;
     xavs2gpu_me_result_t res;
     if (mem) {
         i = (int)(members[G.first + lane] & kIdxMask);
@@ -1122,11 +1105,12 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
         const unsigned long long key = v.keys[i];
         valid = st.valid && key != kNoKey;
         const int w = c_pu_w[p.part], h = c_pu_h[p.part];
-        S.rx[lane] = (int16_t)(p.x - G.cx);
-        S.ry[lane] = (int16_t)(p.y - G.cy);
-        S.rw[lane] = (int16_t)w;
-        S.rh[lane] = (int16_t)h;
-        S.ru4[lane] = (int8_t)(had ? satd_unit4(w, h) : (w == 4 || w == 12));
+        u4 = had ? satd_unit4(w, h) : (w == 4 || w == 12);
+        const int luw = u4 ? 2 : 3, lgc = G.lg - luw;   // log2 of the units' width and of the units in a row
+        const uint32_t run = ((1u << (w >> luw)) - 1) << ((p.x - G.cx) >> luw);
+        for (int k = 0; k < kGrpU8 / 32; k++) S.mask[lane][k] = 0;
+        for (int y = (p.y - G.cy) >> 2, ye = y + (h >> 2); y < ye; y++)
+            S.mask[lane][(y << lgc) >> 5] |= run << ((y << lgc) & 31);
         pmx = p.mvp_x;
         pmy = p.mvp_y;
         if (!valid) {
@@ -1149,29 +1133,21 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
         }
     }
     __syncwarp();
+    const unsigned u4s = __ballot_sync(0xffffffffu, u4);
+    const int nw = cs == 64 ? kGrpU8 / 32 : 1;   // words of a unit mask
     const uint8_t *o = v.cur + (ptrdiff_t)G.cy * g.stride + G.cx;
     const uint8_t *const *planes = v.planes + 16 * G.ref;
     if (prm.fractional_me) {
         const int pat = prm.fast_sub_me ? 1 : 0, step = prm.fast_sub_me ? 2 : 1;
         for (int stage = 0; stage < (prm.fractional_me > 1 ? 2 : 1); stage++) {
             // the stage's positions relative to the centre, in the reference's order
-            int offx[kGrpMaxPos], offy[kGrpMaxPos], P = 0;
-            const int k0 = (stage == 0 && had) ? 1 : 0;
-#pragma unroll
-            for (int k = 0; k < kGrpMaxPos; k++) { offx[k] = 0; offy[k] = 0; }
-            P = k0;
-#pragma unroll
-            for (int pos = 1; pos < 9; pos++) {
-                if ((pos - 1) % step) continue;
-                const int mult = stage == 0 ? 2 : 1;
-#pragma unroll
-                for (int k = 0; k < kGrpMaxPos; k++)
-                    if (k == P) { offx[k] = mult * c_spiral[pat][pos][0]; offy[k] = mult * c_spiral[pat][pos][1]; }
-                P++;
-            }
-            if (lane == 0) {
-#pragma unroll
-                for (int k = 0; k < kGrpMaxPos; k++) { S.offx[k] = offx[k]; S.offy[k] = offy[k]; }
+            const int k0 = (stage == 0 && had) ? 1 : 0, mult = stage == 0 ? 2 : 1;
+            const int P = k0 + (prm.fast_sub_me ? 4 : 8);
+            __syncwarp();   // the last stage's offsets are read
+            if (lane < P) {
+                const int pos = lane < k0 ? 0 : 1 + (lane - k0) * step;
+                S.offx[lane] = lane < k0 ? 0 : mult * c_spiral[pat][pos][0];
+                S.offy[lane] = lane < k0 ? 0 : mult * c_spiral[pat][pos][1];
             }
             __syncwarp();
             unsigned pending = __ballot_sync(0xffffffffu, mem && valid);
@@ -1180,14 +1156,14 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
                 const int ccx = __shfl_sync(0xffffffffu, bx, leader), ccy = __shfl_sync(0xffffffffu, by, leader);
                 const unsigned grp = __ballot_sync(0xffffffffu, mem && valid && bx == ccx && by == ccy) & pending;
                 pending &= ~grp;
-                const bool need8 = __any_sync(0xffffffffu, ((grp >> lane) & 1) && !S.ru4[lane]);
-                const bool need4 = __any_sync(0xffffffffu, ((grp >> lane) & 1) && S.ru4[lane]);
-                if (need8)
-                    group_table<false>(S, grp, had, cs, o, planes, g.stride, G.cx, G.cy, ccx, ccy, P, lane);
+                if (grp & ~u4s)
+                    group_table<false>(S, grp & ~u4s, had, cs, o, planes, g.stride, G.cx, G.cy, ccx, ccy, P, lane);
                 // 4x4 units occur only in 16x16 CUs (4- and 12-wide partitions);
                 // the 4x4 table holds one 16x16 CU
-                if (need4 && cs == 16)
-                    group_table<true>(S, grp, had, cs, o, planes, g.stride, G.cx, G.cy, ccx, ccy, P, lane);
+                if ((grp & u4s) && cs == 16) {
+                    __syncwarp();   // the list is rebuilt
+                    group_table<true>(S, grp & u4s, had, cs, o, planes, g.stride, G.cx, G.cy, ccx, ccy, P, lane);
+                }
                 __syncwarp();
                 // each member's sums over its units
                 int acc[kGrpMaxPos];
@@ -1196,17 +1172,13 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
                 for (unsigned left = grp; left;) {
                     const int m = __ffs(left) - 1;
                     left &= left - 1;
-                    const int u4 = S.ru4[m], uw = u4 ? 4 : 8;
-                    const int nux = S.rw[m] / uw, n = nux * (S.rh[m] >> 2);
-                    const int mnux = (65536 + nux - 1) / nux, cols = cs / uw;
-                    const int base = (S.ry[m] >> 2) * cols + S.rx[m] / uw;
+                    const int(*T)[kGrpMaxPos] = (u4s >> m) & 1 ? S.t4 : S.t8;
                     int part[kGrpMaxPos];
 #pragma unroll
                     for (int k = 0; k < kGrpMaxPos; k++) part[k] = 0;
-                    for (int q = lane; q < n; q += 32) {
-                        const int qy = div_small(q, mnux), qx = q - qy * nux;
-                        const int u = base + qy * cols + qx;
-                        const int *row = u4 ? S.t4[u] : S.t8[u];
+                    for (int w = 0; w < nw; w++) {
+                        if (!((S.mask[m][w] >> lane) & 1)) continue;
+                        const int *row = T[32 * w + lane];
 #pragma unroll
                         for (int k = 0; k < kGrpMaxPos; k++)
                             if (k < P) part[k] += row[k];
@@ -1226,7 +1198,7 @@ __global__ void __launch_bounds__(32 * kGrpWarps, XG_GROUP_MINB) refine_group_ke
 #pragma unroll
                     for (int k = 0; k < kGrpMaxPos; k++) {
                         if (k < k0 || k >= P) continue;
-                        const int mx = ccx + offx[k], my = ccy + offy[k];
+                        const int mx = ccx + S.offx[k], my = ccy + S.offy[k];
                         const int c = acc[k] + mv_cost_hd(lam, mx, my, pmx, pmy);
                         if (c < best) { best = c; nbx = mx; nby = my; }
                     }
