@@ -567,6 +567,31 @@ __device__ __forceinline__ void load8u(const uint8_t *p, uint32_t &lo, uint32_t 
     lo = __funnelshift_r(w0, w1, sh);
     hi = __funnelshift_r(w1, w2, sh);
 }
+// the same from two 8-byte words: for threads that read far apart, where a
+// request costs a cache line per lane whatever its width
+__device__ __forceinline__ void load16w(const uint8_t *p, uint32_t (&w)[4])   // from the last 8-byte boundary
+{
+    const uint2 *q = reinterpret_cast<const uint2 *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)7);
+    const uint2 a = __ldg(q), b = __ldg(q + 1);
+    w[0] = a.x; w[1] = a.y; w[2] = b.x; w[3] = b.y;
+}
+// bytes o .. o + 7 of the 16, o <= 8
+__device__ __forceinline__ void bytes_at(const uint32_t (&w)[4], int o, uint32_t &lo, uint32_t &hi)
+{
+    const uint32_t a = o & 8 ? w[2] : o & 4 ? w[1] : w[0], b = o & 8 ? w[3] : o & 4 ? w[2] : w[1];
+    const uint32_t e = o & 4 ? w[3] : w[2];   // not read at o = 8
+    lo = __funnelshift_r(a, b, 8 * (o & 3));
+    hi = __funnelshift_r(b, e, 8 * (o & 3));
+}
+__device__ __forceinline__ void load8w(const uint8_t *p, uint32_t &lo, uint32_t &hi)
+{
+    const int o = (int)(reinterpret_cast<uintptr_t>(p) & 7);
+    uint32_t w[4];
+    load16w(p, w);
+    const uint32_t a = o & 4 ? w[1] : w[0], b = o & 4 ? w[2] : w[1], e = o & 4 ? w[3] : w[2];
+    lo = __funnelshift_r(a, b, 8 * (o & 3));
+    hi = __funnelshift_r(b, e, 8 * (o & 3));
+}
 
 // (byte k, byte 4 + k) of the 8-byte row (lo, hi) as zero-extended halves
 __device__ __forceinline__ void row_pairs(uint32_t lo, uint32_t hi, uint32_t (&q)[4])
@@ -709,7 +734,7 @@ __device__ __forceinline__ void load_unit_rt(const uint8_t *o, int stride, UnitC
 #pragma unroll
     for (int y = 0; y < 4; y++) {
         uint32_t lo, hi;
-        load8u(o + y * stride, lo, hi);
+        load8w(o + y * stride, lo, hi);
         c.w[y][0] = lo;
         c.w[y][1] = u4 ? 0u : hi;
         row_pairs(lo, c.w[y][1], c.q[y]);
@@ -723,7 +748,7 @@ __device__ __forceinline__ int unit_cost_pre_rt(bool had, bool u4, const UnitCur
 #pragma unroll
         for (int y = 0; y < 4; y++) {
             uint32_t lo, hi;
-            load8u(r + y * stride, lo, hi);
+            load8w(r + y * stride, lo, hi);
             s = sad4_acc(c.w[y][0], lo, s);
             s = sad4_acc(c.w[y][1], u4 ? 0u : hi, s);
         }
@@ -733,7 +758,7 @@ __device__ __forceinline__ int unit_cost_pre_rt(bool had, bool u4, const UnitCur
 #pragma unroll
     for (int y = 0; y < 4; y++) {
         uint32_t lo, hi, q[4];
-        load8u(r + y * stride, lo, hi);
+        load8w(r + y * stride, lo, hi);
         row_pairs(lo, u4 ? 0u : hi, q);
 #pragma unroll
         for (int x = 0; x < 4; x++) d[y][x] = c.q[y][x] - q[x];
@@ -777,11 +802,95 @@ __device__ __forceinline__ void refine_stage_thread(bool had, bool u4, int nux, 
     }
 }
 
+#if XG_REFINE_PACKED
+// The half-pel stage around the full-pel position (px, py) in spiral order
+// (me_subpel_refine): positions 2 quarter-pels apart in x or y are one sample
+// apart in the same plane, so 18 rows serve the nine positions' 36.  The
+// per-thread form is bound by its cache requests, a line per lane: 1080p R = 64
+// search 3.90 ms with three 4-byte words per row, 3.81 with two of 8 bytes,
+// 3.73 with this stage's rows shared.
+// acc[k0 + p - 1] is position p's cost, acc[0] the centre's if k0 is 1.
+template <bool HAD>
+__device__ __forceinline__ void refine_half_thread(bool u4, int nux, int nu, const uint8_t *o,
+                                                   const uint8_t *const *planes, int stride, int px, int py,
+                                                   int (&acc)[9])
+{
+    constexpr int K = HAD ? 0 : -1;   // position p is acc[p + K]
+    const int uw = u4 ? 4 : 8;
+    const uint8_t *pf = planes[0], *ph = planes[2], *pv = planes[8], *pd = planes[10];
+#pragma unroll
+    for (int k = 0; k < 9; k++) acc[k] = 0;
+    for (int u = 0; u < nu; u++) {
+        const int uy = u / nux, ux = u - uy * nux;
+        UnitCur c;
+        load_unit_rt(o + (ptrdiff_t)uy * 4 * stride + ux * uw, stride, c, u4);
+        const ptrdiff_t at = (ptrdiff_t)(py + uy * 4) * stride + px + ux * uw;
+        uint32_t lo[5], hi[5];
+        auto cost = [&](int r0) -> int {   // rows r0 .. r0 + 3 against the unit
+            if (HAD) {
+                uint32_t d[4][4];
+#pragma unroll
+                for (int y = 0; y < 4; y++) {
+                    uint32_t q[4];
+                    row_pairs(lo[r0 + y], u4 ? 0u : hi[r0 + y], q);
+#pragma unroll
+                    for (int x = 0; x < 4; x++) d[y][x] = c.q[y][x] - q[x];
+                }
+                return satd_pairs(d);
+            }
+            uint32_t s = 0;
+#pragma unroll
+            for (int y = 0; y < 4; y++) {
+                s = sad4_acc(c.w[y][0], lo[r0 + y], s);
+                s = sad4_acc(c.w[y][1], u4 ? 0u : hi[r0 + y], s);
+            }
+            return (int)s;
+        };
+        if (HAD) {
+#pragma unroll
+            for (int y = 0; y < 4; y++) load8w(pf + at + y * stride, lo[y], hi[y]);
+            acc[0] += cost(0);
+        }
+        {   // rows py - 1 .. py + 3 of the vertical half-pel plane
+#pragma unroll
+            for (int y = 0; y < 5; y++) load8w(pv + at + (y - 1) * stride, lo[y], hi[y]);
+            acc[1 + K] += cost(0);
+            acc[2 + K] += cost(1);
+        }
+        {   // columns px - 1 .. px + 7 of the horizontal one
+            const int of = (int)(reinterpret_cast<uintptr_t>(ph + at - 1) & 7);   // stride: a multiple of 8
+            uint32_t w[4][4];
+#pragma unroll
+            for (int y = 0; y < 4; y++) load16w(ph + at - 1 + y * stride, w[y]);
+#pragma unroll
+            for (int y = 0; y < 4; y++) bytes_at(w[y], of, lo[y], hi[y]);
+            acc[5 + K] += cost(0);
+#pragma unroll
+            for (int y = 0; y < 4; y++) bytes_at(w[y], of + 1, lo[y], hi[y]);
+            acc[6 + K] += cost(0);
+        }
+        {   // both of the diagonal one
+            const int of = (int)(reinterpret_cast<uintptr_t>(pd + at - 1) & 7);
+            uint32_t w[5][4];
+#pragma unroll
+            for (int y = 0; y < 5; y++) load16w(pd + at - 1 + (y - 1) * stride, w[y]);
+#pragma unroll
+            for (int y = 0; y < 5; y++) bytes_at(w[y], of, lo[y], hi[y]);
+            acc[3 + K] += cost(0);
+            acc[7 + K] += cost(1);
+#pragma unroll
+            for (int y = 0; y < 5; y++) bytes_at(w[y], of + 1, lo[y], hi[y]);
+            acc[4 + K] += cost(0);
+            acc[8 + K] += cost(1);
+        }
+    }
+}
+#endif
+
 // resident CTAs per SM the register budget of the per-thread refinement is
-// sized for (5: 96 registers; serving mix 17.0 ms at 4, 16.8 at 5 and 6, 17.15
-// at 3; 1080p R = 64 search 3.90 ms at 4 and 5, 3.98 at 6)
+// sized for (4: 128 registers; 1080p R = 64 search 3.73 ms, at 5 3.81, at 3 3.76)
 #ifndef XG_REFINE_MINB
-#define XG_REFINE_MINB 5
+#define XG_REFINE_MINB 4
 #endif
 
 // HAD: SATD (1) or SAD (0) unit costs, fixed per launch so that each
@@ -867,7 +976,12 @@ __global__ void __launch_bounds__(128, XG_REFINE_MINB) refine_thread_kernel(cons
                 npos++;
             }
             int acc[9];
-            refine_stage_thread(had, u4, nux, nu, o, planes, g.stride, p.x, p.y, mxs, mys, npos, acc);
+#if XG_REFINE_PACKED
+            if (stage == 0 && !prm.fast_sub_me)
+                refine_half_thread<HAD>(u4, nux, nu, o, planes, g.stride, p.x + (cx >> 2), p.y + (cy >> 2), acc);
+            else
+#endif
+                refine_stage_thread(had, u4, nux, nu, o, planes, g.stride, p.x, p.y, mxs, mys, npos, acc);
             const int k0 = (stage == 0 && had) ? 1 : 0;
             if (k0) best = acc[0] + mv_cost_hd(lam, cx, cy, pmx, pmy);
 #pragma unroll
