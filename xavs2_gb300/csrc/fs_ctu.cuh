@@ -494,25 +494,54 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
         }
         __syncthreads();
     }
+    // four entries per item, the words of several items read before any is
+    // placed (one item at a time waited for memory 40 times over)
     const bool from_stage = use_tma || (staged && !inside);
-    for (int r = warp; r < wrows; r += kCtuWarps) {
-        const uint8_t *row = ref + (ptrdiff_t)min(max(wy0 + r, -kPad), g.H + kPad - 1) * g.stride;
-        auto word = [&](int k) -> uint32_t {   // samples 4k .. 4k + 3 of the window row
-            if (from_stage)
-                return *reinterpret_cast<const uint32_t *>(stage + (k >> 4) * kTmaPieceBytes + r * kTmaBoxCols +
-                                                           4 * (k & 15));
-            if (inside) return __ldg(reinterpret_cast<const uint32_t *>(row + wx0) + k);
-            uint32_t v = 0;
+    const int quads = (pitch + 3) >> 2, items = wrows * quads, mq = (65536 + quads - 1) / quads;
+    auto place = [&](int r, int k, uint32_t lo, uint32_t hi) {
+        if (k >= pitch) return;
+        uint2 *d = win + ctu_entry(r, pitch) + k;
+        d[0] = make_uint2(lo, __byte_perm(lo, hi, 0x4321));
+        d[plane] = make_uint2(__byte_perm(lo, hi, 0x5432), __byte_perm(lo, hi, 0x6543));
+    };
+    if (from_stage || inside) {
+        constexpr int NB = 4;
+        for (int e0 = tid; e0 < items; e0 += NB * kCtuThreads) {
+            uint4 v[NB];
+            uint32_t nx[NB];
 #pragma unroll
-            for (int b = 0; b < 4; b++)
-                v |= (uint32_t)row[min(max(wx0 + 4 * k + b, -kPad), g.W + kPad - 1)] << (8 * b);
-            return v;
-        };
-        uint2 *d = win + ctu_entry(r, pitch);
-        for (int k = lane; k < pitch; k += 32) {
-            const uint32_t lo = word(k), hi = word(k + 1);
-            d[k] = make_uint2(lo, __byte_perm(lo, hi, 0x4321));
-            d[k + plane] = make_uint2(__byte_perm(lo, hi, 0x5432), __byte_perm(lo, hi, 0x6543));
+            for (int b = 0; b < NB; b++) {
+                const int e = min(e0 + b * kCtuThreads, items - 1), r = (e * mq) >> 16, q = e - r * quads;
+                if (from_stage) {
+                    const uint8_t *t = stage + r * kTmaBoxCols;
+                    v[b] = *reinterpret_cast<const uint4 *>(t + (q >> 2) * kTmaPieceBytes + 16 * (q & 3));
+                    nx[b] = *reinterpret_cast<const uint32_t *>(t + ((q + 1) >> 2) * kTmaPieceBytes + 16 * ((q + 1) & 3));
+                } else {
+                    const uint4 *t = reinterpret_cast<const uint4 *>(ref + (ptrdiff_t)(wy0 + r) * g.stride + wx0) + q;
+                    v[b] = __ldg(t);
+                    nx[b] = __ldg(reinterpret_cast<const uint32_t *>(t + 1));
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const int e = e0 + b * kCtuThreads, r = (e * mq) >> 16, k = 4 * (e - r * quads);
+                if (e >= items) break;
+                place(r, k, v[b].x, v[b].y);
+                place(r, k + 1, v[b].y, v[b].z);
+                place(r, k + 2, v[b].z, v[b].w);
+                place(r, k + 3, v[b].w, nx[b]);
+            }
+        }
+    } else {
+        for (int r = warp; r < wrows; r += kCtuWarps) {
+            const uint8_t *row = ref + (ptrdiff_t)min(max(wy0 + r, -kPad), g.H + kPad - 1) * g.stride;
+            for (int k = lane; k < pitch; k += 32) {
+                uint32_t w[2] = {0, 0};
+#pragma unroll
+                for (int b = 0; b < 8; b++)
+                    w[b >> 2] |= (uint32_t)row[min(max(wx0 + 4 * k + b, -kPad), g.W + kPad - 1)] << (8 * (b & 3));
+                place(r, k, w[0], w[1]);
+            }
         }
     }
     __syncthreads();
@@ -558,23 +587,27 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
 #pragma unroll
         for (int k = 0; k < 3; k++) kl[k] = 0xffffffffu;
     };
-    // the warp's minima into the global keys; order(row, dxr) is the visit order
+    // the warp's minima into the global keys; order(row, dxr) is the visit
+    // order.  The slots are read before any of them is needed.
     auto merge = [&](auto order) {
+        int pus[25], pul[3];
+#pragma unroll
+        for (int k = 0; k < 25; k++)
+            if ((LV & 1) || k >= 18) pus[k] = smap[small_slot(rx, ry, half, k)];
+#pragma unroll
+        for (int k = 0; k < 3; k++) pul[k] = lm[k] < 0 ? -1 : smap[k < 2 ? 784 + cu32 * 13 + lm[k] : 836 + lm[k]];
 #pragma unroll
         for (int k = 0; k < 25; k++) {
+            if (!(LV & 1) && k < 18) continue;
             const uint32_t cost = ks[k] >> 11;
-            if (cost >= kPoisonSmall) continue;
-            const int pu = smap[small_slot(rx, ry, half, k)];
-            if (pu >= 0)
-                atomicMin(&keys[pu], ((unsigned long long)cost << 32) | order((ks[k] >> 8) & 7u, ks[k] & 0xffu));
+            if (cost < kPoisonSmall && pus[k] >= 0)
+                atomicMin(&keys[pus[k]], ((unsigned long long)cost << 32) | order((ks[k] >> 8) & 7u, ks[k] & 0xffu));
         }
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             const uint32_t cost = kl[k] >> 11;
-            if (lm[k] < 0 || cost >= kCapLarge) continue;
-            const int pu = smap[k < 2 ? 784 + cu32 * 13 + lm[k] : 836 + lm[k]];
-            if (pu >= 0)
-                atomicMin(&keys[pu], ((unsigned long long)cost << 32) | order((kl[k] >> 8) & 7u, kl[k] & 0xffu));
+            if (cost < kCapLarge && pul[k] >= 0)
+                atomicMin(&keys[pul[k]], ((unsigned long long)cost << 32) | order((kl[k] >> 8) & 7u, kl[k] & 0xffu));
         }
     };
     clear();
@@ -807,9 +840,9 @@ static CtuFit ctu_fit(int dev, int R, int dyw)
 // lets an SM hold more CTAs (R = 64: 2 at 8 rows, 3 at 4; R = 128: 1, 2 at 2),
 // and more CTAs.  So: the most rows at which an SM holds the most CTAs, halved while
 // the launch is below two rounds of the GPU.  Measured, one reference, us at 8 /
-// 4 / 2 rows: 1080p R = 64 1558 / 1422 / 1473, R = 32 372 / 380 / 399, R = 16
-// 125 / 118 / 138; 720p R = 16 104 / 85 / 82; 416x240 R = 16 51 / 34 / 26,
-// R = 64 223 / 165 / 123; 1080p R = 128 7649 / 7845 / 6241.
+// 4 / 2 rows: 1080p R = 64 1440 / 1357 / 1360, R = 32 352 / 356 / 384, R = 16
+// 112 / 106 / 119; 720p R = 16 98 / 78 / 74; 416x240 R = 16 41 / 28 / 20,
+// R = 64 210 / 153 / 112; 1080p R = 128 6848 / 6972 / 5617.
 #ifndef XG_CTU_DYW
 #define XG_CTU_DYW 0   // 0: by the rule
 #endif
