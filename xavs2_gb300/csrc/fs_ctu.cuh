@@ -879,10 +879,11 @@ struct CtuSide {
         if (st) cudaStreamDestroy(st);
     }
 };
-static CtuSide *ctu_side(int dev, int k = 0)   // k: 0 the search's own, 1 the per-PU search's
+// k: 0 the search's own, 1 the per-PU search's, 2 the per-PU search's second
+static CtuSide *ctu_side(int dev, int k = 0)
 {
-    thread_local CtuSide side[2][64];
-    if (dev < 0 || dev >= 64 || k < 0 || k > 1) return nullptr;
+    thread_local CtuSide side[3][64];
+    if (dev < 0 || dev >= 64 || k < 0 || k > 2) return nullptr;
     CtuSide &s = side[k][dev];
     if (!s.st) {
         if (cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking) != cudaSuccess ||
@@ -903,6 +904,7 @@ static void ctu_prime(int R)
     if (XG_CTU_FORK) {
         ctu_side(dev, 0);
         ctu_side(dev, 1);
+        ctu_side(dev, 2);
     }
     if (R < 1 || R > 128) return;
     for (int dyw = 2; dyw <= kDyWarpMax; dyw *= 2) ctu_fit(dev, R, dyw);

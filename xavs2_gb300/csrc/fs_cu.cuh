@@ -511,18 +511,12 @@ static int cu_launch_one(const CuQueues &q, const CuRec *cus, const SessView *vi
     return XAVS2GPU_OK;
 }
 
-// Groups the CUs' partitions and searches the clusters, largest CUs first.
-static int cu_search_launch(const CuQueues &q, const CuRec *cus, int n, const SessView *views, int R, int lambda,
-                            cudaStream_t st)
+// Groups the CUs' partitions into clusters and PUs searched one by one.
+static void cu_cluster_launch(const CuQueues &q, const CuRec *cus, int n, const SessView *views, cudaStream_t st)
 {
     XG_CUDA(cudaMemsetAsync(q.count, 0, sizeof(int) * kCuCounters, st));
     cu_cluster_kernel<<<(n + 127) / 128, 128, 0, st>>>(cus, n, views, q);
     count_launch();
-    int rc = cu_launch_one<64>(q, cus, views, R, lambda, st);
-    if (rc == XAVS2GPU_OK) rc = cu_launch_one<32>(q, cus, views, R, lambda, st);
-    if (rc == XAVS2GPU_OK) rc = cu_launch_one<16>(q, cus, views, R, lambda, st);
-    if (rc == XAVS2GPU_OK) rc = cu_launch_one<8>(q, cus, views, R, lambda, st);
-    return rc;
 }
 
 }  // namespace xg

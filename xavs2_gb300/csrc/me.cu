@@ -418,22 +418,6 @@ struct PerPuList {
     int n_cus = 0, cap_large = 0, cap_small = 0;
     CuQueues q{};
 };
-static int per_pu_launch(const PerPuList &l, const SessView *views, int R, int lambda, cudaStream_t st)
-{
-    int rc = XAVS2GPU_OK;
-    if (l.n_cus) {
-        rc = cu_search_launch(l.q, l.cus, l.n_cus, views, R, lambda, st);
-        if (rc == XAVS2GPU_OK)
-            rc = prune_launch_one<64>(l.q.large, l.cap_large, l.q.count + 4, views, R, lambda, st);
-        if (rc == XAVS2GPU_OK)
-            rc = prune_launch_one<kSmallDim>(l.q.small, l.cap_small, l.q.count + 5, views, R, lambda, st);
-    }
-    if (rc == XAVS2GPU_OK) rc = prune_launch(l.list, l.n_large, l.n_small, views, R, lambda, st);
-    if (rc == XAVS2GPU_OK && l.n_plain)
-        rc = fs_generic_launch(l.list + l.n_large + l.n_small, l.n_plain, views, R, lambda, st);
-    return rc;
-}
-
 // ---- 3. sub-pel refinement ------------------------------------------------------------
 // One warp per PU: the candidate costs of one refinement step are evaluated in
 // parallel, then the first strictly smaller one (spiral order, centre first)
@@ -1347,33 +1331,56 @@ static void launch_groups(const RefineGroup *groups, int n, const uint32_t *memb
 
 namespace xg {
 
-// The refinement's per-warp list on the CTU search's side stream when the
-// per-thread list runs too: the lists are disjoint, and each launch's last
-// wave then overlaps the other's work.  fork returns the stream to launch on.
-static cudaStream_t refine_fork(cudaStream_t st, bool both, CtuSide *&side)
+// Launches beside st on side stream k: fork returns the stream to launch on (st
+// itself without a side stream), join makes st wait for it.
+static cudaStream_t fork_side(cudaStream_t st, bool both, int k, CtuSide *&side)
 {
-    side = XG_CTU_FORK && both ? ctu_side(current_device()) : nullptr;
+    side = XG_CTU_FORK && both ? ctu_side(current_device(), k) : nullptr;
     if (!side) return st;
     XG_CUDA(cudaEventRecord(side->fork, st));
     XG_CUDA(cudaStreamWaitEvent(side->st, side->fork, 0));
     return side->st;
 }
-static void refine_join(cudaStream_t st, CtuSide *side)
+static void join_side(cudaStream_t st, CtuSide *side)
 {
     if (!side) return;
     XG_CUDA(cudaEventRecord(side->join, side->st));
     XG_CUDA(cudaStreamWaitEvent(st, side->join, 0));
 }
+// The refinement's per-warp list on the CTU search's side stream when the
+// per-thread list runs too: the lists are disjoint, and each launch's last
+// wave then overlaps the other's work.
+static cudaStream_t refine_fork(cudaStream_t st, bool both, CtuSide *&side) { return fork_side(st, both, 0, side); }
 
 // The per-PU search beside the CTU search (their PUs are disjoint) on a
 // second side stream, when both have work and phases are not being timed.
-static cudaStream_t search_fork(cudaStream_t st, bool both, CtuSide *&side)
+static cudaStream_t search_fork(cudaStream_t st, bool both, CtuSide *&side) { return fork_side(st, both, 1, side); }
+
+// The six searches after the clustering are of disjoint PUs: the 64x64 CUs' and
+// the small PUs' on st, the others' beside them.  One after the other each
+// leaves the GPU idle behind its longest cluster (264x128, R = 48: 237 us for
+// the 64x64 CUs, 280 for the others).
+static int per_pu_launch(const PerPuList &l, const SessView *views, int R, int lambda, cudaStream_t st)
 {
-    side = XG_CTU_FORK && both ? ctu_side(current_device(), 1) : nullptr;
-    if (!side) return st;
-    XG_CUDA(cudaEventRecord(side->fork, st));
-    XG_CUDA(cudaStreamWaitEvent(side->st, side->fork, 0));
-    return side->st;
+    int rc = XAVS2GPU_OK;
+    if (l.n_cus) {
+        cu_cluster_launch(l.q, l.cus, l.n_cus, views, st);
+        CtuSide *side = nullptr;
+        const cudaStream_t st2 = fork_side(st, true, 2, side);
+        rc = cu_launch_one<64>(l.q, l.cus, views, R, lambda, st);
+        if (rc == XAVS2GPU_OK) rc = cu_launch_one<32>(l.q, l.cus, views, R, lambda, st2);
+        if (rc == XAVS2GPU_OK) rc = cu_launch_one<16>(l.q, l.cus, views, R, lambda, st2);
+        if (rc == XAVS2GPU_OK) rc = cu_launch_one<8>(l.q, l.cus, views, R, lambda, st2);
+        if (rc == XAVS2GPU_OK)
+            rc = prune_launch_one<64>(l.q.large, l.cap_large, l.q.count + 4, views, R, lambda, st2);
+        if (rc == XAVS2GPU_OK)
+            rc = prune_launch_one<kSmallDim>(l.q.small, l.cap_small, l.q.count + 5, views, R, lambda, st);
+        join_side(st, side);
+    }
+    if (rc == XAVS2GPU_OK) rc = prune_launch(l.list, l.n_large, l.n_small, views, R, lambda, st);
+    if (rc == XAVS2GPU_OK && l.n_plain)
+        rc = fs_generic_launch(l.list + l.n_large + l.n_small, l.n_plain, views, R, lambda, st);
+    return rc;
 }
 
 // ---- session ---------------------------------------------------------------------
@@ -2061,7 +2068,7 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     if (gside && m.n_generic) {
         const int rc = per_pu_launch(per_pu, m.d_view, R, lam, gst);
         if (rc != XAVS2GPU_OK) {
-            refine_join(m.st, gside);
+            join_side(m.st, gside);
             return rc;
         }
     }
@@ -2071,7 +2078,7 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
         const int rc = per_pu_launch(per_pu, m.d_view, R, lam, m.st);
         if (rc != XAVS2GPU_OK) return rc;
     }
-    refine_join(m.st, gside);
+    join_side(m.st, gside);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[3], m.st));
     // the CU-grouped refinement follows the reference's per-PU order, which
     // with PMVR depends on each PU's predictor; PMVR keeps the per-PU kernels
@@ -2096,7 +2103,7 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
             reinterpret_cast<const uint32_t *>(lst_l), nl, m.d_view, R, *prm);
         count_launch();
     }
-    refine_join(m.st, side);
+    join_side(m.st, side);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[4], m.st));
     XG_CUDA(cudaGetLastError());
     return XAVS2GPU_OK;
@@ -2530,7 +2537,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     if (gside) {
         const int rc = per_pu_launch(per_pu, bb.d_views, R, lam, gst);
         if (rc != XAVS2GPU_OK) {
-            refine_join(st, gside);
+            join_side(st, gside);
             return rc;
         }
     }
@@ -2539,7 +2546,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         const int rc = per_pu_launch(per_pu, bb.d_views, R, lam, st);
         if (rc != XAVS2GPU_OK) return rc;
     }
-    refine_join(st, gside);
+    join_side(st, gside);
     if (ngr) launch_groups(bb.d_groups, (int)ngr, d_members, bb.d_views, R, *prm, st);
     CtuSide *side = nullptr;
     const cudaStream_t wst = refine_fork(st, ns && nl, side);
@@ -2556,7 +2563,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
                                                                                            bb.d_views, R, *prm);
         count_launch();
     }
-    refine_join(st, side);
+    join_side(st, side);
     XG_CUDA(cudaEventRecord(bb.done, st));
     bb.used = true;
     XG_CUDA(cudaGetLastError());
