@@ -74,3 +74,46 @@ def test_skip_costs(gpu, olib, w, h, nrefs):
     assert np.array_equal(d_cost.cpu().numpy(), e_cost)
     assert np.array_equal(d_best.cpu().numpy(), e_best)
     sess.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 700, 2400])
+def test_skip_extreme_samples_and_small_lists(gpu, olib, n):
+    """Pictures of 0 and 255 alone (the largest differences and Hadamard sums)
+    and lists that end inside a CU, a warp's share or a class; with 2400, more
+    warps' worth of work than the smallest launch holds."""
+    import torch
+    import xavs2_gb300 as xg
+    import xavs2_gb300.synth as synth
+    rng = np.random.default_rng(n)
+    w, h = 264, 200
+    yy, xx = np.mgrid[0:h, 0:w]
+    cur = (((xx ^ yy) & 1) * 255).astype(np.uint8)
+    cur[:64, :64] = 255
+    cur[64:, 128:] = rng.integers(0, 2, (h - 64, w - 128)) * 255
+    refs = [255 - cur, np.zeros_like(cur)]
+    cands, n_cu = synth.skip_candidates(rng, w, h, 2, motion=(-4, 6), cand_dtype=xg.SKIP_CAND_DTYPE)
+    at = int(rng.integers(0, max(1, len(cands) - n)))
+    cands = np.ascontiguousarray(cands[at:at + n])
+    lam = 3.5
+    flats, tab, stride = _planes(olib, refs)
+    e_dist, e_cost, e_best = np.zeros(len(cands), np.int32), np.zeros(len(cands)), np.zeros(n_cu, np.int32)
+    olib.xo_skip_costs(oracle.ptr(cur), w, tab, stride, w, h, 2, oracle.ptr(cands), len(cands), lam, n_cu,
+                       oracle.ptr(e_dist), oracle.ptr(e_cost), oracle.ptr(e_best))
+    sess = xg.MeSession(w, h, 2, 1)
+    sess.set_picture(-1, cur)
+    for i, r in enumerate(refs):
+        sess.set_picture(i, r)
+    sess.sync()
+    d_c = torch.from_numpy(cands.view(np.uint8).copy()).cuda()
+    d_dist = torch.zeros(len(cands), dtype=torch.int32, device="cuda")
+    d_cost = torch.zeros(len(cands), dtype=torch.float64, device="cuda")
+    d_best = torch.zeros(n_cu, dtype=torch.int32, device="cuda")
+    rc = gpu.xavs2gpu_skip_costs(ctypes.c_void_p(sess.h), ctypes.c_void_p(d_c.data_ptr()), len(cands), lam,
+                                 n_cu, ctypes.c_void_p(d_dist.data_ptr()), ctypes.c_void_p(d_cost.data_ptr()),
+                                 ctypes.c_void_p(d_best.data_ptr()), None)
+    assert rc == 0
+    sess.sync()
+    assert np.array_equal(d_dist.cpu().numpy(), e_dist)
+    assert np.array_equal(d_cost.cpu().numpy(), e_cost)
+    assert np.array_equal(d_best.cpu().numpy(), e_best)
+    sess.close()

@@ -9,6 +9,8 @@
 // same CU is not evaluated (update_skip_mv_list, rdo.c:2366-2389).
 #include "xavs2gpu_common.cuh"
 
+#include <algorithm>
+
 namespace xg {
 namespace skp {
 
@@ -105,15 +107,37 @@ __device__ __forceinline__ uint32_t ld4u(const uint8_t *p)
 // bytewise (a + b + 1) >> 1 of four packed samples (pixel_avg, pixel.c:680-700)
 __device__ __forceinline__ uint32_t avg4(uint32_t a, uint32_t b) { return (a | b) - (((a ^ b) >> 1) & 0x7F7F7F7Fu); }
 
-// |H8 (src - pred) H8^T| of the 8x8 block at (X, Y); the prediction of
-// sample (x, y) comes from src4[(y >= 4) * 2 + (x >= 4)] (four 4x4 PUs of an
-// 8x8 CU) or from src4[0] everywhere, relative to each PU's own corner.
+// |H8 (src - pred) H8^T| of the 8x8 block at (X, Y), predicted by candidate
+// k's PU `pu`, or (QUAD) by its four 4x4 PUs, the block's quadrants.
 // Rows are read as words: the current block's aligned, the prediction's at
 // any alignment.
-template <bool QUAD>
-__device__ int hsum8_pred(const Ctx &c, int X, int Y, const PuSrc *src4)
+// Samples k and k + 4 of a row share an integer (hi * 2^16 + lo, signed), so a
+// plain add or subtract is one butterfly of both; the last stage, across the
+// two halves, is |a + b| + |a - b| = 2 max(|a|, |b|), taken of two integers'
+// halves at a time with the values (at most 8160 before it) biased to unsigned.
+// Half the instructions and registers of 64 separate samples.
+constexpr uint32_t kSkipBias = 0x20002000u;
+__device__ __forceinline__ void byte_pairs(uint32_t lo, uint32_t hi, uint32_t (&q)[4])
 {
-    int m[8][8];
+    const uint32_t t = __byte_perm(lo, hi, 0x5140), u = __byte_perm(lo, hi, 0x7362);   // b0 b4 b1 b5 | b2 b6 b3 b7
+    q[0] = __byte_perm(t, 0, 0x7170);
+    q[1] = __byte_perm(t, 0, 0x7372);
+    q[2] = __byte_perm(u, 0, 0x7170);
+    q[3] = __byte_perm(u, 0, 0x7372);
+}
+__device__ __forceinline__ void butterfly(uint32_t &a, uint32_t &b)
+{
+    const uint32_t s = a + b;
+    b = a - b;
+    a = s;
+}
+
+template <bool QUAD>
+__device__ int hsum8_pred(const Ctx &c, const xavs2gpu_skip_cand_t &k, int X, int Y, int pu)
+{
+    uint32_t m[8][4];   // [row][k]: columns k and k + 4
+    PuSrc src[2];       // of the block, or of the quadrants of rows y .. y + 3
+    if (!QUAD) src[0] = pu_src(c, k, pu, X, Y);
 #pragma unroll
     for (int y = 0; y < 8; y++) {
         // the current picture is the session's plane: stride a multiple of
@@ -122,9 +146,12 @@ __device__ int hsum8_pred(const Ctx &c, int X, int Y, const PuSrc *src4)
         const uint32_t c0 = cw.x, c1 = cw.y;
         uint32_t pw[2];
         if (QUAD) {
+            if ((y & 3) == 0)
+#pragma unroll
+                for (int h = 0; h < 2; h++) src[h] = pu_src(c, k, (y >> 2) * 2 + h, X + 4 * h, Y + y);
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const PuSrc &ps = src4[(y >= 4) * 2 + h];
+                const PuSrc &ps = src[h];
                 const long long o = (long long)(y & 3) * c.stride;
                 const uint32_t a = ld4u(ps.p[0] + o);
                 pw[h] = ps.n == 2 ? avg4(a, ld4u(ps.p[1] + o)) : a;   // one list: the plane's samples
@@ -140,50 +167,61 @@ __device__ int hsum8_pred(const Ctx &c, int X, int Y, const PuSrc *src4)
                 hi = __funnelshift_r(w1, w2, sh);
             };
             const long long o = (long long)y * c.stride;
-            ld8u(src4[0].p[0] + o, pw[0], pw[1]);
-            if (src4[0].n == 2) {
+            ld8u(src[0].p[0] + o, pw[0], pw[1]);
+            if (src[0].n == 2) {
                 uint32_t b0, b1;
-                ld8u(src4[0].p[1] + o, b0, b1);
+                ld8u(src[0].p[1] + o, b0, b1);
                 pw[0] = avg4(pw[0], b0);
                 pw[1] = avg4(pw[1], b1);
             }
         }
-        int t[8];
+        uint32_t cq[4], pq[4];
+        byte_pairs(c0, c1, cq);
+        byte_pairs(pw[0], pw[1], pq);
 #pragma unroll
-        for (int x = 0; x < 8; x++) {
-            const uint32_t cv = x < 4 ? c0 : c1, pv = pw[x >> 2];
-            t[x] = (int)((cv >> (8 * (x & 3))) & 0xFFu) - (int)((pv >> (8 * (x & 3))) & 0xFFu);
+        for (int x = 0; x < 4; x++) m[y][x] = cq[x] - pq[x];
+        butterfly(m[y][0], m[y][1]);
+        butterfly(m[y][2], m[y][3]);
+        butterfly(m[y][0], m[y][2]);
+        butterfly(m[y][1], m[y][3]);
+    }
+    uint32_t s = 0;
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1)
+#pragma unroll
+            for (int y = 0; y < 8; y++)
+                if (!(y & d)) butterfly(m[y][x], m[y + d][x]);
+#pragma unroll
+        for (int y = 0; y < 8; y += 2) {
+            const uint32_t u = m[y][x] + kSkipBias, v = m[y + 1][x] + kSkipBias;
+            const uint32_t a = __byte_perm(u, v, 0x5410), b = __byte_perm(u, v, 0x7632);
+            s = __dp2a_lo(__vmaxu2(__vmaxu2(a, b), 2 * kSkipBias - __vminu2(a, b)), 0x0101u, s);
         }
-        int u[8];
-#pragma unroll
-        for (int i = 0; i < 4; i++) { u[i] = t[i] + t[i + 4]; u[i + 4] = t[i] - t[i + 4]; }
-        fwht4_d(u[0], u[1], u[2], u[3]);
-        fwht4_d(u[4], u[5], u[6], u[7]);
-#pragma unroll
-        for (int x = 0; x < 8; x++) m[y][x] = u[x];
     }
-    int s = 0;
-#pragma unroll
-    for (int x = 0; x < 8; x++) {
-        int u[8];
-#pragma unroll
-        for (int i = 0; i < 4; i++) { u[i] = m[i][x] + m[i + 4][x]; u[i + 4] = m[i][x] - m[i + 4][x]; }
-        fwht4_d(u[0], u[1], u[2], u[3]);
-        fwht4_d(u[4], u[5], u[6], u[7]);
-#pragma unroll
-        for (int i = 0; i < 8; i++) s += iabs_d(u[i]);
-    }
-    return s;
+    return 2 * ((int)s - 32 * 0x2000);
 }
 
-// 1. per-size counts (warp-aggregated); malformed candidates are reported here
+// Candidate classes: by CU size (0..3: 8x8 .. 64x64), the 8x8 CUs with four 4x4
+// PUs by themselves (4: their code reads quadrants, and a warp that held both
+// kinds ran both).
+constexpr int kClasses = 5;
+__device__ __forceinline__ int class_of(const xavs2gpu_skip_cand_t &k)
+{
+    const int sl = k.size_log2;
+    if (sl < 3 || sl > 6) return -1;
+    return sl == 3 && k.n_pu == 4 ? 4 : sl - 3;
+}
+__device__ __forceinline__ int class_lanes(int cl) { return cl == 4 ? 1 : min(32, 1 << (2 * cl)); }
+
+// 1. per-class counts (warp-aggregated); malformed candidates are reported here
 __global__ void skip_count_kernel(Ctx c, int *__restrict__ counts)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     int cl = -1;
     if (i < c.n) {
-        const int sl = c.cands[i].size_log2;
-        cl = (sl >= 3 && sl <= 6) ? sl - 3 : -1;
+        cl = class_of(c.cands[i]);
         if (cl < 0) {
             c.dist[i] = -1;
             c.cost[i] = (double)(1LL << 50);
@@ -196,104 +234,109 @@ __global__ void skip_count_kernel(Ctx c, int *__restrict__ counts)
     }
 }
 
-// 2. scatter into size order
+// 2. scatter into class order; a candidate that is not evaluated enters as ~i.
+// (The comparison with the CU's earlier candidates is a chain of dependent
+// reads: here a thread per candidate hides it, in the cost kernel it stood
+// before every warp's gathers.)
 __global__ void skip_scatter_kernel(Ctx c, const int *__restrict__ counts, int *__restrict__ cursor,
                                     int *__restrict__ sorted)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    int cl = -1;
-    if (i < c.n) {
-        const int sl = c.cands[i].size_log2;
-        cl = (sl >= 3 && sl <= 6) ? sl - 3 : -1;
-    }
+    const int cl = i < c.n ? class_of(c.cands[i]) : -1;
     const unsigned valid = __ballot_sync(0xffffffffu, cl >= 0);
     if (cl < 0) return;
     const unsigned same = __match_any_sync(valid, cl);
     const int leader = __ffs(same) - 1;
     int base = 0;
     if (lane == leader) base = atomicAdd(&cursor[cl], __popc(same));
+    const bool ok = cand_ok(c, i, c.cands[i]);
+    __syncwarp(same);
     base = __shfl_sync(same, base, leader);
     int start = 0;
     for (int k = 0; k < cl; k++) start += counts[k];
-    sorted[start + base + __popc(same & ((1u << lane) - 1))] = i;
+    sorted[start + base + __popc(same & ((1u << lane) - 1))] = ok ? i : ~i;
 }
 
-// 3. costs: a warp takes 32 / L candidates of one size, L = min(32, number
+// 3. costs: a warp takes 32 / L candidates of one class, L = min(32, number
 // of 8x8 blocks) lanes each; lane s of a candidate takes 8x8 blocks s and
 // s + 32 in z-order, so the four blocks of a 16x16 SA8D unit sit in four
 // consecutive lanes (their sums are rounded together, pixel.c:470-500).
-// resident 128-thread CTAs per SM the register budget is sized for (4: 128
-// registers; the kernel waits on plane gathers, and 4 CTAs measured faster
-// than 3 (the compiler's own 134 registers), 5 and 6)
+// The CTAs that fit walk the warps' worth of work, largest CUs first (the
+// number of warps is known on the device alone: a grid for the most there
+// could be, one per candidate, was 92 % empty CTAs for a 1080p picture).
+// Bound by the latency of its plane gathers: XG_SKIP_MINB resident 128-thread
+// CTAs (a 1080p picture's 214,500 candidates, whole call: 4 CTAs of 128
+// registers 50.4 us, 6 48.8, 8 47.0; 110 before the classes, the walk, the
+// repeated-motion check in the scatter and the paired transform).
 #ifndef XG_SKIP_MINB
-#define XG_SKIP_MINB 4
+#define XG_SKIP_MINB 8
 #endif
 __global__ void __launch_bounds__(128, XG_SKIP_MINB) skip_cost_kernel(Ctx c, const int *__restrict__ counts,
                                                                       const int *__restrict__ sorted)
 {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    int start = 0, first = 0, cl = -1;
-    for (int k = 0; k < 4; k++) {
-        const int L = min(32, 1 << (2 * k)), groups = (counts[k] * L + 31) / 32;
-        if (cl < 0 && warp < first + groups) {
-            cl = k;
-            start += (warp - first) * (32 / L);
-            break;
-        }
-        first += groups;
-        start += counts[k];
-    }
-    if (cl < 0) return;
-    const int L = min(32, 1 << (2 * cl)), nsub = 1 << (2 * cl);
-    const int slot = lane / L, sub = lane - slot * L;
-    const int end = [&]() { int e = 0; for (int k = 0; k <= cl; k++) e += counts[k]; return e; }();
-    const int pos = start + slot;
-    const bool live = pos < end;
-    const int i = live ? sorted[pos] : -1;
-    xavs2gpu_skip_cand_t k{};
-    bool ok = false;
-    if (live) {
-        k = c.cands[i];
-        if (sub == 0) ok = cand_ok(c, i, k);
-    }
-    ok = __shfl_sync(0xffffffffu, ok, lane - sub) && live;
-    int acc = 0;
-    const int S = ok ? 1 << k.size_log2 : 8, hp = k.n_pu == 4 ? S >> 1 : S;
-    const bool quad = ok && k.n_pu == 4 && S == 8;
-    for (int s0 = 0; s0 < nsub; s0 += 32) {   // the same trip count for every lane of the warp
-        const int s = s0 + sub;
-        int h = 0;
-        if (ok && s < nsub) {
-            // z-order position of 8x8 block s
-            int bx = 0, by = 0;
+    int cnt[kClasses];
 #pragma unroll
-            for (int b = 0; b < 3; b++) {
-                bx |= ((s >> (2 * b)) & 1) << b;
-                by |= ((s >> (2 * b + 1)) & 1) << b;
+    for (int k = 0; k < kClasses; k++) cnt[k] = counts[k];
+    for (int item = warp;; item += gridDim.x * (blockDim.x >> 5)) {
+        int cl = -1, pos = 0, end = 0;   // this warp's class, first list position, the class's end
+        int first = 0;
+#pragma unroll
+        for (int t = 0; t < kClasses; t++) {
+            const int k = t < 3 ? 3 - t : t == 3 ? 4 : 0;   // 64x64, 32x32, 16x16, 8x8 of four PUs, 8x8
+            int start = 0;
+#pragma unroll
+            for (int j = 0; j < k; j++) start += cnt[j];
+            const int L = class_lanes(k), groups = (cnt[k] * L + 31) / 32;
+            if (cl < 0 && item < first + groups) {
+                cl = k;
+                pos = start + (item - first) * (32 / L);
+                end = start + cnt[k];
             }
-            const int X = k.x + 8 * bx, Y = k.y + 8 * by;
-            PuSrc src4[4];
-            if (quad) {
+            first += groups;
+        }
+        if (cl < 0) return;
+        const int L = class_lanes(cl), nsub = cl == 4 ? 1 : 1 << (2 * cl);
+        const int slot = lane / L, sub = lane - slot * L;
+        pos += slot;
+        const bool live = pos < end;
+        const int e = live ? sorted[pos] : -1, i = e < 0 ? ~e : e;
+        const bool ok = e >= 0;
+        // fields are read where they are used (a copy indexed by PU lives in
+        // local memory); lane 0 of a warp is always live, i = 0 stands in for -1
+        const xavs2gpu_skip_cand_t &k = c.cands[live ? i : 0];
+        int acc = 0;
+        const int hp = ok ? (1 << k.size_log2) >> (k.n_pu == 4) : 8;
+        for (int s0 = 0; s0 < nsub; s0 += 32) {   // the same trip count for every lane of the warp
+            const int s = s0 + sub;
+            int h = 0;
+            if (ok && s < nsub) {
+                // z-order position of 8x8 block s
+                int bx = 0, by = 0;
 #pragma unroll
-                for (int q = 0; q < 4; q++) src4[q] = pu_src(c, k, q, k.x + (q & 1) * 4, k.y + (q >> 1) * 4);
+                for (int b = 0; b < 3; b++) {
+                    bx |= ((s >> (2 * b)) & 1) << b;
+                    by |= ((s >> (2 * b + 1)) & 1) << b;
+                }
+                const int X = k.x + 8 * bx, Y = k.y + 8 * by;
+                if (cl == 4)
+                    h = hsum8_pred<true>(c, k, X, Y, 0);
+                else
+                    h = hsum8_pred<false>(c, k, X, Y, k.n_pu == 4 ? (8 * bx >= hp) + 2 * (8 * by >= hp) : 0);
+            }
+            if (cl == 0 || cl == 4) {
+                acc += (h + 2) >> 2;                          // one 8x8 SA8D unit
             } else {
-                const int q = k.n_pu == 4 ? (8 * bx >= hp) + 2 * (8 * by >= hp) : 0;
-                src4[0] = pu_src(c, k, q, X, Y);
+                h += __shfl_xor_sync(0xffffffffu, h, 1);      // the 16x16 unit of 4 lanes
+                h += __shfl_xor_sync(0xffffffffu, h, 2);
+                if ((sub & 3) == 0) acc += (h + 2) >> 2;
             }
-            h = quad ? hsum8_pred<true>(c, X, Y, src4) : hsum8_pred<false>(c, X, Y, src4);
         }
-        if (cl == 0) {
-            acc += (h + 2) >> 2;                          // one 8x8 SA8D unit
-        } else {
-            h += __shfl_xor_sync(0xffffffffu, h, 1);      // the 16x16 unit of 4 lanes
-            h += __shfl_xor_sync(0xffffffffu, h, 2);
-            if ((sub & 3) == 0) acc += (h + 2) >> 2;
+        for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (live && sub == 0) {
+            c.dist[i] = ok ? acc : -1;
+            c.cost[i] = ok ? __dadd_rn((double)acc, __dmul_rn(c.lambda, (double)k.rate)) : (double)(1LL << 50);
         }
-    }
-    for (int o = L >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (live && sub == 0) {
-        c.dist[i] = ok ? acc : -1;
-        c.cost[i] = ok ? __dadd_rn((double)acc, __dmul_rn(c.lambda, (double)k.rate)) : (double)(1LL << 50);
     }
 }
 
@@ -334,7 +377,7 @@ extern "C" int xavs2gpu_skip_costs(xavs2gpu_me_session_t *s, const xavs2gpu_skip
     if (n == 0) return XAVS2GPU_OK;
     skp::Ctx c{xavs2gpu_me_plane_device(s, -1, 0), xavs2gpu_me_plane_table_device(s), xavs2gpu_me_plane_stride(s), W, H,
                nrefs, cands, n, lambda, dist, cost};
-    // scratch: size counts and cursors, then the size-ordered list
+    // scratch: class counts and cursors, then the class-ordered list
     int *scratch = nullptr;
     XG_CUDA(cudaMallocAsync((void **)&scratch, sizeof(int) * (16 + (size_t)n), st));
     if (!scratch) return XAVS2GPU_ERR_CUDA;
@@ -343,8 +386,10 @@ extern "C" int xavs2gpu_skip_costs(xavs2gpu_me_session_t *s, const xavs2gpu_skip
     const int nb = (n + 255) / 256;
     skp::skip_count_kernel<<<nb, 256, 0, st>>>(c, counts);
     skp::skip_scatter_kernel<<<nb, 256, 0, st>>>(c, counts, cursor, sorted);
-    // warps: at most one per candidate (sizes with fewer lanes share warps)
-    skp::skip_cost_kernel<<<(unsigned)(((long long)n * 32 + 127) / 128), 128, 0, st>>>(c, counts, sorted);
+    // the CTAs that fit, or fewer where even a warp per candidate is fewer
+    const long long most = ((long long)n * 32 + 127) / 128;
+    skp::skip_cost_kernel<<<(unsigned)std::min<long long>(most, (long long)sm_count() * XG_SKIP_MINB), 128, 0, st>>>(
+        c, counts, sorted);
     count_launch(3);
     XG_CUDA(cudaFreeAsync(scratch, st));
     if (n_cus > 0) {
