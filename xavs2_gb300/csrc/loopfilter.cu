@@ -93,44 +93,35 @@ __device__ __forceinline__ uint32_t ge_bytes(uint32_t a, uint32_t b)
     const uint32_t t = (a | 0x80808080u) - (b & 0x7F7F7F7Fu);
     return ((a & ~b) | (~(a ^ b) & t)) & 0x80808080u;
 }
-// bytewise min(a + b, 255): the sum without carries between bytes, the
-// carry out of each byte, and a byte of ones where it is set
-__device__ __forceinline__ uint32_t addus_bytes(uint32_t a, uint32_t b)
-{
-    const uint32_t s = ((a & 0x7F7F7F7Fu) + (b & 0x7F7F7F7Fu)) ^ ((a ^ b) & 0x80808080u);
-    const uint32_t cy = ((a & b) | ((a | b) & ~s)) & 0x80808080u;
-    return s | cy | (cy - (cy >> 7));
-}
-// bytewise max(a - b, 0) = 255 - min(255 - a + b, 255)
-__device__ __forceinline__ uint32_t subus_bytes(uint32_t a, uint32_t b) { return ~addus_bytes(~a, b); }
+// the even and the odd samples of a word as 16-bit halves, and back
+__device__ __forceinline__ uint32_t even_halves(uint32_t w) { return w & 0x00FF00FFu; }
+__device__ __forceinline__ uint32_t odd_halves(uint32_t w) { return __byte_perm(w, 0, 0x4341); }
+__device__ __forceinline__ uint32_t join_halves(uint32_t ev, uint32_t od) { return __byte_perm(ev, od, 0x6240); }
 
-// SAO edge class per byte: sign(s - n1) + sign(s - n2) + 2, each term
-// sign(s - n) + 1 = [s >= n] + (1 - [n >= s]); the sum is at most 4
-__device__ __forceinline__ uint32_t eo_class(uint32_t s, uint32_t n1, uint32_t n2)
-{
-    const uint32_t H = 0x80808080u;
-    return ((ge_bytes(s, n1) >> 7) + (ge_bytes(s, n2) >> 7)) +
-           (((ge_bytes(n1, s) ^ H) >> 7) + ((ge_bytes(n2, s) ^ H) >> 7));
-}
-// the edge-offset table of eo_apply: the offsets of classes 0-4 clipped to
-// [0, 255] (words 0-1) and their negations clipped likewise (words 2-3)
+// the edge-offset table of eo_filter: the offsets of classes 0-4 plus 128
 __device__ __forceinline__ void eo_table(const int8_t *offset, uint32_t *tab)
 {
-    uint32_t ad[2] = {0, 0}, sb[2] = {0, 0};
-    for (int k = 0; k < 5; k++) {
-        const int o = offset[k];
-        ad[k >> 2] |= (uint32_t)min(max(o, 0), 255) << (8 * (k & 3));
-        sb[k >> 2] |= (uint32_t)min(max(-o, 0), 255) << (8 * (k & 3));
-    }
-    tab[0] = ad[0]; tab[1] = ad[1]; tab[2] = sb[0]; tab[3] = sb[1];
+    uint32_t t[2] = {0, 0};
+    for (int k = 0; k < 5; k++) t[k >> 2] |= (uint32_t)(offset[k] + 128) << (8 * (k & 3));
+    tab[0] = t[0];
+    tab[1] = t[1];
 }
-// clip(s + offset[class], 0, 255) per byte: the classes (0..4) packed into
-// the 4 selector nibbles of a byte permute over the offsets' positive and
-// negative parts (each clipped to 255, which leaves the clipped sum exact)
-__device__ __forceinline__ uint32_t eo_apply(uint32_t s, uint32_t cls, const uint32_t *tab)
+// clip(s + offset[class], 0, 255) of four samples, class = sign(s - n1) +
+// sign(s - n2) + 2.  In 16-bit halves, where the packed minimum and maximum are
+// single instructions: 256 + s - n clamped to 255 .. 257 is a sign plus 256; the
+// classes are the selector nibbles of a byte permute over the table.  32
+// instructions; compares and saturating sums put together bytewise took 47.
+__device__ __forceinline__ uint32_t eo_filter(uint32_t s, uint32_t n1, uint32_t n2, const uint32_t *tab)
 {
-    const uint32_t sel = __byte_perm(cls | (cls >> 4), 0, 0x0020);
-    return subus_bytes(addus_bytes(s, __byte_perm(tab[0], tab[1], sel)), __byte_perm(tab[2], tab[3], sel));
+    auto sign = [](uint32_t a, uint32_t b) {
+        return __vminu2(__vmaxu2((a | 0x01000100u) - b, 0x00FF00FFu), 0x01010101u);
+    };
+    const uint32_t se = even_halves(s), so = odd_halves(s);
+    const uint32_t ce = sign(se, even_halves(n1)) + sign(se, even_halves(n2)) - 0x01FE01FEu;
+    const uint32_t co = sign(so, odd_halves(n1)) + sign(so, odd_halves(n2)) - 0x01FE01FEu;
+    const uint32_t o = __byte_perm(tab[0], tab[1], __byte_perm(ce + 16 * co, 0, 0x0020));
+    auto clip = [](uint32_t v) { return __vminu2(__vmaxu2(v, 0x00800080u), 0x017F017Fu) - 0x00800080u; };
+    return join_halves(clip(se + even_halves(o)), clip(so + odd_halves(o)));
 }
 
 // Four lines across one edge at once, a line per byte lane: w[0..5] hold
@@ -504,7 +495,7 @@ __global__ void __launch_bounds__(kSaoThreads, 8) sao_lcu_kernel(SaoPic sp)
     __shared__ int off[32];
     __shared__ int nb[8][7];
     __shared__ int n_nb;
-    __shared__ uint32_t eo_tab[4];
+    __shared__ uint32_t eo_tab[2];
     if (threadIdx.x < 32) off[threadIdx.x] = q.offset[c][threadIdx.x];
     if (threadIdx.x == 32) eo_table(q.offset[c], eo_tab);
     if (threadIdx.x == 0) {
@@ -608,7 +599,7 @@ __global__ void __launch_bounds__(kSaoThreads, 8) sao_lcu_kernel(SaoPic sp)
             case 2: n1 = lft(0); n2 = rgt(2); break;
             default: n1 = rgt(0); n2 = lft(2); break;
             }
-            res = eo_apply(cur, eo_class(cur, n1, n2), eo_tab);
+            res = eo_filter(cur, n1, n2, eo_tab);
         }
         const uint32_t m = ((wrote * 0x00204081u) & 0x01010101u) * 0xFFu;   // bit k -> byte k
         const uint32_t out = (res & m) | (old & ~m);
@@ -688,9 +679,9 @@ __device__ __forceinline__ void deblock_tile(uint8_t (*t)[kLfPitch], const uint3
 }
 
 #ifndef XG_LF_MINB
-// resident CTAs per SM the register budget is sized for (0: the compiler's
-// choice, 48 registers and 10 CTAs; 16 CTAs at 32 registers, a few spilled
-// words, measured 0.041 against 0.044 ms per 2160p picture, 12 CTAs 0.044)
+// resident CTAs per SM the register budget is sized for (16: 32 registers, a
+// few spilled words, 36.2 us per 2160p picture; 12 and 0, the compiler's choice,
+// 36.9; 38.4 with bytewise SAO and its row range worked out for every row)
 #define XG_LF_MINB 16
 #endif
 __global__ void
@@ -704,7 +695,8 @@ loopfilter_lcu_kernel(FusedPic fp)
     __shared__ __align__(16) uint8_t t[kLfRows][kLfPitch];
     __shared__ uint32_t ev[kLfScus], eh[kLfScus];   // edge words, vertical / horizontal
     __shared__ int off[32];
-    __shared__ uint32_t eo_tab[4];   // edge-offset classes 0-4: added bytes (words 0-1), subtracted (2-3)
+    __shared__ uint32_t eo_tab[2];
+    __shared__ int rng[3][2];        // SAO's column range of the first, the middle and the last rows
     const int l = blockIdx.x, c = blockIdx.y, tid = threadIdx.x, nt = blockDim.x;
     const bool chroma = c != 0;
     const int lx = l % fp.wl, ly = l / fp.wl;
@@ -718,6 +710,15 @@ loopfilter_lcu_kernel(FusedPic fp)
     const int tx0 = max(rx - 8, 0), tx1 = min(rx + rw + 8, W), ty0 = max(ry - 8, 0), ty1 = min(ry + rh + 8, H);
     if (tid < 32) off[tid] = q.offset[c][tid];
     if (tid == 32) eo_table(q.offset[c], eo_tab);
+    if (tid >= 64 && tid < 67) {
+        const int k = tid - 64;
+        int x0 = 0, x1 = 0;
+        if (q.type[c] < 0 || q.type[c] > 4 ||
+            !sao_row_range(q.type[c], full_avail(q.avail), k == 0 ? 0 : k == 1 ? 1 : rh - 1, rw, rh, x0, x1))
+            x0 = x1 = 0;
+        rng[k][0] = x0;
+        rng[k][1] = x1;
+    }
     // edge words of the 8x8 blocks the tile touches
     const int sh = chroma ? 2 : 3;
     const int sx0 = tx0 >> sh, sy0 = ty0 >> sh, nsx = ((tx1 - 1) >> sh) - sx0 + 1, nsy = ((ty1 - 1) >> sh) - sy0 + 1;
@@ -758,7 +759,7 @@ loopfilter_lcu_kernel(FusedPic fp)
     // SAO of the region from the deblocked tile, a word (4 samples) at a
     // time; dst written whole; a thread keeps one word column and walks the
     // rows
-    const int ty = q.type[c], av = full_avail(q.avail), rwords = rw >> 2;
+    const int ty = q.type[c], rwords = rw >> 2;
     const int wi = tid % rwords, r0 = tid / rwords, rs = nt / rwords;
     if (r0 >= rs) return;
     const int x = rx + 4 * wi;
@@ -768,9 +769,9 @@ loopfilter_lcu_kernel(FusedPic fp)
         const uint8_t *d = &t[y - ty0][x - tx0];
         const uint32_t cur = *reinterpret_cast<const uint32_t *>(d);
         uint32_t out = cur;
-        int x0 = 0, x1 = 0;
-        if (ty >= 0 && ty <= 4 && sao_row_range(ty, av, yy, rw, rh, x0, x1)) {
-            const int lo = max(x0 - 4 * wi, 0), hi = min(x1 - 4 * wi, 4);
+        const int rk = yy == 0 ? 0 : yy == rh - 1 ? 2 : 1;
+        {
+            const int lo = max(rng[rk][0] - 4 * wi, 0), hi = min(rng[rk][1] - 4 * wi, 4);
             if (lo < hi) {
                 uint32_t res;
                 if (ty == 4) {
@@ -800,7 +801,7 @@ loopfilter_lcu_kernel(FusedPic fp)
                     case 2: n1 = lft(-1); n2 = rgt(1); break;
                     default: n1 = rgt(-1); n2 = lft(1); break;
                     }
-                    res = eo_apply(cur, eo_class(cur, n1, n2), eo_tab);
+                    res = eo_filter(cur, n1, n2, eo_tab);
                 }
                 const uint32_t m = (0xFFFFFFFFu << (8 * lo)) & (0xFFFFFFFFu >> (8 * (4 - hi)));
                 out = (res & m) | (cur & ~m);
