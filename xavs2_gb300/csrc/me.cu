@@ -982,51 +982,26 @@ __global__ void __launch_bounds__(128, XG_REFINE_MINB) refine_thread_kernel(cons
     out[i] = res;
 }
 
-// Warp-cooperative cost of the PU at quarter-pel (mx, my): lanes take the
-// PU's rounding units (4x4 or 8x4; the same tiling sums the SAD) in turn,
-// rows read as aligned words.
-__device__ int qpel_cost_warp_vec(const xavs2gpu_pu_t &p, int w, int h, bool had, const uint8_t *o,
-                                  const uint8_t *const *planes, int stride, int mx, int my, int lane)
-{
-    const bool u4 = had ? satd_unit4(w, h) : (w == 4 || w == 12);
-    const int uw = u4 ? 4 : 8, nux = w / uw, nu = nux * (h >> 2);
-    const uint8_t *r = planes[((my & 3) << 2) + (mx & 3)] + (ptrdiff_t)(p.y + (my >> 2)) * stride + p.x + (mx >> 2);
-    int s = 0;
-    for (int u = lane; u < nu; u += 32) {
-        const int uy = u / nux, ux = u - uy * nux;
-        const ptrdiff_t off = (ptrdiff_t)uy * 4 * stride + ux * uw;
-        UnitC c;
-        if (u4) {
-            load_unit<true>(o + off, stride, c);
-            s += unit_cost_pre<true>(had, c, r + off, stride);
-        } else {
-            load_unit<false>(o + off, stride, c);
-            s += unit_cost_pre<false>(had, c, r + off, stride);
-        }
-    }
-    return warp_sum_i(s);
-}
-
-// One warp per search for the larger PUs, over a list.
+// One warp per search for the larger PUs, over a list.  Per stage the lanes take
+// (position, unit) pairs, position by position, and add their costs in shared
+// memory: a 16x16 PU has 8 units, so a warp that took the positions one after the
+// other left 24 lanes idle in each of 17 passes (416x240, every PU a warp: 141
+// us, 70 now; the 64x64 PUs' 68 passes are what remains).
 __global__ void __launch_bounds__(128) refine_warp_list_kernel(const uint32_t *__restrict__ list, int n,
                                                                const SessView *__restrict__ views, int R,
                                                                xavs2gpu_me_params_t prm)
 {
-    const int wt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    __shared__ int s_cost[4][9], s_mx[4][9], s_my[4][9];
+    const int wt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (wt >= n) return;
     const uint32_t e = list[wt];
     const SessView &v = views[e >> kSessShift];
     const int i = (int)(e & kIdxMask);
-    const xavs2gpu_pu_t *__restrict__ pus = v.pus;
-    const PuState *__restrict__ state = v.state;
-    const unsigned long long *__restrict__ keys = v.keys;
-    const uint8_t *__restrict__ cur = v.cur;
-    const uint8_t *const *ref_planes = v.planes;
     const Geometry g = v.g;
     xavs2gpu_me_result_t *__restrict__ out = v.res;
-    const xavs2gpu_pu_t p = pus[i];
-    const PuState st = state[i];
-    const unsigned long long key = keys[i];
+    const xavs2gpu_pu_t p = v.pus[i];
+    const PuState st = v.state[i];
+    const unsigned long long key = v.keys[i];
     xavs2gpu_me_result_t res;
     if (!st.valid || key == kNoKey) {
         res.bmv_x = res.bmv_y = res.imv_x = res.imv_y = 0;
@@ -1050,34 +1025,69 @@ __global__ void __launch_bounds__(128) refine_warp_list_kernel(const uint32_t *_
     if (prm.fractional_me) {
         const int w = c_pu_w[p.part], h = c_pu_h[p.part];
         const bool had = prm.use_hadamard != 0;
-        const uint8_t *o = cur + (ptrdiff_t)p.y * g.stride + p.x;
-        const uint8_t *const *planes = ref_planes + 16 * p.ref;
+        const bool u4 = had ? satd_unit4(w, h) : (w == 4 || w == 12);
+        const int uw = u4 ? 4 : 8, nux = w / uw, nu = nux * (h >> 2);
+        const int mu = (65536 + nu - 1) / nu, mx1 = (65536 + nux - 1) / nux;   // e / nu, u / nux: exact below 9 nu, nu
+        const uint8_t *o = v.cur + (ptrdiff_t)p.y * g.stride + p.x;
+        const uint8_t *const *planes = v.planes + 16 * p.ref;
         const int pat = prm.fast_sub_me ? 1 : 0, step = prm.fast_sub_me ? 2 : 1;
-        int cx = bx, cy = by;
-        if (had) best = qpel_cost_warp_vec(p, w, h, true, o, planes, g.stride, cx, cy, lane) + mv_cost_hd(lam, cx, cy, pmx, pmy);
-        for (int pos = 1; pos < 9; pos += step) {
-            int mx = cx + 2 * c_spiral[pat][pos][0], my = cy + 2 * c_spiral[pat][pos][1];
-            int c = qpel_cost_warp_vec(p, w, h, had, o, planes, g.stride, mx, my, lane) + mv_cost_hd(lam, mx, my, pmx, pmy);
-            if (c < best) { best = c; bx = mx; by = my; }
-        }
-        if (prm.fractional_me > 1) {
-            cx = bx; cy = by;
-            const int ctr_x = (pmx >> 1) << 1, ctr_y = (pmy >> 1) << 1;
-            for (int pos = 1; pos < 9; pos += step) {
-                int sx = c_spiral[pat][pos][0], sy = c_spiral[pat][pos][1], mx, my;
-                if (prm.enable_pmvr) {
-                    if (abs(cx - ctr_x) > 2 || abs(cy - ctr_y) > 2) {
-                        mx = cx + 2 * sx; my = cy + 2 * sy;
-                        if (abs(mx - ctr_x) <= 2 && abs(my - ctr_y) <= 2) continue;
+        const int ctr_x = (pmx >> 1) << 1, ctr_y = (pmy >> 1) << 1;
+        for (int stage = 0; stage < (prm.fractional_me > 1 ? 2 : 1); stage++) {
+            // lane k: position k (with SATD the first stage begins at the centre)
+            const int k0 = stage == 0 && had ? 1 : 0, count = k0 + 8 / step;
+            bool ok = lane < count;
+            int mx = bx, my = by;
+            if (ok && lane >= k0) {
+                const int pos = 1 + (lane - k0) * step, sx = c_spiral[pat][pos][0], sy = c_spiral[pat][pos][1];
+                const int two = stage == 0 ? 2 : 1;
+                mx = bx + two * sx;
+                my = by + two * sy;
+                if (stage == 1 && prm.enable_pmvr) {
+                    // pmvr_adapt_mv (me.c:412-424), TH_PMVR = 2
+                    if (abs(bx - ctr_x) > 2 || abs(by - ctr_y) > 2) {
+                        mx = bx + 2 * sx; my = by + 2 * sy;
+                        ok = !(abs(mx - ctr_x) <= 2 && abs(my - ctr_y) <= 2);
                     } else {
-                        mx = cx + sx; my = cy + sy;
-                        if (abs(mx - ctr_x) > 2 || abs(my - ctr_y) > 2) continue;
+                        ok = !(abs(mx - ctr_x) > 2 || abs(my - ctr_y) > 2);
                     }
-                } else {
-                    mx = cx + sx; my = cy + sy;
                 }
-                int c = qpel_cost_warp_vec(p, w, h, had, o, planes, g.stride, mx, my, lane) + mv_cost_hd(lam, mx, my, pmx, pmy);
-                if (c < best) { best = c; bx = mx; by = my; }
+            }
+            if (lane < count) {
+                s_mx[warp][lane] = mx;
+                s_my[warp][lane] = my;
+                s_cost[warp][lane] = 0;
+            }
+            const unsigned oks = __ballot_sync(0xffffffffu, ok);
+            __syncwarp();
+            for (int q = lane; q < count * nu; q += 32) {
+                const int k = (q * mu) >> 16, u = q - k * nu, uy = (u * mx1) >> 16, ux = u - uy * nux;
+                if (!((oks >> k) & 1)) continue;
+                const ptrdiff_t off = (ptrdiff_t)uy * 4 * g.stride + ux * uw;
+                const int qx = s_mx[warp][k], qy = s_my[warp][k];
+                const uint8_t *r = planes[((qy & 3) << 2) + (qx & 3)] + (ptrdiff_t)(p.y + (qy >> 2)) * g.stride + p.x +
+                                   (qx >> 2) + off;
+                UnitC c;
+#if XG_REFINE_PACKED
+                load_unit_rt(o + off, g.stride, c, u4);
+                atomicAdd(&s_cost[warp][k], unit_cost_pre_rt(had, u4, c, r, g.stride));
+#else
+                if (u4) load_unit<true>(o + off, g.stride, c);
+                else load_unit<false>(o + off, g.stride, c);
+                atomicAdd(&s_cost[warp][k], u4 ? unit_cost_pre<true>(had, c, r, g.stride)
+                                               : unit_cost_pre<false>(had, c, r, g.stride));
+#endif
+            }
+            __syncwarp();
+            // the first position of the least cost; without the centre among
+            // them it must be strictly smaller than the cost so far
+            const int c = ok ? s_cost[warp][lane] + mv_cost_hd(lam, mx, my, pmx, pmy) : 0x7fffffff;
+            const int least = __reduce_min_sync(0xffffffffu, c);
+            const unsigned at = __ballot_sync(0xffffffffu, ok && c == least);
+            if (at && (k0 || least < best)) {
+                const int win = __ffs(at) - 1;
+                best = least;
+                bx = __shfl_sync(0xffffffffu, mx, win);
+                by = __shfl_sync(0xffffffffu, my, win);
             }
         }
     }
