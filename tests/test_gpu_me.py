@@ -99,6 +99,28 @@ def test_ctu_rows_per_cta(gpu, olib, R, w, h, nrefs, extra):
     _assert_same(got, _oracle(olib, cur, [ref0, ref1][:nrefs], pus, prm), pus)
 
 
+@pytest.mark.parametrize("R,w,h,nrefs,extra", [(20, 776, 648, 2, 200), (28, 1288, 968, 2, 200), (28, 72, 136, 1, 200),
+                                               (36, 520, 392, 1, 100), (50, 200, 136, 2, 60), (60, 760, 632, 1, 60),
+                                               (60, 416, 240, 4, 20), (92, 200, 136, 1, 0), (124, 200, 136, 1, 0)])
+def test_ctu_ranges_off_sixteen(gpu, olib, R, w, h, nrefs, extra):
+    """Ranges that are no multiple of 16: windows off the 16-byte boundary,
+    2R = 4 mod 8, and 72 + 2R a multiple of 64 (28, 60, 92, 124), where the
+    last samples of a window row fill its staging area to the end."""
+    import xavs2_gb300 as xg
+    rng = np.random.default_rng(R + w + nrefs)
+    cur, ref0 = _frames(rng, w, h)
+    refs = [ref0] + [_frames(rng, w, h, shift=(-3, 4 + k))[1] for k in range(nrefs - 1)]
+    pus = xg.frame_pus(w, h, nrefs)
+    order = rng.permutation(len(pus))
+    ctu = (pus["ref"].astype(np.int64) << 32) + ((pus["y"].astype(np.int64) >> 6) << 16) + (pus["x"] >> 6)
+    _, first = np.unique(ctu[order], return_index=True)
+    pus = pus[np.unique(np.concatenate([order[first], order[:extra]]))]
+    prm = xg.MeParams(R, oracle.lambda_factor(32), 1, 0, 0, 0)
+    got, stats = _run(cur, refs, pus, prm)
+    assert stats[0] == len(pus) and stats[1] == 0, stats
+    _assert_same(got, _oracle(olib, cur, refs, pus, prm), pus)
+
+
 @pytest.mark.parametrize("lam,on_ctu", [(1 << 25, True), (1 << 27, False)])
 def test_large_lambda(gpu, olib, lam, on_ctu):
     """Large MV costs: lambda 2^25 keeps the CTU search (its 32-bit keys hold

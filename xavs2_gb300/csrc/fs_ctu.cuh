@@ -43,13 +43,12 @@
 // PUs containing such a block then never win and are not merged.
 #pragma once
 
+#include "ctu_layout.h"
+
 namespace xg {
 
 constexpr int kSlots = 849;
-constexpr int kCtuWarps = 4;
 constexpr int kCtuThreads = 32 * kCtuWarps;
-constexpr int kDyWarpMax = 8;           // search rows per warp: 8, 4 or 2 (3 key bits)
-constexpr int kDyChunkMax = kCtuWarps * kDyWarpMax;
 constexpr uint32_t kPoisonSmall = 126976u;     // > any valid cost of a PU up to 16x16
 constexpr uint32_t kPoisonLarge = 1u << 22;    // replaces a 4x4 SAD outside the limits
 constexpr uint32_t kCapLarge = 2000000u;       // > any valid cost of a 64x64 PU
@@ -151,25 +150,6 @@ __device__ __forceinline__ uint32_t addmin(uint32_t a, uint32_t b, uint32_t c)
 {
     return __viaddmin_u32(a, b, c);   // min(a + b, c)
 }
-
-// Window layout in 8-byte entries: a row is ctu_pitch(R) entries (15 + R/2:
-// word 4*rx + c + (displacement >> 2) of rx, c <= 3), one entry is skipped
-// after every 8 rows, and the second plane follows the first.  An 8-byte shared
-// load serves 16 lanes at a time; lane bits 0-3 are half, rx bit 0, ry bit 0 and
-// rx bit 1, so these read rows 8q + t of four consecutive q = 2*ry + half
-// (skewed by 0..3 entries) at entries 4*rx: 16 distinct pairs of banks.
-__host__ __device__ __forceinline__ int ctu_pitch(int R) { return 15 + (R >> 1); }
-__host__ __device__ __forceinline__ int ctu_entry(int row, int pitch) { return row * pitch + (row >> 3); }
-
-// bytes of a chunk's MV-cost keys and of its window (multiples of 128), and
-// the distance of the window's planes in entries
-__host__ __device__ __forceinline__ uint32_t ctu_key_bytes(int R, int dyw) { return 4u * (uint32_t)(kCtuWarps * dyw * 2 * R); }
-__host__ __device__ __forceinline__ uint32_t ctu_win_bytes(int R, int dyw)
-{
-    const int rows = 64 + kCtuWarps * dyw - 1;   // two planes of 8-byte entries
-    return (uint32_t)(ctu_entry(rows - 1, ctu_pitch(R)) + ctu_pitch(R) + 7) / 8 * 128;
-}
-__host__ __device__ __forceinline__ int ctu_plane(int R, int dyw) { return (int)(ctu_win_bytes(R, dyw) >> 4); }
 
 // slot of small key k (0..24) of a lane
 __device__ __forceinline__ int small_slot(int rx, int ry, int half, int k)
@@ -354,12 +334,7 @@ __device__ __forceinline__ void sad_at(const uint2 *win, int pitch, int row0, in
 #ifndef XG_CTU_TMA
 #define XG_CTU_TMA 1
 #endif
-constexpr int kTmaBoxCols = 64;
-constexpr int kTmaBoxRows = 64 + kDyChunkMax - 1;
-constexpr int kTmaPieceBytes = (kTmaBoxCols * kTmaBoxRows + 127) / 128 * 128;   // 6144
 constexpr int kWaitLimit = 1 << 20;   // mbarrier polls before a CTA gives up its window
-
-__host__ __device__ constexpr int tma_pieces(int R) { return (64 + 2 * R + 8 + kTmaBoxCols - 1) / kTmaBoxCols; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -438,7 +413,7 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
     unsigned long long *__restrict__ keys = view.keys;
     const int rows = kCtuWarps * dyw;                 // search rows of the chunk
     const int dy0 = -R + chunk * rows;
-    const int wrows = 64 + rows - 1, pitch = ctu_pitch(R), nd = 2 * R;
+    const int wrows = ctu_window_rows(dyw), pitch = ctu_pitch(R), nd = 2 * R;
     uint32_t *mvk = reinterpret_cast<uint32_t *>(smem);                      // [rows][nd] MV-cost keys
     uint2 *win = reinterpret_cast<uint2 *>(smem + ctu_key_bytes(R, dyw));    // the window's entries
     const int plane = ctu_plane(R, dyw);
@@ -489,15 +464,14 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
         for (int r = warp; r < wrows; r += kCtuWarps) {
             const uint8_t *row = ref + (ptrdiff_t)min(max(wy0 + r, -kPad), g.H + kPad - 1) * g.stride;
             for (int c = lane; c < 64 + 2 * R; c += 32)
-                stage[(c >> 6) * kTmaPieceBytes + r * kTmaBoxCols + (c & (kTmaBoxCols - 1))] =
-                    row[min(max(wx0 + c, -kPad), g.W + kPad - 1)];
+                stage[ctu_stage_at(r, c)] = row[min(max(wx0 + c, -kPad), g.W + kPad - 1)];
         }
         __syncthreads();
     }
     // four entries per item, the words of several items read before any is
     // placed (one item at a time waited for memory 40 times over)
     const bool from_stage = use_tma || (staged && !inside);
-    const int quads = (pitch + 3) >> 2, items = wrows * quads, mq = (65536 + quads - 1) / quads;
+    const int quads = ctu_quads(pitch), items = wrows * quads, mq = (65536 + quads - 1) / quads;
     auto place = [&](int r, int k, uint32_t lo, uint32_t hi) {
         if (k >= pitch) return;
         uint2 *d = win + ctu_entry(r, pitch) + k;
@@ -512,14 +486,14 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
 #pragma unroll
             for (int b = 0; b < NB; b++) {
                 const int e = min(e0 + b * kCtuThreads, items - 1), r = (e * mq) >> 16, q = e - r * quads;
+                const bool full = ctu_quad_full(q, pitch);   // else the word after is not there to read
                 if (from_stage) {
-                    const uint8_t *t = stage + r * kTmaBoxCols;
-                    v[b] = *reinterpret_cast<const uint4 *>(t + (q >> 2) * kTmaPieceBytes + 16 * (q & 3));
-                    nx[b] = *reinterpret_cast<const uint32_t *>(t + ((q + 1) >> 2) * kTmaPieceBytes + 16 * ((q + 1) & 3));
+                    v[b] = *reinterpret_cast<const uint4 *>(stage + ctu_stage_at(r, 16 * q));
+                    nx[b] = full ? *reinterpret_cast<const uint32_t *>(stage + ctu_stage_at(r, 16 * q + 16)) : 0u;
                 } else {
                     const uint4 *t = reinterpret_cast<const uint4 *>(ref + (ptrdiff_t)(wy0 + r) * g.stride + wx0) + q;
                     v[b] = __ldg(t);
-                    nx[b] = __ldg(reinterpret_cast<const uint32_t *>(t + 1));
+                    nx[b] = full ? __ldg(reinterpret_cast<const uint32_t *>(t + 1)) : 0u;
                 }
             }
 #pragma unroll
@@ -779,11 +753,6 @@ static void ctu_plan_build(CtuPlan &p, const std::vector<xavs2gpu_pu_t> &pus, in
 }
 
 constexpr int kCtuSmemMax = 227 * 1024;
-static inline size_t ctu_smem_bytes(int R, int dyw, bool staging)
-{
-    const size_t b = (size_t)ctu_key_bytes(R, dyw) + ctu_win_bytes(R, dyw);
-    return staging ? b + (size_t)tma_pieces(R) * kTmaPieceBytes + 16 : b;   // the boxes and their barrier
-}
 
 // The kernels' dynamic shared-memory limit (the largest range's need), once
 // per device; launches and occupancy queries come after it.
