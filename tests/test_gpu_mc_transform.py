@@ -413,3 +413,50 @@ def test_tq_batch_forms(gpu, olib, n):
             assert nnz[r * m + i] == nz
             assert np.array_equal(coef[r * coff + co:r * coff + co + nc], cf[:nc]), (i, p, r)
             assert np.array_equal(rec[r * off + o:r * off + o + k], blk), (i, p, r)
+
+
+def test_tq_batch_beside_a_capture(gpu):
+    """Batches long enough for two launches side by side, on one stream under
+    capture and on another that is not, from one thread and before the capture
+    ends: the eager ones run at once, the captured one on replay, all with the
+    results of a batch by itself."""
+    import torch
+    import xavs2_gb300 as xg
+    import xavs2_gb300.synth as synth
+    n = 6000
+    blocks, nres, ncoef, _ = synth.tq_blocks(n, seed=11, parts=tuple(TU_PARTS))
+    res = synth.tq_residual(blocks, np.zeros(n, bool), nres, seed=5)
+    d_blocks, d_res = torch.from_numpy(blocks.view(np.uint8).copy()).cuda(), res.cuda()
+    want = _run_tq_batch(blocks, res.numpy(), nres, ncoef)
+
+    def outputs():
+        return [torch.full((k,), 0x5A5A, dtype=t, device="cuda")
+                for k, t in ((ncoef, torch.int16), (nres, torch.int16), (n, torch.int32))]
+
+    def enqueue(out, stream):
+        return xg.fn("xavs2gpu_tq_batch")(d_blocks.data_ptr(), n, d_res.data_ptr(), out[0].data_ptr(),
+                                          out[1].data_ptr(), out[2].data_ptr(), ctypes.c_void_p(stream.cuda_stream))
+
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    eager, captured = [outputs(), outputs()], outputs()
+    torch.cuda.synchronize()
+    lib = xg.load()
+    lib.xavs2gpu_set_abort_on_error(0)
+    try:
+        assert enqueue(outputs(), a) == 0            # side stream and kernels exist before the capture
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=a, capture_error_mode="relaxed"):
+            assert enqueue(captured, a) == 0
+            assert enqueue(eager[0], b) == 0
+            assert enqueue(captured, a) == 0
+            assert enqueue(eager[1], b) == 0
+        assert lib.xavs2gpu_get_status() == 0, lib.xavs2gpu_get_error()
+        g.replay()
+        torch.cuda.synchronize()
+    finally:
+        lib.xavs2gpu_clear_error()
+        lib.xavs2gpu_set_abort_on_error(1)
+    for out in eager + [captured]:
+        for got, exp in zip(out, want):
+            assert np.array_equal(got.cpu().numpy(), exp)

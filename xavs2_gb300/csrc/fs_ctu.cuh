@@ -848,8 +848,10 @@ struct CtuSide {
         if (st) cudaStreamDestroy(st);
     }
 };
-// k: 0 the search's own, 1 the per-PU search's, 2 the per-PU search's second
-static CtuSide *ctu_side(int dev, int k = 0)
+// Side stream k (0 the search's own, 1 the per-PU search's, 2 the per-PU
+// search's second) for launches beside `st`, or null: the launches then stay
+// on st.
+static CtuSide *ctu_side(int dev, cudaStream_t st, int k = 0)
 {
     thread_local CtuSide side[3][64];
     if (dev < 0 || dev >= 64 || k < 0 || k > 2) return nullptr;
@@ -859,10 +861,10 @@ static CtuSide *ctu_side(int dev, int k = 0)
             cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess) {
             cudaGetLastError();
-            return nullptr;   // the launches then stay on the caller's stream
+            return nullptr;
         }
     }
-    return &s;
+    return side_usable(st, s.st) ? &s : nullptr;
 }
 
 // Creates what a search at range R launches with on this thread -- the side
@@ -871,9 +873,7 @@ static void ctu_prime(int R)
 {
     const int dev = current_device();
     if (XG_CTU_FORK) {
-        ctu_side(dev, 0);
-        ctu_side(dev, 1);
-        ctu_side(dev, 2);
+        for (int k = 0; k < 3; k++) ctu_side(dev, nullptr, k);
     }
     if (R < 1 || R > 128) return;
     for (int dyw = 2; dyw <= kDyWarpMax; dyw *= 2) ctu_fit(dev, R, dyw);
@@ -895,7 +895,7 @@ static void ctu_jobs_run(const CtuJob *d_jobs, int n_jobs, int n_border, const S
     const int grid = n_jobs * nchunks;
     const int lam = prm.lambda_factor;
     // the border launch on the side stream when both variants run
-    CtuSide *side = XG_CTU_FORK && n_border > 0 && n_border < n_jobs ? ctu_side(dev) : nullptr;
+    CtuSide *side = XG_CTU_FORK && n_border > 0 && n_border < n_jobs ? ctu_side(dev, st) : nullptr;
     cudaStream_t bst = st;
     if (side) {
         XG_CUDA(cudaEventRecord(side->fork, st));

@@ -1345,7 +1345,7 @@ namespace xg {
 // itself without a side stream), join makes st wait for it.
 static cudaStream_t fork_side(cudaStream_t st, bool both, int k, CtuSide *&side)
 {
-    side = XG_CTU_FORK && both ? ctu_side(current_device(), k) : nullptr;
+    side = XG_CTU_FORK && both ? ctu_side(current_device(), st, k) : nullptr;
     if (!side) return st;
     XG_CUDA(cudaEventRecord(side->fork, st));
     XG_CUDA(cudaStreamWaitEvent(side->st, side->fork, 0));

@@ -1066,7 +1066,8 @@ constexpr int kDirectMinB = 5;   // CTAs of 4 warps per SM: 96 registers (8 meas
 
 // The two launches of the ordered form beside each other up to this many TUs:
 // the second on a side stream forked from the caller's and joined back (per
-// host thread and device; none is made during a stream capture).  Their tails
+// host thread and device; none is made during a stream capture, and one that is
+// part of another capture is left alone).  Their tails
 // then overlap (us, forked / in turn: 6000 TUs of all shapes 33.8 / 43.7, 16000
 // 58 / 66, 64000 201 / 207); larger batches fill the GPU with either launch and
 // lose by sharing it (200,000 644 / 602, 10^6 squares 2.61 / 2.55 ms).
@@ -1100,7 +1101,7 @@ static TqSide *tq_side(int dev, cudaStream_t stream)
             return nullptr;
         }
     }
-    return &s;
+    return side_usable(stream, s.st) ? &s : nullptr;
 }
 
 template <int WARPS>

@@ -57,6 +57,22 @@ int sm_count();
 int reference_planes_from(const uint8_t *src, int src_stride, int width, int height, int pad, uint8_t *const planes[16],
                           int stride, cudaStream_t st);
 
+// Whether work forked from `stream` may go to `side` now.  A stream that was
+// joined to a capture belongs to it until that capture ends; from any other
+// stream it must not be forked to meanwhile (the launches then stay on `stream`).
+static inline bool side_usable(cudaStream_t stream, cudaStream_t side)
+{
+    cudaStreamCaptureStatus a = cudaStreamCaptureStatusNone, b = cudaStreamCaptureStatusNone;
+    unsigned long long ia = 0, ib = 0;
+    if (cudaStreamGetCaptureInfo(side, &a, &ia) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a == cudaStreamCaptureStatusNone) return true;
+    if (cudaStreamGetCaptureInfo(stream, &b, &ib) != cudaSuccess) cudaGetLastError();
+    return a == cudaStreamCaptureStatusActive && b == a && ia == ib;
+}
+
 // Byte offset rounded up to 256 for staging sub-buffers.
 static inline size_t align_up(size_t v, size_t a = 256) { return (v + a - 1) / a * a; }
 
