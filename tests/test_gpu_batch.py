@@ -73,3 +73,45 @@ def test_rotate_refs(gpu):
     assert got.tobytes() == t.results().tobytes()
     s.close()
     t.close()
+
+
+def test_run_captured_after_batch(gpu):
+    """A session of PUs with their own predictors whose plan a batch has made,
+    then captured searching by itself: nothing is allocated inside the
+    capture, and the replay's results are the batch's, as are an eager run's
+    after it and those of a second capture."""
+    import torch
+    import xavs2_gb300 as xg
+    s, _ = _session(xg, 192, 136, 51)
+    rng = np.random.default_rng(52)
+    pus = s._pus.copy()
+    pus["mvp_x"], pus["mvp_y"] = rng.integers(9, 25, len(pus)), rng.integers(-24, -8, len(pus))
+    s.set_pus(pus)
+    prm = xg.MeParams(8, oracle.lambda_factor(32), 1, 2, 0, 0)
+    stream = torch.cuda.Stream()
+    s.sync()
+    s.set_stream(stream.cuda_stream)
+    batch = xg.MeBatch()
+    lib = xg.load()
+    lib.xavs2gpu_set_abort_on_error(0)
+    try:
+        batch.run([s], prm, stream.cuda_stream)
+        want = s.results()
+        assert (want["bcost"] < 1 << 30).all()
+        for _ in range(2):                        # the second capture follows an eager run
+            g = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(g, stream=stream, capture_error_mode="thread_local"):
+                s.run(prm)
+            assert lib.xavs2gpu_get_status() == 0, lib.xavs2gpu_get_error()
+            with torch.cuda.stream(stream):
+                g.replay()
+            assert s.results().tobytes() == want.tobytes()
+            s.run(prm)
+            assert s.results().tobytes() == want.tobytes()
+    finally:
+        lib.xavs2gpu_clear_error()
+        lib.xavs2gpu_set_abort_on_error(1)
+    s.set_stream(None)
+    batch.close()
+    s.close()

@@ -1460,6 +1460,7 @@ struct MeSessionImpl {
     uint8_t *d_cu = nullptr;
     size_t cap_cu = 0;
     bool cu_stale = true;            // the per-PU list changed since they were made
+    bool per_pu_stale = true;        // neither was tried for the plan
     PerPuList cu_list;
     std::vector<uint32_t> h_generic, h_small, h_large;
     // CU-grouped refinement: the groups, their members, and the thread /
@@ -1913,6 +1914,7 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     XG_CUDA(cudaStreamSynchronize(m.st));
     m.plan_R = R;
     m.plan_ctu = ctu;
+    m.per_pu_stale = true;
 }
 
 // Per-PU searches from which a run computes the references' block means (a
@@ -2033,10 +2035,18 @@ static void ensure_cu_search(MeSessionImpl &m)
 
 // The session's means buffer, on the first plan that has use for it (without
 // the memory for it the per-PU search runs unbounded, with the same results),
-// and the CU search of the plan's per-PU list.
+// and the CU search of the plan's per-PU list.  Tried once per plan, and never
+// inside a capture, where allocating is an error: a run captured before any
+// other of its plan takes the unbounded search.
 static void ensure_per_pu(MeSessionImpl &m)
 {
-    if (m.n_generic < kMeansMinPus) return;
+    if (!m.per_pu_stale || m.n_generic < kMeansMinPus) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(m.st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return;
+    }
+    m.per_pu_stale = false;
     if (!m.d_means) {
         if (cudaMalloc((void **)&m.d_means, m.plane_bytes * m.nrefs + 256) != cudaSuccess) {
             cudaGetLastError();
@@ -2065,7 +2075,7 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     XG_CUDA(cudaMemsetAsync(m.d_keys, 0xff, sizeof(unsigned long long) * m.n, m.st));
     const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
     PerPuList per_pu{gen, 0, 0, m.n_generic};
-    const bool bounded = m.n_generic >= kMeansMinPus && m.d_means && prune_ok(lam);
+    const bool bounded = m.n_generic >= kMeansMinPus && !m.per_pu_stale && m.d_means && prune_ok(lam);
     if (bounded) per_pu = m.cu_list;
     if (m.n_generic) {
         me_init_list_kernel<<<(m.n_generic * 32 + 127) / 128, 128, 0, m.st>>>(gen, m.n_generic, m.d_view, lam);
