@@ -781,7 +781,11 @@ XAVS2GPU_API int xavs2gpu_chain_graph_kernels(const xavs2gpu_chain_t *c);
  * references and their planes resident; a stream is admitted when its
  * resident memory fits both hbm_budget_bytes (if set) and the device's free
  * memory at that moment (cudaMemGetInfo) less hbm_reserve_bytes and less
- * what streams admitted but not yet allocated will take.  The first two
+ * what streams admitted but not yet allocated will take.  Streams whose PUs
+ * are searched one by one (odd ranges, own predictors) also get a buffer of
+ * block means, one plane per reference, where both leave room for it when
+ * they open; the buffers are given back before they would keep a later
+ * stream out (the search is then slower, with the same results).  The first two
  * pictures of a stream only fill its
  * references (ref_only results); every later picture is searched against
  * the two before it. */
@@ -823,6 +827,7 @@ XAVS2GPU_API int xavs2gpu_server_submit(xavs2gpu_server_t *s, int stream, const 
                                         int64_t tag);
 /* Completed pictures (waits up to timeout_ms for the first). */
 XAVS2GPU_API int xavs2gpu_server_poll(xavs2gpu_server_t *s, xavs2gpu_server_result_t *out, int max, int timeout_ms);
+/* hbm_used: batch buffers, admitted streams and their block means. */
 XAVS2GPU_API void xavs2gpu_server_stats(xavs2gpu_server_t *s, int64_t *hbm_used, int64_t *batches, int64_t *frames,
                                         int64_t *pending);
 /* Sum over completed batches of their device time (first to last command)

@@ -138,3 +138,65 @@ def test_server_admission_free_memory(gpu):
     srv = xg.Server(xg.ServerConfig(0, 1 << 18, 4, QP, prm))
     assert srv.open_stream(w, h, pus, cus) >= 0
     srv.close()
+
+
+def test_server_block_means_memory(gpu):
+    """Block means of the per-PU search (an odd range: every PU): counted, kept
+    inside the budget, given back before they would keep a later stream out,
+    and without influence on the results."""
+    import torch
+    import xavs2_gb300 as xg
+    w, h = 3840, 2160
+    rng = np.random.default_rng(77)
+    base = np.kron(rng.integers(16, 236, (h // 16, w // 16)), np.ones((16, 16), np.int64)).astype(np.uint8)
+    frames = [np.roll(base, (k, -2 * k), (0, 1)) ^ rng.integers(0, 4, (h, w), dtype=np.uint8) for k in range(3)]
+    pus, cus = xg.cu_pus(xg.split_map_cus(w, h, 5, p_split=(0.5, 0.3, 0.2)), w, h, 2)
+    means = 2 * ((w + 160 + 63) // 64 * 64) * (h + 160)
+
+    def used():
+        free_b, total_b = torch.cuda.mem_get_info()
+        return total_b - free_b
+
+    def server(rng_, budget=0):
+        prm = xg.MeParams(rng_, oracle.lambda_factor(QP), 1, 2, 0, 0)
+        return xg.Server(xg.ServerConfig(budget, w * h, 4, QP, prm))
+
+    def serve(srv, sid):
+        for f in frames:
+            assert srv.submit(sid, f) == 0
+        got = []
+        t0 = time.time()
+        while len(got) < len(frames) and time.time() - t0 < 60:
+            got.extend(srv.poll(16, 200).tolist())
+        return [int(r["hash"]) for r in np.array(got, dtype=xg.SERVER_RESULT_DTYPE)]
+
+    grown = {}
+    for name, rng_, spare in (("even", 8, None), ("plain", 7, 0), ("free", 7, None), ("two", 7, -1)):
+        srv = server(rng_)
+        empty = srv.stats()["hbm_used"]
+        srv.close()
+        need = grown.get("need", 0)
+        budget = 0 if spare is None else empty + need if spare == 0 else empty + 2 * need
+        srv = server(rng_, budget)
+        m0 = used()
+        sid = srv.open_stream(w, h, pus, cus, ring=4)
+        assert sid >= 0
+        held = srv.stats()["hbm_used"] - empty
+        m1 = used()
+        hashes = serve(srv, sid)
+        m2 = used()
+        grown[name] = (held, m1 - m0, m2 - m1, hashes)
+        if name == "even":
+            grown["need"] = held
+        if name == "two":
+            assert srv.open_stream(w, h, pus, cus, ring=4) >= 0
+            assert srv.stats()["hbm_used"] == budget
+            assert serve(srv, sid)[2] == hashes[2]
+        srv.close()
+    need = grown["need"]
+    assert grown["plain"][0] == need and means <= grown["free"][0] - need <= means + 4096
+    assert grown["two"][0] == grown["free"][0]
+    # the device's memory: nothing of the means' size beyond what is counted
+    for at in (1, 2):
+        assert grown["plain"][at] - grown["even"][at] < means // 2, grown
+    assert grown["plain"][3] == grown["free"][3] == grown["two"][3]

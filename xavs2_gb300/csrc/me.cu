@@ -1454,13 +1454,17 @@ struct MeSessionImpl {
     cudaStream_t own_st = nullptr;   // the stream the session created
     SessView h_view{};
     SessView *d_view = nullptr;      // this session as the kernels see it
-    uint8_t *d_means = nullptr;      // 4x4 block means of the references (per-PU search), made with the plan
+    // 4x4 block means of the references (per-PU search): tried once per plan
+    // by the searches that use them, or (means_owned) given and taken by the
+    // session's owner alone
+    uint8_t *d_means = nullptr;
+    bool means_tried = false, means_owned = false;
     // CUs whose partitions have their own centres, the queues of their
     // search, and the per-PU list of the rest (all in d_cu)
     uint8_t *d_cu = nullptr;
     size_t cap_cu = 0;
     bool cu_stale = true;            // the per-PU list changed since they were made
-    bool per_pu_stale = true;        // neither was tried for the plan
+    bool per_pu_stale = true;        // they were not looked at since the plan was made
     PerPuList cu_list;
     std::vector<uint32_t> h_generic, h_small, h_large;
     // CU-grouped refinement: the groups, their members, and the thread /
@@ -1914,6 +1918,7 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     XG_CUDA(cudaStreamSynchronize(m.st));
     m.plan_R = R;
     m.plan_ctu = ctu;
+    m.means_tried = false;
     m.per_pu_stale = true;
 }
 
@@ -1957,7 +1962,6 @@ static void ensure_cu_search(MeSessionImpl &m)
     m.cu_list.list = gen;
     m.cu_list.n_large = m.n_generic_large;
     m.cu_list.n_small = m.n_generic - m.n_generic_large;
-    if (!m.d_means || m.n_generic < kMeansMinPus) return;
     std::vector<CuRec> recs;
     std::vector<uint32_t> rest;
     std::vector<int> at[4];          // record of each CU position, per size
@@ -2033,30 +2037,87 @@ static void ensure_cu_search(MeSessionImpl &m)
     l.q.small = reinterpret_cast<uint32_t *>(m.d_cu + o_small);
 }
 
-// The session's means buffer, on the first plan that has use for it (without
-// the memory for it the per-PU search runs unbounded, with the same results),
-// and the CU search of the plan's per-PU list.  Tried once per plan, and never
-// inside a capture, where allocating is an error: a run captured before any
-// other of its plan takes the unbounded search.
-static void ensure_per_pu(MeSessionImpl &m)
+static size_t means_bytes(const MeSessionImpl &m) { return m.plane_bytes * m.nrefs + 256; }
+
+// Whether a search of the session's plan with factor lambda uses block means.
+static bool means_wanted(const MeSessionImpl &m, int lambda)
 {
-    if (!m.per_pu_stale || m.n_generic < kMeansMinPus) return;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(m.st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return;
-    }
-    m.per_pu_stale = false;
-    if (!m.d_means) {
-        if (cudaMalloc((void **)&m.d_means, m.plane_bytes * m.nrefs + 256) != cudaSuccess) {
-            cudaGetLastError();
-            m.d_means = nullptr;
-            return;
-        }
-        refresh_view(m);
-    }
-    ensure_cu_search(m);
+    return m.n_generic >= kMeansMinPus && prune_ok(lambda);
 }
+
+static bool capturing(const MeSessionImpl &m)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool none = cudaStreamIsCapturing(m.st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    if (!none) cudaGetLastError();
+    return !none;
+}
+
+static bool means_alloc(MeSessionImpl &m)
+{
+    if (cudaMalloc((void **)&m.d_means, means_bytes(m)) != cudaSuccess) {
+        cudaGetLastError();
+        m.d_means = nullptr;
+        return false;
+    }
+    refresh_view(m);
+    return true;
+}
+
+// The session's means buffer, where the plan has use for it and the memory is
+// there (without it the per-PU search runs unbounded, with the same results).
+// Never allocated inside a capture, where that is an error.
+static bool ensure_means(MeSessionImpl &m, int lambda)
+{
+    if (!means_wanted(m, lambda)) return false;
+    if (!m.d_means && !m.means_owned && !m.means_tried && !capturing(m)) {
+        m.means_tried = true;
+        means_alloc(m);
+    }
+    return m.d_means != nullptr;
+}
+
+// That, and the CU search of the plan's per-PU list: whether a run takes
+// cu_list.  A run captured before any other of its plan takes the unbounded
+// search.
+static bool ensure_per_pu(MeSessionImpl &m, int lambda)
+{
+    if (!ensure_means(m, lambda)) return false;
+    if (m.per_pu_stale) {
+        if (capturing(m)) return false;
+        m.per_pu_stale = false;
+        ensure_cu_search(m);
+    }
+    return true;
+}
+
+namespace xg {
+
+// For sessions searched in batches alone, whose owner decides about the
+// memory for block means: the plan without any, the bytes a search would use,
+// and the memory itself.  A search must not be in flight when it is taken.
+void me_prepare_batched(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm)
+{
+    MeSessionImpl &m = s->impl;
+    XG_CUDA(cudaSetDevice(m.device));
+    m.means_owned = true;
+    ensure_plan(m, prm->search_range, prm->lambda_factor);
+    ctu_prime(prm->search_range);
+}
+int64_t me_means_bytes(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm)
+{
+    return means_wanted(s->impl, prm->lambda_factor) ? (int64_t)means_bytes(s->impl) : 0;
+}
+bool me_give_means(xavs2gpu_me_session_t *s) { return s->impl.d_means || means_alloc(s->impl); }
+void me_take_means(xavs2gpu_me_session_t *s)
+{
+    MeSessionImpl &m = s->impl;
+    cudaFree(m.d_means);
+    m.d_means = nullptr;
+    refresh_view(m);
+}
+
+}  // namespace xg
 
 extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm)
 {
@@ -2070,12 +2131,11 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     XG_CUDA(cudaSetDevice(m.device));
     const int R = prm->search_range, lam = prm->lambda_factor;
     ensure_plan(m, R, lam);
-    ensure_per_pu(m);
+    const bool bounded = ensure_per_pu(m, lam);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[0], m.st));
     XG_CUDA(cudaMemsetAsync(m.d_keys, 0xff, sizeof(unsigned long long) * m.n, m.st));
     const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
     PerPuList per_pu{gen, 0, 0, m.n_generic};
-    const bool bounded = m.n_generic >= kMeansMinPus && !m.per_pu_stale && m.d_means && prune_ok(lam);
     if (bounded) per_pu = m.cu_list;
     if (m.n_generic) {
         me_init_list_kernel<<<(m.n_generic * 32 + 127) / 128, 128, 0, m.st>>>(gen, m.n_generic, m.d_view, lam);
@@ -2225,7 +2285,7 @@ extern "C" int xavs2gpu_me_prepare(xavs2gpu_me_session_t *s, const xavs2gpu_me_p
     }
     XG_CUDA(cudaSetDevice(s->impl.device));
     ensure_plan(s->impl, prm->search_range, prm->lambda_factor);
-    ensure_per_pu(s->impl);
+    ensure_per_pu(s->impl, prm->lambda_factor);
     ctu_prime(prm->search_range);   // nothing created inside a capture that follows
     return XAVS2GPU_OK;
 }
@@ -2355,8 +2415,7 @@ struct BatchBuf {
     uint32_t *d_lists = nullptr;    // generic | small | large | group members
     SessView *d_views = nullptr;
     RefineGroup *d_groups = nullptr;
-    uint8_t *d_means = nullptr;     // block means of the sessions with per-PU searches
-    size_t cap_jobs = 0, cap_lists = 0, cap_views = 0, cap_groups = 0, cap_means = 0;
+    size_t cap_jobs = 0, cap_lists = 0, cap_views = 0, cap_groups = 0;
     uint8_t *h_stage = nullptr;     // pinned: jobs | lists | views (uploads without a stream wait)
     size_t cap_stage = 0;
     cudaEvent_t done = nullptr;
@@ -2391,8 +2450,7 @@ extern "C" void xavs2gpu_me_batch_destroy(xavs2gpu_me_batch_t *b)
     for (auto &x : b->buf) {
         if (x.used) cudaEventSynchronize(x.done);
         cudaEventDestroy(x.done);
-        cudaFree(x.d_jobs); cudaFree(x.d_lists); cudaFree(x.d_views); cudaFree(x.d_groups);
-        cudaFree(x.d_means); cudaFreeHost(x.h_stage);
+        cudaFree(x.d_jobs); cudaFree(x.d_lists); cudaFree(x.d_views); cudaFree(x.d_groups); cudaFreeHost(x.h_stage);
     }
     delete b;
 }
@@ -2407,24 +2465,6 @@ static void grow(T *&p, size_t &cap, size_t need, cudaStream_t st)
     if (p) XG_CUDA(cudaFreeAsync(p, st));
     cap = need + need / 2 + 64;
     XG_CUDA(cudaMallocAsync((void **)&p, sizeof(T) * cap, st));
-}
-
-// The same for a buffer the launch can do without: false (and no buffer)
-// when the memory is not there.
-template <typename T>
-static bool grow_if_room(T *&p, size_t &cap, size_t need, cudaStream_t st)
-{
-    if (need <= cap) return need != 0;
-    if (p) XG_CUDA(cudaFreeAsync(p, st));
-    p = nullptr;
-    cap = 0;
-    if (cudaMallocAsync((void **)&p, sizeof(T) * need, st) != cudaSuccess) {
-        cudaGetLastError();
-        p = nullptr;
-        return false;
-    }
-    cap = need;
-    return true;
 }
 
 extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session_t *const *sessions, int n,
@@ -2442,8 +2482,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     // pass 1: plans and sizes
     const bool grouped = !prm->enable_pmvr && use_groups();
     size_t nj = 0, ng = 0, ns = 0, nl = 0, nm = 0, nheavy = 0, ngr = 0;
-    size_t nmeans = 0, ngl = 0, ngs = 0;   // means bytes, per-PU searches of bounded sessions
-    auto bounded = [&](const MeSessionImpl &m) { return prune_ok(lam) && m.n_generic >= kMeansMinPus; };
+    size_t ngl = 0, ngs = 0;   // per-PU searches of sessions with block means
     int nborder = 0, max_refs = 0;
     int block = 128;
     for (int k = 0; k < n; k++) {
@@ -2457,8 +2496,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         nj += m.plan.h_jobs.size();
         nborder += m.plan.n_border;
         ng += m.h_generic.size();
-        if (bounded(m)) {
-            nmeans += m.plane_bytes * m.nrefs + 256;
+        if (ensure_means(m, lam)) {
             max_refs = std::max(max_refs, m.nrefs);
             ngl += m.n_generic_large;
             ngs += m.n_generic - m.n_generic_large;
@@ -2480,8 +2518,6 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     grow(bb.d_lists, bb.cap_lists, nlist, st);
     grow(bb.d_views, bb.cap_views, (size_t)n, st);
     grow(bb.d_groups, bb.cap_groups, ngr, st);
-    if (!grow_if_room(bb.d_means, bb.cap_means, nmeans, st)) nmeans = ngl = ngs = 0;
-    size_t means_at = 0;
     const size_t bj = sizeof(CtuJob) * nj, bl = sizeof(uint32_t) * nlist;
     const size_t bv = sizeof(SessView) * n, bg = sizeof(RefineGroup) * ngr;
     const size_t oj = 0, ol = align_up(bj), ov = ol + align_up(bl), og = ov + align_up(bv), need = og + align_up(bg);
@@ -2511,14 +2547,12 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         const bool g = grouped && m.cu_groups;
         const uint32_t tag = (uint32_t)k << kSessShift;
         V[k] = m.h_view;
-        V[k].means = nullptr;
         const uint32_t *gen = m.h_generic.data();
-        if (nmeans && bounded(m)) {
-            V[k].means = bb.d_means + means_at;
-            means_at += m.plane_bytes * m.nrefs + 256;
+        if (m.d_means && means_wanted(m, lam)) {
             put_n(Lgl, gen, m.n_generic_large, tag);
             put_n(Lgs, gen + m.n_generic_large, m.n_generic - m.n_generic_large, tag);
         } else {
+            V[k].means = nullptr;
             put_n(Lgp, gen, m.n_generic, tag);
         }
         for (const CtuJob &j0 : m.plan.h_jobs) {
@@ -2549,7 +2583,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
     if (ng) {
         me_init_list_kernel<<<(unsigned)((ng * 32 + 127) / 128), 128, 0, st>>>(d_gen, (int)ng, bb.d_views, lam);
         count_launch();
-        if (nmeans) mean_planes_run(bb.d_views, n, max_refs, st);
+        if (max_refs) mean_planes_run(bb.d_views, n, max_refs, st);
     }
     const PerPuList per_pu{d_gen, (int)ngl, (int)ngs, (int)(ng - ngl - ngs)};
     CtuSide *gside = nullptr;

@@ -45,6 +45,10 @@ namespace xg {
 
 int tq_batch_launch(const xavs2gpu_tq_block_t *blocks, int n, const int16_t *residual, int16_t *coef,
                     int16_t *recon, int32_t *nnz, int warps, cudaStream_t stream);
+void me_prepare_batched(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm);
+int64_t me_means_bytes(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm);
+bool me_give_means(xavs2gpu_me_session_t *s);
+void me_take_means(xavs2gpu_me_session_t *s);
 bool build_candidates(const xavs2gpu_cu_t *cus, int n_cus, const xavs2gpu_pu_t *pus, int n_pus, int W, int H,
                       int nrefs, std::vector<xavs2gpu_cand_t> &cands, std::vector<int32_t> &cu_cand, int64_t &n_res,
                       int64_t &n_coef);
@@ -109,7 +113,9 @@ struct Stream {
     int frames = 0;                               // pictures submitted
     int loaded = 0;                               // pictures that reached the device
     bool in_flight = false;
+    bool hold = false;                            // batched again only when its block means are back
     int64_t bytes = 0;
+    int64_t means = 0;                            // bytes of its search's block means (counted in hbm_used)
 };
 
 struct Job {
@@ -145,6 +151,7 @@ struct xavs2gpu_server {
     int device = 0;
     int64_t hbm_used = 0;
     int64_t hbm_pending = 0;                  // admitted streams whose memory is not allocated yet
+    bool means_off = false;                   // block means were given back for a stream's sake
     int64_t max_cus = 0, max_cands = 0;
     std::vector<Stream *> streams;
     BatchSet sets[XG_SERVE_SETS];
@@ -274,7 +281,7 @@ void scheduler(xavs2gpu_server_t *s)
                 int64_t backlog = 0;
                 for (const Job &j : s->pending) {
                     Stream &S = *s->streams[j.stream];
-                    if (S.in_flight || used[j.stream]) continue;
+                    if (S.in_flight || S.hold || used[j.stream]) continue;
                     used[j.stream] = 1;
                     backlog += (int64_t)S.W * S.H;
                 }
@@ -286,7 +293,7 @@ void scheduler(xavs2gpu_server_t *s)
                 const int64_t p = (int64_t)S.W * S.H;
                 // a batch's first picture may take the full size (a picture
                 // larger than the target never waits for a backlog)
-                if (S.in_flight || used[it->stream] || pix + p > (take.empty() ? s->cfg.max_batch_pixels : cap)) {
+                if (S.in_flight || S.hold || used[it->stream] || pix + p > (take.empty() ? s->cfg.max_batch_pixels : cap)) {
                     ++it;
                     continue;
                 }
@@ -369,6 +376,42 @@ void free_set(BatchSet &b)
     if (b.done) cudaEventDestroy(b.done);
     if (b.start) cudaEventDestroy(b.start);
     if (b.st) cudaStreamDestroy(b.st);
+}
+
+}  // namespace
+
+namespace {
+
+// Why `bytes` more do not fit (s->mu held): 1 the budget, 2 the device's free
+// memory now, less the reserve and what streams admitted before still have to
+// allocate; 0 when they fit.
+int refusal(xavs2gpu_server_t *s, int64_t bytes)
+{
+    if (s->cfg.hbm_budget_bytes > 0 && s->hbm_used + bytes > s->cfg.hbm_budget_bytes) return 1;
+    size_t free_b = 0, total_b = 0;
+    XG_CUDA(cudaSetDevice(s->device));
+    XG_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    const int64_t reserve = s->cfg.hbm_reserve_bytes > 0 ? s->cfg.hbm_reserve_bytes
+                                                        : std::max<int64_t>((int64_t)total_b / 32, (int64_t)1 << 30);
+    return bytes + s->hbm_pending > (int64_t)free_b - reserve ? 2 : 0;
+}
+
+// Takes every stream's block means back, each once its picture in flight has
+// completed (lk holds s->mu; released while waiting), and gives out no more.
+void reclaim_means(xavs2gpu_server_t *s, std::unique_lock<std::mutex> &lk)
+{
+    s->means_off = true;
+    for (size_t k = 0; k < s->streams.size(); k++) {
+        Stream &S = *s->streams[k];
+        if (!S.means) continue;
+        S.hold = true;
+        s->cv.wait(lk, [&] { return s->stop || !S.in_flight; });
+        S.hold = false;
+        if (s->stop || !S.means) continue;
+        me_take_means(S.sess);
+        s->hbm_used -= S.means;
+        S.means = 0;
+    }
 }
 
 }  // namespace
@@ -475,22 +518,20 @@ extern "C" int xavs2gpu_server_open_stream(xavs2gpu_server_t *s, int width, int 
                          (int64_t)cands.size() * 24 + 2 * (int64_t)width * height + (int64_t)n_cus * 849 * 4 / 16 +
                          (int64_t)cands.size() * 16 + (int64_t)n_cus * 16;
     std::unique_lock<std::mutex> lk(s->mu);
-    if (s->cfg.hbm_budget_bytes > 0 && s->hbm_used + need > s->cfg.hbm_budget_bytes) {
-        fail(XAVS2GPU_ERR_CAPACITY, "xavs2gpu_server_open_stream", "device-memory budget exhausted");
-        return -XAVS2GPU_ERR_CAPACITY;
-    }
-    // admission by the device's free memory now, less the reserve and what
-    // streams admitted before us still have to allocate
-    {
-        size_t free_b = 0, total_b = 0;
-        XG_CUDA(cudaSetDevice(s->device));
-        XG_CUDA(cudaMemGetInfo(&free_b, &total_b));
-        const int64_t reserve = s->cfg.hbm_reserve_bytes > 0 ? s->cfg.hbm_reserve_bytes
-                                                            : std::max<int64_t>((int64_t)total_b / 32, (int64_t)1 << 30);
-        if (need + s->hbm_pending > (int64_t)free_b - reserve) {
-            fail(XAVS2GPU_ERR_CAPACITY, "xavs2gpu_server_open_stream", "not enough free device memory");
-            return -XAVS2GPU_ERR_CAPACITY;
+    int why = refusal(s, need);
+    if (why) {
+        // block means only speed a search up: they never keep a stream out
+        int64_t held = 0;
+        for (const Stream *S : s->streams) held += S->means;
+        if (held && !refusal(s, need - held)) {
+            reclaim_means(s, lk);
+            why = refusal(s, need);
         }
+    }
+    if (why) {
+        fail(XAVS2GPU_ERR_CAPACITY, "xavs2gpu_server_open_stream",
+             why == 1 ? "device-memory budget exhausted" : "not enough free device memory");
+        return -XAVS2GPU_ERR_CAPACITY;
     }
     s->hbm_used += need;
     s->hbm_pending += need;
@@ -501,8 +542,7 @@ extern "C" int xavs2gpu_server_open_stream(xavs2gpu_server_t *s, int width, int 
     S->n_cus = n_cus;
     S->n_pus = n_pus;
     S->sess = xavs2gpu_me_create(width, height, 2, n_pus);
-    if (!S->sess || xavs2gpu_me_set_pus(S->sess, pus, n_pus) != XAVS2GPU_OK ||
-        xavs2gpu_me_prepare(S->sess, &s->cfg.me) != XAVS2GPU_OK) {
+    if (!S->sess || xavs2gpu_me_set_pus(S->sess, pus, n_pus) != XAVS2GPU_OK) {
         if (S->sess) xavs2gpu_me_destroy(S->sess);
         delete S;
         lk.lock();
@@ -510,6 +550,7 @@ extern "C" int xavs2gpu_server_open_stream(xavs2gpu_server_t *s, int width, int 
         s->hbm_pending -= need;
         return -XAVS2GPU_ERR_ARG;
     }
+    me_prepare_batched(S->sess, &s->cfg.me);
     S->n_res = n_res;
     S->n_coef = n_coef;
     S->n_cands = (int)cands.size();
@@ -530,6 +571,12 @@ extern "C" int xavs2gpu_server_open_stream(xavs2gpu_server_t *s, int width, int 
     XG_CUDA(cudaMallocHost((void **)&S->h_ring, (size_t)width * height * ring));
     lk.lock();
     s->hbm_pending -= need;
+    // its block means, while there is room for them
+    const int64_t means = me_means_bytes(S->sess, &s->cfg.me);
+    if (means && !s->means_off && !refusal(s, means) && me_give_means(S->sess)) {
+        S->means = means;
+        s->hbm_used += means;
+    }
     S->id = (int)s->streams.size();
     s->streams.push_back(S);
     return S->id;
