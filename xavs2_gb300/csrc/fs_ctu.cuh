@@ -44,10 +44,10 @@
 #pragma once
 
 #include "ctu_layout.h"
+#include "pu_lists.h"
 
 namespace xg {
 
-constexpr int kSlots = 849;
 constexpr int kCtuThreads = 32 * kCtuWarps;
 constexpr uint32_t kPoisonSmall = 126976u;     // > any valid cost of a PU up to 16x16
 constexpr uint32_t kPoisonLarge = 1u << 22;    // replaces a 4x4 SAD outside the limits
@@ -70,78 +70,6 @@ struct CtuPlan {
     CtuJob *d_jobs = nullptr;
     int32_t *d_slots = nullptr;   // [n_jobs][kSlots]: PU index or -1
     std::vector<CtuJob> h_jobs;   // host copy (sess = 0), for multi-session launches
-};
-
-// ---- slot geometry (host) --------------------------------------------------------
-struct SlotGeom { int ox, oy, part; };
-
-static inline int part_of(int w, int h)
-{
-    for (int i = 0; i < kNumParts; i++)
-        if (h_pu_w[i] == w && h_pu_h[i] == h) return i;
-    return -1;
-}
-
-// mode m of an N x N CU at (cx, cy): 0 2Nx2N, 1-2 2NxN, 3-4 Nx2N, 5-6 2NxnU,
-// 7-8 2NxnD, 9-10 nLx2N, 11-12 nRx2N
-static inline SlotGeom cu_mode_geom(int N, int cx, int cy, int m)
-{
-    const int h2 = N / 2, q = N / 4, q3 = 3 * N / 4;
-    switch (m) {
-    case 0: return {cx, cy, part_of(N, N)};
-    case 1: return {cx, cy, part_of(N, h2)};
-    case 2: return {cx, cy + h2, part_of(N, h2)};
-    case 3: return {cx, cy, part_of(h2, N)};
-    case 4: return {cx + h2, cy, part_of(h2, N)};
-    case 5: return {cx, cy, part_of(N, q)};
-    case 6: return {cx, cy + q, part_of(N, q3)};
-    case 7: return {cx, cy, part_of(N, q3)};
-    case 8: return {cx, cy + q3, part_of(N, q)};
-    case 9: return {cx, cy, part_of(q, N)};
-    case 10: return {cx + q, cy, part_of(q3, N)};
-    case 11: return {cx, cy, part_of(q3, N)};
-    default: return {cx + q3, cy, part_of(q, N)};
-    }
-}
-
-static SlotGeom slot_geom(int s)
-{
-    if (s < 576) {
-        int cu = s / 9, m = s % 9, cx = (cu % 8) * 8, cy = (cu / 8) * 8;
-        switch (m) {
-        case 0: return {cx, cy, part_of(8, 8)};
-        case 1: return {cx, cy, part_of(8, 4)};
-        case 2: return {cx, cy + 4, part_of(8, 4)};
-        case 3: return {cx, cy, part_of(4, 8)};
-        case 4: return {cx + 4, cy, part_of(4, 8)};
-        case 5: return {cx, cy, 0};
-        case 6: return {cx + 4, cy, 0};
-        case 7: return {cx, cy + 4, 0};
-        default: return {cx + 4, cy + 4, 0};
-        }
-    }
-    if (s < 784) {
-        int cu = (s - 576) / 13, m = (s - 576) % 13;
-        return cu_mode_geom(16, (cu % 4) * 16, (cu / 4) * 16, m);
-    }
-    if (s < 836) {
-        int cu = (s - 784) / 13, m = (s - 784) % 13;
-        return cu_mode_geom(32, (cu % 2) * 32, (cu / 2) * 32, m);
-    }
-    return cu_mode_geom(64, 0, 0, s - 836);
-}
-
-// (part, ox/4, oy/4) -> slot, -1 if none
-struct SlotTable {
-    int16_t t[kNumParts][16][16];
-    SlotTable()
-    {
-        memset(t, 0xff, sizeof(t));
-        for (int s = 0; s < kSlots; s++) {
-            SlotGeom g = slot_geom(s);
-            t[g.part][g.oy >> 2][g.ox >> 2] = (int16_t)s;
-        }
-    }
 };
 
 // ---- device helpers ------------------------------------------------------------------
@@ -691,7 +619,7 @@ static inline bool same_range_in_window(int lo, int hi, int rule_lo, int rule_hi
 static void ctu_plan_build(CtuPlan &p, const std::vector<xavs2gpu_pu_t> &pus, int W, int H, int nrefs, int R,
                            bool allow, std::vector<int> &generic, cudaStream_t st)
 {
-    static const SlotTable table;
+    const SlotTable &table = slot_table();
     const int cw = (W + 63) / 64, ch = (H + 63) / 64;
     const int ngroups = cw * ch * nrefs;
     std::vector<int> group_job(ngroups, -1);

@@ -47,16 +47,9 @@
 namespace xg {
 
 constexpr int kCuReach = 6;      // pixels between a cluster's first member's centre and the others'
-constexpr int kCuMembers = 13;
 constexpr int kCuOut = 0x3fffffff;   // above any sum of two lambda x bits (lambda < 2^23); twice it fits an int
 constexpr int kCuThreads = 256;
 
-struct CuRec {                   // a CU with PUs in the per-PU search, one reference
-    int16_t x, y;
-    uint8_t lg, ref;             // size 1 << lg
-    uint16_t pad_;
-    int32_t pu[kCuMembers];      // PU of each partition slot (cu_mode_geom's order; 8x8 CUs as slot_geom's), -1 none
-};
 struct CuWork {
     uint32_t cu, mask;           // members (slots) of the cluster
 };

@@ -42,6 +42,8 @@
 // reference is blocky and the best match poor.
 #pragma once
 
+#include "pu_lists.h"
+
 #ifndef XG_PRUNE_SMALL
 #define XG_PRUNE_SMALL 128
 #endif
@@ -61,7 +63,6 @@ namespace xg {
 // and 25 KB of shared memory a CTA at R = 64; with 256 threads the fixed work
 // per thread took 7.7 us of SM time per 4x4 PU against 4.4) and the larger
 // ones.
-constexpr int kSmallDim = 16;
 template <int DIM> struct PruneShape {
     static constexpr int kThreads = DIM <= kSmallDim ? XG_PRUNE_SMALL : XG_PRUNE_LARGE;
     static constexpr int kWarps = kThreads / 32;

@@ -1757,9 +1757,12 @@ extern "C" int xavs2gpu_me_set_pus(xavs2gpu_me_session_t *s, const xavs2gpu_pu_t
             return XAVS2GPU_ERR_ARG;
         }
     }
+    // the CU records depend on the PUs' shapes, places and references alone
+    bool same = n == m.n;
+    for (int i = 0; i < n && same; i++) same = memcmp(&pus[i], &m.h_pus[i], offsetof(xavs2gpu_pu_t, mvp_x)) == 0;
+    m.cu_stale = m.cu_stale || !same;
     m.n = n;
     m.h_pus.assign(pus, pus + n);
-    m.cu_stale = true;
     XG_CUDA(cudaStreamSynchronize(m.st));
     if (n) XG_CUDA(cudaMemcpyAsync(m.d_pus, pus, sizeof(xavs2gpu_pu_t) * n, cudaMemcpyHostToDevice, m.st));
     refresh_view(m);
@@ -1859,15 +1862,7 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     std::vector<int> generic;
     ctu_plan_build(m.plan, m.h_pus, m.W, m.H, m.nrefs, R, ctu, generic, m.st);
     m.n_generic = (int)generic.size();
-    // largest first: by area the PUs with a side above 16, then the others
-    auto side = [&](int i) { return std::max(h_pu_w[m.h_pus[i].part], h_pu_h[m.h_pus[i].part]); };
-    auto pixels = [&](int i) { return h_pu_w[m.h_pus[i].part] * h_pu_h[m.h_pus[i].part]; };
-    const auto small_from = std::stable_partition(generic.begin(), generic.end(),
-                                                  [&](int i) { return side(i) > kSmallDim; });
-    m.n_generic_large = (int)(small_from - generic.begin());
-    auto larger = [&](int a, int b) { return pixels(a) > pixels(b); };
-    std::stable_sort(generic.begin(), small_from, larger);
-    std::stable_sort(small_from, generic.end(), larger);
+    m.n_generic_large = per_pu_order(m.h_pus, generic);
     m.n_ctu_pus = m.n - m.n_generic;
     m.cu_stale = m.cu_stale || !std::equal(generic.begin(), generic.end(), m.h_generic.begin(), m.h_generic.end());
     m.h_generic.assign(generic.begin(), generic.end());
@@ -1928,29 +1923,6 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
 // launches (64 PUs of 16x16 at R = 64 take 8 us on 152 SMs).
 constexpr int kMeansMinPus = 64;
 
-// slot of a PU among the partitions of its CU (side 1 << lg, corner cx, cy),
-// -1 when it is none of them
-static int cu_slot(const xavs2gpu_pu_t &p, int &lg, int &cx, int &cy)
-{
-    const int w = h_pu_w[p.part], h = h_pu_h[p.part], S = std::max(8, std::max(w, h));
-    lg = S == 8 ? 3 : S == 16 ? 4 : S == 32 ? 5 : S == 64 ? 6 : 0;
-    if (!lg) return -1;
-    cx = p.x & ~(S - 1);
-    cy = p.y & ~(S - 1);
-    for (int m = 0; m < (S == 8 ? 9 : 13); m++) {
-        SlotGeom g;
-        if (S == 8) {
-            g = slot_geom(m);   // the CTU's first 8x8 CU
-            g.ox += cx;
-            g.oy += cy;
-        } else {
-            g = cu_mode_geom(S, cx, cy, m);
-        }
-        if (g.part == p.part && g.ox == p.x && g.oy == p.y) return m;
-    }
-    return -1;
-}
-
 // The CU records of the per-PU list and the device memory of their search.
 // Without the memory for it every PU keeps to the per-PU search.
 static void ensure_cu_search(MeSessionImpl &m)
@@ -1962,51 +1934,16 @@ static void ensure_cu_search(MeSessionImpl &m)
     m.cu_list.list = gen;
     m.cu_list.n_large = m.n_generic_large;
     m.cu_list.n_small = m.n_generic - m.n_generic_large;
-    std::vector<CuRec> recs;
-    std::vector<uint32_t> rest;
-    std::vector<int> at[4];          // record of each CU position, per size
-    int n_rec[4] = {0, 0, 0, 0}, rest_large = 0, cap_large = 0, cap_small = 0;
-    for (int k = 0; k < 4; k++)
-        at[k].assign((size_t)m.nrefs * ((m.W >> (3 + k)) + 1) * ((m.H >> (3 + k)) + 1), -1);
-    for (int q = 0; q < m.n_generic; q++) {
-        const int i = (int)m.h_generic[q];
-        const xavs2gpu_pu_t &p = m.h_pus[i];
-        int lg = 0, cx = 0, cy = 0;
-        const int slot = cu_slot(p, lg, cx, cy);
-        bool in = slot >= 0;
-        if (in) {
-            const int k = lg - 3, cols = (m.W >> lg) + 1, rows = (m.H >> lg) + 1;
-            int &r = at[k][((size_t)p.ref * rows + (cy >> lg)) * cols + (cx >> lg)];
-            if (r < 0) {
-                r = (int)recs.size();
-                CuRec c{};
-                c.x = (int16_t)cx;
-                c.y = (int16_t)cy;
-                c.lg = (uint8_t)lg;
-                c.ref = p.ref;
-                for (int &u : c.pu) u = -1;
-                recs.push_back(c);
-                n_rec[k]++;
-            }
-            int32_t &u = recs[r].pu[slot];
-            in = u < 0;              // a second PU of the same partition searches alone
-            if (in) {
-                u = i;
-                (q < m.n_generic_large ? cap_large : cap_small)++;
-            }
-        }
-        if (!in) {
-            rest.push_back((uint32_t)i);
-            rest_large += q < m.n_generic_large ? 1 : 0;
-        }
-    }
+    const CuLists c = cu_lists(m.h_pus, m.h_generic, m.n_generic_large, m.W, m.H, m.nrefs);
+    const std::vector<CuRec> &recs = c.recs;
+    const std::vector<uint32_t> &rest = c.rest;
     if (recs.empty()) return;
     // records | counters | clusters per size (at least two members each) | lone PUs | rest
     size_t need = 0, o_work[4];
     auto take = [&](size_t bytes) { const size_t o = need; need += align_up(bytes); return o; };
     const size_t o_rec = take(sizeof(CuRec) * recs.size()), o_cnt = take(sizeof(int) * kCuCounters);
-    for (int k = 0; k < 4; k++) o_work[k] = take(sizeof(CuWork) * (kCuMembers / 2) * n_rec[k] + 1);
-    const size_t o_large = take(sizeof(uint32_t) * cap_large + 1), o_small = take(sizeof(uint32_t) * cap_small + 1);
+    for (int k = 0; k < 4; k++) o_work[k] = take(sizeof(CuWork) * (kCuMembers / 2) * c.n_rec[k] + 1);
+    const size_t o_large = take(sizeof(uint32_t) * c.cap_large + 1), o_small = take(sizeof(uint32_t) * c.cap_small + 1);
     const size_t o_rest = take(sizeof(uint32_t) * rest.size() + 1);
     if (need > m.cap_cu) {
         cudaFree(m.d_cu);
@@ -2025,12 +1962,12 @@ static void ensure_cu_search(MeSessionImpl &m)
     XG_CUDA(cudaStreamSynchronize(m.st));
     PerPuList &l = m.cu_list;
     l.list = reinterpret_cast<const uint32_t *>(m.d_cu + o_rest);
-    l.n_large = rest_large;
-    l.n_small = (int)rest.size() - rest_large;
+    l.n_large = c.rest_large;
+    l.n_small = (int)rest.size() - c.rest_large;
     l.cus = reinterpret_cast<const CuRec *>(m.d_cu + o_rec);
     l.n_cus = (int)recs.size();
-    l.cap_large = cap_large;
-    l.cap_small = cap_small;
+    l.cap_large = c.cap_large;
+    l.cap_small = c.cap_small;
     l.q.count = reinterpret_cast<int *>(m.d_cu + o_cnt);
     for (int k = 0; k < 4; k++) l.q.work[k] = reinterpret_cast<CuWork *>(m.d_cu + o_work[k]);
     l.q.large = reinterpret_cast<uint32_t *>(m.d_cu + o_large);

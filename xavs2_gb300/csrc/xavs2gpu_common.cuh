@@ -8,21 +8,16 @@
 #include <stddef.h>
 
 #include "../../include/xavs2_gb300.h"
+#include "pu_shapes.h"
 
 namespace xg {
 
-// LumaPU order (pixel.h:50-65 of the reference)
-constexpr int kNumParts = 25;
 // (one copy per translation unit: the library is built without relocatable
 // device code)
 static __constant__ uint8_t c_pu_w[kNumParts] = {4, 8, 16, 32, 64, 8, 4, 16, 8, 32, 16, 64, 32,
                                                  16, 12, 16, 4, 32, 24, 32, 8, 64, 48, 64, 16};
 static __constant__ uint8_t c_pu_h[kNumParts] = {4, 8, 16, 32, 64, 4, 8, 8, 16, 16, 32, 32, 64,
                                                  12, 16, 4, 16, 24, 32, 8, 32, 48, 64, 16, 64};
-static const uint8_t h_pu_w[kNumParts] = {4, 8, 16, 32, 64, 8, 4, 16, 8, 32, 16, 64, 32,
-                                          16, 12, 16, 4, 32, 24, 32, 8, 64, 48, 64, 16};
-static const uint8_t h_pu_h[kNumParts] = {4, 8, 16, 32, 64, 4, 8, 8, 16, 16, 32, 32, 64,
-                                          12, 16, 4, 16, 24, 32, 8, 32, 48, 64, 16, 64};
 
 // ---- error channel ---------------------------------------------------------
 // The reference's primitive signatures have no error return.  Failures are
