@@ -64,6 +64,51 @@ def test_noalloc_matches_session_entry(gpu):
     sess.close()
 
 
+@pytest.mark.parametrize("w,h,R,layout", [(640, 360, 48, "sparse"), (640, 360, 48, "split"), (640, 360, 16, "split"),
+                                          (640, 360, 24, "sparse"), (416, 240, 16, "whole"), (416, 240, 57, "whole"),
+                                          (320, 192, 64, "few")])
+def test_per_pu_routes_match(gpu, w, h, R, layout):
+    """Lists of PUs with their own predictors that a session searches by
+    clusters, bounded, plain or by all three (by how many of a CU's partitions
+    they hold), alone and in a batch: the results of the allocation-free entry,
+    which has the plain search alone."""
+    import torch
+    import xavs2_gb300 as xg
+    import xavs2_gb300.synth as synth
+    lib = xg.load()
+    rng = np.random.default_rng(w + R)
+    f0 = synth.base_picture(rng, w, h)
+    f1 = synth.next_picture(rng, f0, 6, 6)
+    f2 = synth.next_picture(rng, f1, 6, 6)
+    pus = xg.frame_pus(w, h, 2)
+    keep = {"whole": pus["ref"] == 0, "sparse": rng.random(len(pus)) < 0.3, "few": np.arange(len(pus)) < 4000,
+            "split": (pus["x"] < w // 3) | (rng.random(len(pus)) < 0.25)}[layout]
+    pus = pus[keep][:65536].copy()
+    pus["mvp_x"], pus["mvp_y"] = rng.integers(5, 22, len(pus)), rng.integers(-21, -4, len(pus))
+    prm = xg.MeParams(R, oracle.lambda_factor(32), 1, 1, 0, 0)
+    sess = xg.MeSession(w, h, 2, len(pus))
+    for slot, pic in ((-1, f2), (0, f1), (1, f0)):
+        sess.set_picture(slot, pic)
+    sess.set_pus(pus)
+    sess.run(prm)
+    got = sess.results()
+    batch = xg.MeBatch()
+    batch.run([sess], prm, sess.stream())
+    batched = sess.results()
+    batch.close()
+    planes = (ctypes.c_void_p * 32)(*[sess.plane_ptr(r, k) for r in range(2) for k in range(16)])
+    d_pus = torch.from_numpy(pus.view(np.uint8).copy()).cuda()
+    d_out = torch.zeros(len(pus) * xg.RESULT_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    assert _noalloc(lib)(sess.plane_ptr(-1, 0), sess.plane_stride(), w, h, planes, 2, d_pus.data_ptr(), len(pus),
+                         ctypes.byref(prm), d_out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    want = d_out.cpu().numpy().view(xg.RESULT_DTYPE)
+    assert got.tobytes() == want.tobytes()
+    assert batched.tobytes() == want.tobytes()
+    sess.close()
+
+
 def test_noalloc_rejects_oversized_requests(gpu):
     import xavs2_gb300 as xg
     lib = xg.load()

@@ -417,6 +417,13 @@ struct PerPuList {
     const CuRec *cus = nullptr;
     int n_cus = 0, cap_large = 0, cap_small = 0;
     CuQueues q{};
+    bool means() const { return n_large + n_small + n_cus > 0; }
+    void take_bounded(const BoundedPart &b)   // of n_plain PUs
+    {
+        n_large = b.n_large;
+        n_small = b.n_small;
+        n_plain -= n_large + n_small;
+    }
 };
 // ---- 3. sub-pel refinement ------------------------------------------------------------
 // One warp per PU: the candidate costs of one refinement step are evaluated in
@@ -1366,17 +1373,23 @@ static cudaStream_t refine_fork(cudaStream_t st, bool both, CtuSide *&side) { re
 // second side stream, when both have work and phases are not being timed.
 static cudaStream_t search_fork(cudaStream_t st, bool both, CtuSide *&side) { return fork_side(st, both, 1, side); }
 
-// The six searches after the clustering are of disjoint PUs: the 64x64 CUs' and
-// the small PUs' on st, the others' beside them.  One after the other each
-// leaves the GPU idle behind its longest cluster (264x128, R = 48: 237 us for
-// the 64x64 CUs, 280 for the others).
+// All searches of a list are of disjoint PUs and run beside each other on st and
+// a side stream: one after the other each leaves the GPU idle behind its longest
+// PU or cluster (264x128, R = 48: 237 us for the 64x64 CUs, 280 for the others).  The side stream begins with what needs no
+// clustering.
 static int per_pu_launch(const PerPuList &l, const SessView *views, int R, int lambda, cudaStream_t st)
 {
-    int rc = XAVS2GPU_OK;
-    if (l.n_cus) {
+    CtuSide *side = nullptr;
+    const cudaStream_t st2 = fork_side(st, l.n_cus || (l.means() && l.n_plain), 2, side);
+    int rc = prune_launch(l.list, l.n_large, l.n_small, views, R, lambda, st2);
+    if (rc == XAVS2GPU_OK && l.n_plain)
+        rc = fs_generic_launch(l.list + l.n_large + l.n_small, l.n_plain, views, R, lambda, l.n_cus ? st2 : st);
+    if (rc == XAVS2GPU_OK && l.n_cus) {
         cu_cluster_launch(l.q, l.cus, l.n_cus, views, st);
-        CtuSide *side = nullptr;
-        const cudaStream_t st2 = fork_side(st, true, 2, side);
+        if (side) {
+            XG_CUDA(cudaEventRecord(side->fork, st));
+            XG_CUDA(cudaStreamWaitEvent(st2, side->fork, 0));
+        }
         rc = cu_launch_one<64>(l.q, l.cus, views, R, lambda, st);
         if (rc == XAVS2GPU_OK) rc = cu_launch_one<32>(l.q, l.cus, views, R, lambda, st2);
         if (rc == XAVS2GPU_OK) rc = cu_launch_one<16>(l.q, l.cus, views, R, lambda, st2);
@@ -1385,11 +1398,8 @@ static int per_pu_launch(const PerPuList &l, const SessView *views, int R, int l
             rc = prune_launch_one<64>(l.q.large, l.cap_large, l.q.count + 4, views, R, lambda, st2);
         if (rc == XAVS2GPU_OK)
             rc = prune_launch_one<kSmallDim>(l.q.small, l.cap_small, l.q.count + 5, views, R, lambda, st);
-        join_side(st, side);
     }
-    if (rc == XAVS2GPU_OK) rc = prune_launch(l.list, l.n_large, l.n_small, views, R, lambda, st);
-    if (rc == XAVS2GPU_OK && l.n_plain)
-        rc = fs_generic_launch(l.list + l.n_large + l.n_small, l.n_plain, views, R, lambda, st);
+    join_side(st, side);
     return rc;
 }
 
@@ -1433,7 +1443,9 @@ struct MeSessionImpl {
     unsigned long long *d_keys = nullptr;
     PuState *d_state = nullptr;
     int *d_generic = nullptr;
-    int n_generic = 0, n_generic_large = 0;   // those with a side above 16 come first
+    int n_generic = 0;
+    PerPuCounts counts;            // of the per-PU list
+    BoundedPart bounded;           // of the per-PU list where it is searched without clusters
     CtuPlan plan;
     int plan_R = -1;               // search range the plan was built for (-1: stale)
     bool plan_ctu = true;          // whether the plan could use the CTU search
@@ -1463,7 +1475,8 @@ struct MeSessionImpl {
     // search, and the per-PU list of the rest (all in d_cu)
     uint8_t *d_cu = nullptr;
     size_t cap_cu = 0;
-    bool cu_stale = true;            // the per-PU list changed since they were made
+    bool cu_stale = true;            // the per-PU list or the range changed since they were made
+    int cu_R = 0;
     bool per_pu_stale = true;        // they were not looked at since the plan was made
     PerPuList cu_list;
     std::vector<uint32_t> h_generic, h_small, h_large;
@@ -1759,7 +1772,10 @@ extern "C" int xavs2gpu_me_set_pus(xavs2gpu_me_session_t *s, const xavs2gpu_pu_t
     }
     // the CU records depend on the PUs' shapes, places and references alone
     bool same = n == m.n;
-    for (int i = 0; i < n && same; i++) same = memcmp(&pus[i], &m.h_pus[i], offsetof(xavs2gpu_pu_t, mvp_x)) == 0;
+    for (int i = 0; i < n && same; i++) {
+        const xavs2gpu_pu_t &a = pus[i], &b = m.h_pus[i];
+        same = a.x == b.x && a.y == b.y && a.part == b.part && a.ref == b.ref;
+    }
     m.cu_stale = m.cu_stale || !same;
     m.n = n;
     m.h_pus.assign(pus, pus + n);
@@ -1849,6 +1865,8 @@ static void build_groups(MeSessionImpl &m, const std::vector<int> &small, const 
                                 m.st));
 }
 
+static size_t means_bytes(const MeSessionImpl &m) { return m.plane_bytes * m.nrefs + 256; }
+
 // (Re)builds the split into CTU jobs and per-PU searches for window size R.
 // The CTU search keeps (cost << 11 | order) keys in 32 bits, which holds the
 // MV costs of every lambda below 2^26 (the reference's QP range needs below
@@ -1862,9 +1880,11 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     std::vector<int> generic;
     ctu_plan_build(m.plan, m.h_pus, m.W, m.H, m.nrefs, R, ctu, generic, m.st);
     m.n_generic = (int)generic.size();
-    m.n_generic_large = per_pu_order(m.h_pus, generic);
+    m.counts = per_pu_order(m.h_pus, generic);
+    m.bounded = bounded_batch(m.counts, R, means_bytes(m));
     m.n_ctu_pus = m.n - m.n_generic;
-    m.cu_stale = m.cu_stale || !std::equal(generic.begin(), generic.end(), m.h_generic.begin(), m.h_generic.end());
+    m.cu_stale = m.cu_stale || m.cu_R != R || !std::equal(generic.begin(), generic.end(), m.h_generic.begin(), m.h_generic.end());
+    m.cu_R = R;
     m.h_generic.assign(generic.begin(), generic.end());
     if (m.n_generic)
         XG_CUDA(cudaMemcpyAsync(m.d_generic, generic.data(), sizeof(int) * m.n_generic, cudaMemcpyHostToDevice, m.st));
@@ -1917,27 +1937,23 @@ static void ensure_plan(MeSessionImpl &m, int R, int lambda)
     m.per_pu_stale = true;
 }
 
-// Per-PU searches from which a run computes the references' block means (a
-// launch of 3-7 us a plane) and groups CUs (a launch and up to six more for
-// the queues): below it the plain search of that many PUs is shorter than the
-// launches (64 PUs of 16x16 at R = 64 take 8 us on 152 SMs).
-constexpr int kMeansMinPus = 64;
-
 // The CU records of the per-PU list and the device memory of their search.
-// Without the memory for it every PU keeps to the per-PU search.
+// Without the memory for it the list is searched without clusters.
 static void ensure_cu_search(MeSessionImpl &m)
 {
     if (!m.cu_stale) return;
     m.cu_stale = false;
     m.cu_list = PerPuList{};
-    const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
-    m.cu_list.list = gen;
-    m.cu_list.n_large = m.n_generic_large;
-    m.cu_list.n_small = m.n_generic - m.n_generic_large;
-    const CuLists c = cu_lists(m.h_pus, m.h_generic, m.n_generic_large, m.W, m.H, m.nrefs);
+    m.cu_list.list = reinterpret_cast<const uint32_t *>(m.d_generic);
+    m.cu_list.n_plain = m.n_generic;
+    const CuLists c = cu_lists(m.h_pus, m.h_generic, m.counts, m.W, m.H, m.nrefs, m.plan_R, means_bytes(m));
     const std::vector<CuRec> &recs = c.recs;
     const std::vector<uint32_t> &rest = c.rest;
-    if (recs.empty()) return;
+    if (!c.use) return;
+    if (recs.empty()) {
+        m.cu_list.take_bounded(c.bounded);
+        return;
+    }
     // records | counters | clusters per size (at least two members each) | lone PUs | rest
     size_t need = 0, o_work[4];
     auto take = [&](size_t bytes) { const size_t o = need; need += align_up(bytes); return o; };
@@ -1951,6 +1967,7 @@ static void ensure_cu_search(MeSessionImpl &m)
         if (cudaMalloc((void **)&m.d_cu, need) != cudaSuccess) {
             cudaGetLastError();
             m.d_cu = nullptr;
+            m.cu_list.take_bounded(m.bounded);
             return;
         }
         m.cap_cu = need;
@@ -1962,8 +1979,8 @@ static void ensure_cu_search(MeSessionImpl &m)
     XG_CUDA(cudaStreamSynchronize(m.st));
     PerPuList &l = m.cu_list;
     l.list = reinterpret_cast<const uint32_t *>(m.d_cu + o_rest);
-    l.n_large = c.rest_large;
-    l.n_small = (int)rest.size() - c.rest_large;
+    l.n_plain = (int)rest.size();
+    l.take_bounded(c.bounded);
     l.cus = reinterpret_cast<const CuRec *>(m.d_cu + o_rec);
     l.n_cus = (int)recs.size();
     l.cap_large = c.cap_large;
@@ -1972,14 +1989,6 @@ static void ensure_cu_search(MeSessionImpl &m)
     for (int k = 0; k < 4; k++) l.q.work[k] = reinterpret_cast<CuWork *>(m.d_cu + o_work[k]);
     l.q.large = reinterpret_cast<uint32_t *>(m.d_cu + o_large);
     l.q.small = reinterpret_cast<uint32_t *>(m.d_cu + o_small);
-}
-
-static size_t means_bytes(const MeSessionImpl &m) { return m.plane_bytes * m.nrefs + 256; }
-
-// Whether a search of the session's plan with factor lambda uses block means.
-static bool means_wanted(const MeSessionImpl &m, int lambda)
-{
-    return m.n_generic >= kMeansMinPus && prune_ok(lambda);
 }
 
 static bool capturing(const MeSessionImpl &m)
@@ -2001,12 +2010,11 @@ static bool means_alloc(MeSessionImpl &m)
     return true;
 }
 
-// The session's means buffer, where the plan has use for it and the memory is
-// there (without it the per-PU search runs unbounded, with the same results).
-// Never allocated inside a capture, where that is an error.
-static bool ensure_means(MeSessionImpl &m, int lambda)
+// The session's means buffer, where the memory is there (without it the per-PU
+// search runs unbounded, with the same results).  Never allocated inside a
+// capture, where that is an error.
+static bool ensure_means(MeSessionImpl &m)
 {
-    if (!means_wanted(m, lambda)) return false;
     if (!m.d_means && !m.means_owned && !m.means_tried && !capturing(m)) {
         m.means_tried = true;
         means_alloc(m);
@@ -2014,18 +2022,27 @@ static bool ensure_means(MeSessionImpl &m, int lambda)
     return m.d_means != nullptr;
 }
 
-// That, and the CU search of the plan's per-PU list: whether a run takes
-// cu_list.  A run captured before any other of its plan takes the unbounded
-// search.
-static bool ensure_per_pu(MeSessionImpl &m, int lambda)
+// Whether a batched search of the plan bounds some of its per-PU searches.
+static bool batch_bounds(const MeSessionImpl &m, int lambda)
 {
-    if (!ensure_means(m, lambda)) return false;
+    return m.bounded.n_large + m.bounded.n_small > 0 && prune_ok(lambda);
+}
+
+// The per-PU list of a run: with clusters and bounded searches as the plan
+// has use and memory for them, else plain.  A run captured before any other of
+// its plan is plain.
+static PerPuList ensure_per_pu(MeSessionImpl &m, int lambda)
+{
+    PerPuList plain;
+    plain.list = reinterpret_cast<const uint32_t *>(m.d_generic);
+    plain.n_plain = m.n_generic;
+    if (m.n_generic == 0 || !prune_ok(lambda)) return plain;
     if (m.per_pu_stale) {
-        if (capturing(m)) return false;
+        if (capturing(m)) return plain;
         m.per_pu_stale = false;
         ensure_cu_search(m);
     }
-    return true;
+    return m.cu_list.means() && ensure_means(m) ? m.cu_list : plain;
 }
 
 namespace xg {
@@ -2043,7 +2060,7 @@ void me_prepare_batched(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *pr
 }
 int64_t me_means_bytes(xavs2gpu_me_session_t *s, const xavs2gpu_me_params_t *prm)
 {
-    return means_wanted(s->impl, prm->lambda_factor) ? (int64_t)means_bytes(s->impl) : 0;
+    return batch_bounds(s->impl, prm->lambda_factor) ? (int64_t)means_bytes(s->impl) : 0;
 }
 bool me_give_means(xavs2gpu_me_session_t *s) { return s->impl.d_means || means_alloc(s->impl); }
 void me_take_means(xavs2gpu_me_session_t *s)
@@ -2068,16 +2085,14 @@ extern "C" int xavs2gpu_me_run(xavs2gpu_me_session_t *s, const xavs2gpu_me_param
     XG_CUDA(cudaSetDevice(m.device));
     const int R = prm->search_range, lam = prm->lambda_factor;
     ensure_plan(m, R, lam);
-    const bool bounded = ensure_per_pu(m, lam);
+    const PerPuList per_pu = ensure_per_pu(m, lam);
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[0], m.st));
     XG_CUDA(cudaMemsetAsync(m.d_keys, 0xff, sizeof(unsigned long long) * m.n, m.st));
     const uint32_t *gen = reinterpret_cast<const uint32_t *>(m.d_generic);
-    PerPuList per_pu{gen, 0, 0, m.n_generic};
-    if (bounded) per_pu = m.cu_list;
     if (m.n_generic) {
         me_init_list_kernel<<<(m.n_generic * 32 + 127) / 128, 128, 0, m.st>>>(gen, m.n_generic, m.d_view, lam);
         count_launch();
-        if (bounded) mean_planes_run(m.d_view, 1, m.nrefs, m.st);
+        if (per_pu.means()) mean_planes_run(m.d_view, 1, m.nrefs, m.st);
     }
     if (m.profiling) XG_CUDA(cudaEventRecord(m.ev[1], m.st));
     CtuSide *gside = nullptr;
@@ -2433,10 +2448,10 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         nj += m.plan.h_jobs.size();
         nborder += m.plan.n_border;
         ng += m.h_generic.size();
-        if (ensure_means(m, lam)) {
+        if (batch_bounds(m, lam) && ensure_means(m)) {
             max_refs = std::max(max_refs, m.nrefs);
-            ngl += m.n_generic_large;
-            ngs += m.n_generic - m.n_generic_large;
+            ngl += m.bounded.n_large;
+            ngs += m.bounded.n_small;
         }
         ns += g ? m.h_small_g.size() : m.h_small.size();
         nl += g ? m.h_large_g.size() : m.h_large.size();
@@ -2485,13 +2500,12 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         const uint32_t tag = (uint32_t)k << kSessShift;
         V[k] = m.h_view;
         const uint32_t *gen = m.h_generic.data();
-        if (m.d_means && means_wanted(m, lam)) {
-            put_n(Lgl, gen, m.n_generic_large, tag);
-            put_n(Lgs, gen + m.n_generic_large, m.n_generic - m.n_generic_large, tag);
-        } else {
-            V[k].means = nullptr;
-            put_n(Lgp, gen, m.n_generic, tag);
-        }
+        BoundedPart bd;
+        if (batch_bounds(m, lam) && m.d_means) bd = m.bounded;
+        else V[k].means = nullptr;
+        put_n(Lgl, gen, bd.n_large, tag);
+        put_n(Lgs, gen + bd.n_large, bd.n_small, tag);
+        put_n(Lgp, gen + bd.n_large + bd.n_small, m.n_generic - bd.n_large - bd.n_small, tag);
         for (const CtuJob &j0 : m.plan.h_jobs) {
             *J = j0;
             J->sess = (uint8_t)k;
