@@ -143,3 +143,34 @@ def test_cost_batch(gpu, olib):
         exp = [getattr(olib, name)(int(j["part"]), oracle.ptr(base1, int(j["off1"])), 128,
                                    oracle.ptr(base2, int(j["off2"])), 160) for j in jobs]
         assert np.array_equal(got, exp), name
+
+
+@pytest.mark.parametrize("w,h", [(64, 64), (4096, 1), (65, 64), (1, 4097), (300, 211)])
+def test_block_ssd_either_side_of_the_copy(gpu, olib, w, h):
+    """The SSD of any w x h reads the page-locked buffer up to 4096 samples
+    and a device copy beyond."""
+    import xavs2_gb300 as xg
+    rng = np.random.default_rng(w * 7 + h)
+    a, b = (rng.integers(0, 256, (h, w + 5), dtype=np.uint8) for _ in range(2))
+    assert xg.fn("xavs2gpu_get_block_ssd")(xg.ptr(a), w + 5, xg.ptr(b), w + 5, w, h) == \
+        olib.xo_ssd_block(oracle.ptr(a), w + 5, oracle.ptr(b), w + 5, w, h)
+
+
+def _shortest(f, n=300):
+    import time
+    best = 1.0
+    for _ in range(n):
+        t = time.perf_counter()
+        f()
+        best = min(best, time.perf_counter() - t)
+    return best
+
+
+def test_block_ssd_time_grows_with_a_copy(gpu):
+    """A 256x256 SSD is a copy and a sum, not 131,072 single reads over the
+    host link: it takes about 4 times a 64x64 one (8 times read in place)."""
+    import xavs2_gb300 as xg
+    a, b = np.zeros((256, 256), np.uint8), np.ones((256, 256), np.uint8)
+    f = xg.fn("xavs2gpu_get_block_ssd")
+    small, large = (_shortest(lambda: f(xg.ptr(a), 256, xg.ptr(b), 256, n, n)) for n in (64, 256))
+    assert large < 6 * small, (small, large)
