@@ -174,3 +174,15 @@ def test_block_ssd_time_grows_with_a_copy(gpu):
     f = xg.fn("xavs2gpu_get_block_ssd")
     small, large = (_shortest(lambda: f(xg.ptr(a), 256, xg.ptr(b), 256, n, n)) for n in (64, 256))
     assert large < 6 * small, (small, large)
+
+
+def test_sa8d_time_at_odd_addresses(gpu):
+    """The SA8D of a 16x16 block in place: a unit's reads in flight together
+    at any address (odd ones took 1.6 times as long one after the other)."""
+    import xavs2_gb300 as xg
+    if not gpu.xavs2gpu_percall_in_place():
+        pytest.skip("the device does not read pageable host memory")
+    a, b = np.zeros((32, 128), np.uint8), np.ones((32, 128), np.uint8)
+    f = xg.pixel_fn("sa8d", 2)
+    even, odd = (_shortest(lambda: f(xg.ptr(a, o), 128, xg.ptr(b, o), 128)) for o in (0, 3))
+    assert odd < 1.35 * even, (even, odd)
