@@ -186,3 +186,26 @@ def test_sa8d_time_at_odd_addresses(gpu):
     f = xg.pixel_fn("sa8d", 2)
     even, odd = (_shortest(lambda: f(xg.ptr(a, o), 128, xg.ptr(b, o), 128)) for o in (0, 3))
     assert odd < 1.35 * even, (even, odd)
+
+
+def test_sa8d_batch_time(gpu):
+    """A batch of 16x16 SA8D against one of SATD of the same blocks: about 2.6
+    times (5 times and more with a unit's samples read as words)."""
+    import torch
+    import xavs2_gb300 as xg
+    n = 20000
+    rng = np.random.default_rng(3)
+    jobs = np.zeros(n, xg.COST_JOB_DTYPE)
+    jobs["part"], jobs["s1"], jobs["s2"] = 2, 2048, 2240
+    jobs["off1"], jobs["off2"] = (rng.integers(0, (1 << 22) - 16 * 2304, n) for _ in range(2))
+    planes = [torch.randint(0, 256, (1 << 22,), dtype=torch.uint8, device="cuda") for _ in range(2)]
+    d_jobs = torch.from_numpy(jobs.view(np.uint8).copy()).cuda()
+    out = torch.zeros(n, dtype=torch.int32, device="cuda")
+
+    def run(kind):
+        assert xg.fn("xavs2gpu_cost_batch")(kind, d_jobs.data_ptr(), n, planes[0].data_ptr(), planes[1].data_ptr(),
+                                            out.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+
+    satd, sa8d = (_shortest(lambda: run(k), 50) for k in (1, 2))
+    assert sa8d < 4 * satd, (satd, sa8d)

@@ -446,8 +446,8 @@ __device__ int qpel_cost_warp(const xavs2gpu_pu_t &p, int w, int h, bool hadamar
         const int uw = u4 ? 4 : 8, nux = w / uw, nu = nux * (h >> 2);
         for (int u = lane; u < nu; u += 32) {
             int uy = u / nux, ux = u - uy * nux;
-            s += satd_unit_d(u4, o + (ptrdiff_t)uy * 4 * g.stride + ux * uw, g.stride,
-                             r + (ptrdiff_t)uy * 4 * g.stride + ux * uw, g.stride);
+            s += satd_unit_d<false>(u4, o + (ptrdiff_t)uy * 4 * g.stride + ux * uw, g.stride,
+                                    r + (ptrdiff_t)uy * 4 * g.stride + ux * uw, g.stride);
         }
     }
     return warp_sum_i(s);

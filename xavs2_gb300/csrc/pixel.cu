@@ -49,7 +49,8 @@ __device__ __forceinline__ int job_cost_lane(const CostJob &j, int lane)
         const int uw = u4 ? 4 : 8, nux = w / uw, nu = nux * (h >> 2);
         for (int u = lane; u < nu; u += 32) {
             int uy = u / nux, ux = u - uy * nux;
-            s += satd_unit_d(u4, j.p1 + uy * 4 * j.s1 + ux * uw, j.s1, j.p2 + uy * 4 * j.s2 + ux * uw, j.s2);
+            s += satd_unit_d<KIND == 1>(u4, j.p1 + uy * 4 * j.s1 + ux * uw, j.s1, j.p2 + uy * 4 * j.s2 + ux * uw,
+                                        j.s2);
         }
     } else if (kind == 1) {
         const int nux = w >> 3, nu = nux * (h >> 3);

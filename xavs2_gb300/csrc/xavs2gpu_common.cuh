@@ -97,17 +97,6 @@ __device__ __forceinline__ uint32_t ld4_in(const uint8_t *p)
     const uint32_t lo = w[0];
     return a & 3 ? __funnelshift_r(lo, w[1], 8 * (int)(a & 3)) : lo;
 }
-// The same with an aligned word read twice rather than the second behind a
-// branch, which kept a thread's reads from being in flight together: for
-// threads that read a whole unit (16x16 SA8D on host memory, aligned and odd,
-// us: 24.6 and 40.5 with the branch, 21.0 and 22.7; a lane's single words of
-// the 64x64 SAD 34.5 and 30.2, 36.2 and 36.3).
-__device__ __forceinline__ uint32_t ld4_unit(const uint8_t *p)
-{
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    return __funnelshift_r(w[0], w[(a & 3) != 0], 8 * (int)(a & 3));
-}
 // byte k of a minus byte k of b
 __device__ __forceinline__ int byte_diff(uint32_t a, uint32_t b, int k)
 {
@@ -165,14 +154,26 @@ __device__ __forceinline__ int sad_pairs(uint32_t (&d)[4][4])
     return (int)(s & 0xFFFFu) + (int)(s >> 16) - 2 * 16 * 2048;
 }
 
-// sum of |H D H^T| over the 4x4 difference block at (p1, p2)
+// sum of |H D H^T| over the 4x4 difference block at (p1, p2); WORDS: a row of
+// a block as words, for blocks read once (20,000 SATD of 64x64 scattered over a
+// plane 50 us, 85 by bytes); by bytes where a warp's rows come from the cache
+// again and again (60,000 PUs refined at 17 positions 1640 us, 1700 by words)
+template <bool WORDS>
 __device__ __forceinline__ int hsum4_d(const uint8_t *p1, intptr_t s1, const uint8_t *p2, intptr_t s2)
 {
     int m[4][4];
 #pragma unroll
     for (int y = 0; y < 4; y++) {
-        const uint32_t u = ld4_unit(p1 + y * s1), v = ld4_unit(p2 + y * s2);
-        int a = byte_diff(u, v, 0), b = byte_diff(u, v, 1), c = byte_diff(u, v, 2), d = byte_diff(u, v, 3);
+        int v[4];
+        if (WORDS) {
+            const uint32_t q1 = ld4_in(p1 + y * s1), q2 = ld4_in(p2 + y * s2);
+#pragma unroll
+            for (int x = 0; x < 4; x++) v[x] = byte_diff(q1, q2, x);
+        } else {
+#pragma unroll
+            for (int x = 0; x < 4; x++) v[x] = p1[y * s1 + x] - p2[y * s2 + x];
+        }
+        int a = v[0], b = v[1], c = v[2], d = v[3];
         fwht4_d(a, b, c, d);
         m[y][0] = a; m[y][1] = b; m[y][2] = c; m[y][3] = d;
     }
@@ -186,7 +187,9 @@ __device__ __forceinline__ int hsum4_d(const uint8_t *p1, intptr_t s1, const uin
     return s;
 }
 
-// sum of |H8 D H8^T| over one 8x8 difference block
+// sum of |H8 D H8^T| over one 8x8 difference block, by bytes: a lane waits for
+// its own unit, and bytes are all in flight together (20,000 SA8D of 16x16 83 us,
+// 115-143 by words; a 16x16 in host memory at an odd address 23 us, 36-40 by words)
 __device__ __forceinline__ int hsum8_d(const uint8_t *p1, intptr_t s1, const uint8_t *p2, intptr_t s2)
 {
     int m[8][8];
@@ -194,11 +197,7 @@ __device__ __forceinline__ int hsum8_d(const uint8_t *p1, intptr_t s1, const uin
     for (int y = 0; y < 8; y++) {
         int v[8];
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const uint32_t a = ld4_unit(p1 + y * s1 + 4 * q), b = ld4_unit(p2 + y * s2 + 4 * q);
-#pragma unroll
-            for (int x = 0; x < 4; x++) v[4 * q + x] = byte_diff(a, b, x);
-        }
+        for (int x = 0; x < 8; x++) v[x] = p1[y * s1 + x] - p2[y * s2 + x];
         int t[8];
 #pragma unroll
         for (int i = 0; i < 4; i++) { t[i] = v[i] + v[i + 4]; t[i + 4] = v[i] - v[i + 4]; }
@@ -226,10 +225,11 @@ __device__ __forceinline__ int hsum8_d(const uint8_t *p1, intptr_t s1, const uin
 __host__ __device__ __forceinline__ bool satd_unit4(int w, int h) { return w == 4 || (w == 12 && h == 16); }
 
 // Cost of one SATD unit whose top-left corner is (x, y) inside the block.
+template <bool WORDS>
 __device__ __forceinline__ int satd_unit_d(bool u4, const uint8_t *p1, intptr_t s1, const uint8_t *p2, intptr_t s2)
 {
-    if (u4) return hsum4_d(p1, s1, p2, s2) >> 1;
-    return (hsum4_d(p1, s1, p2, s2) + hsum4_d(p1 + 4, s1, p2 + 4, s2)) >> 1;
+    if (u4) return hsum4_d<WORDS>(p1, s1, p2, s2) >> 1;
+    return (hsum4_d<WORDS>(p1, s1, p2, s2) + hsum4_d<WORDS>(p1 + 4, s1, p2 + 4, s2)) >> 1;
 }
 
 // SA8D unit kind for a shape: 0 = alias of SATD, 1 = 8x8 units, 2 = 16x16 units
