@@ -414,14 +414,14 @@ __device__ __forceinline__ void ctu_search(const CtuJob &job, int chunk, int dyw
 #pragma unroll
             for (int b = 0; b < NB; b++) {
                 const int e = min(e0 + b * kCtuThreads, items - 1), r = (e * mq) >> 16, q = e - r * quads;
-                const bool full = ctu_quad_full(q, pitch);   // else the word after is not there to read
+                const int after = ctu_quad_full(q, pitch) ? 16 : 0;   // where there is no word after, any in its place
                 if (from_stage) {
                     v[b] = *reinterpret_cast<const uint4 *>(stage + ctu_stage_at(r, 16 * q));
-                    nx[b] = full ? *reinterpret_cast<const uint32_t *>(stage + ctu_stage_at(r, 16 * q + 16)) : 0u;
+                    nx[b] = *reinterpret_cast<const uint32_t *>(stage + ctu_stage_at(r, 16 * q + after));
                 } else {
                     const uint4 *t = reinterpret_cast<const uint4 *>(ref + (ptrdiff_t)(wy0 + r) * g.stride + wx0) + q;
                     v[b] = __ldg(t);
-                    nx[b] = full ? __ldg(reinterpret_cast<const uint32_t *>(t + 1)) : 0u;
+                    nx[b] = __ldg(reinterpret_cast<const uint32_t *>(t) + after / 4);
                 }
             }
 #pragma unroll
@@ -626,9 +626,10 @@ static void ctu_plan_build(CtuPlan &p, const std::vector<xavs2gpu_pu_t> &pus, in
     std::vector<CtuJob> jobs;
     std::vector<int32_t> slots;
     generic.clear();
-    // the CTU kernel walks a search row in steps of 4 displacements, so it
-    // takes ranges whose 2R is a multiple of 4 (odd R: every PU per-PU)
-    const bool range_ok = allow && (2 * R) % 4 == 0;
+    // the CTU kernel takes even ranges (odd R: every PU per-PU): displacements in
+    // pairs from -R on, an entry each, so that displacement 0 begins one, and
+    // search rows in pairs
+    const bool range_ok = allow && R % 2 == 0;
     for (int i = 0; i < (int)pus.size(); i++) {
         const xavs2gpu_pu_t &u = pus[i];
         const int w = h_pu_w[u.part], h = h_pu_h[u.part];
