@@ -1991,10 +1991,10 @@ static void ensure_cu_search(MeSessionImpl &m)
     l.q.small = reinterpret_cast<uint32_t *>(m.d_cu + o_small);
 }
 
-static bool capturing(const MeSessionImpl &m)
+static bool capturing(cudaStream_t st)
 {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    const bool none = cudaStreamIsCapturing(m.st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+    const bool none = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
     if (!none) cudaGetLastError();
     return !none;
 }
@@ -2011,11 +2011,11 @@ static bool means_alloc(MeSessionImpl &m)
 }
 
 // The session's means buffer, where the memory is there (without it the per-PU
-// search runs unbounded, with the same results).  Never allocated inside a
-// capture, where that is an error.
-static bool ensure_means(MeSessionImpl &m)
+// search runs unbounded, with the same results).  Never allocated while st, the
+// search's stream, is captured, where that is an error.
+static bool ensure_means(MeSessionImpl &m, cudaStream_t st)
 {
-    if (!m.d_means && !m.means_owned && !m.means_tried && !capturing(m)) {
+    if (!m.d_means && !m.means_owned && !m.means_tried && !capturing(st) && !capturing(m.st)) {
         m.means_tried = true;
         means_alloc(m);
     }
@@ -2038,11 +2038,11 @@ static PerPuList ensure_per_pu(MeSessionImpl &m, int lambda)
     plain.n_plain = m.n_generic;
     if (m.n_generic == 0 || !prune_ok(lambda)) return plain;
     if (m.per_pu_stale) {
-        if (capturing(m)) return plain;
+        if (capturing(m.st)) return plain;
         m.per_pu_stale = false;
         ensure_cu_search(m);
     }
-    return m.cu_list.means() && ensure_means(m) ? m.cu_list : plain;
+    return m.cu_list.means() && ensure_means(m, m.st) ? m.cu_list : plain;
 }
 
 namespace xg {
@@ -2448,7 +2448,7 @@ extern "C" int xavs2gpu_me_batch_run(xavs2gpu_me_batch_t *b, xavs2gpu_me_session
         nj += m.plan.h_jobs.size();
         nborder += m.plan.n_border;
         ng += m.h_generic.size();
-        if (batch_bounds(m, lam) && ensure_means(m)) {
+        if (batch_bounds(m, lam) && ensure_means(m, st)) {
             max_refs = std::max(max_refs, m.nrefs);
             ngl += m.bounded.n_large;
             ngs += m.bounded.n_small;
