@@ -164,6 +164,9 @@ def test_server_block_means_memory(gpu):
     def serve(srv, sid):
         for f in frames:
             assert srv.submit(sid, f) == 0
+        return collect(srv)
+
+    def collect(srv):
         got = []
         t0 = time.time()
         while len(got) < len(frames) and time.time() - t0 < 60:
@@ -189,9 +192,12 @@ def test_server_block_means_memory(gpu):
         if name == "even":
             grown["need"] = held
         if name == "two":
+            for f in frames:                      # in flight while the second stream opens
+                assert srv.submit(sid, f) == 0
             assert srv.open_stream(w, h, pus, cus, ring=4) >= 0
             assert srv.stats()["hbm_used"] == budget
-            assert serve(srv, sid)[2] == hashes[2]
+            again = collect(srv)
+            assert again[2] == hashes[2] and len(set(again)) == 3
         srv.close()
     need = grown["need"]
     assert grown["plain"][0] == need and means <= grown["free"][0] - need <= means + 4096

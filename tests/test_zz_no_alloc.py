@@ -70,8 +70,9 @@ def test_noalloc_matches_session_entry(gpu):
 def test_per_pu_routes_match(gpu, w, h, R, layout):
     """Lists of PUs with their own predictors that a session searches by
     clusters, bounded, plain or by all three (by how many of a CU's partitions
-    they hold), alone and in a batch: the results of the allocation-free entry,
-    which has the plain search alone."""
+    they hold), alone, in a batch and captured after a prepare that is the first
+    to see the list: the results of the allocation-free entry, which has the
+    plain search alone."""
     import torch
     import xavs2_gb300 as xg
     import xavs2_gb300.synth as synth
@@ -106,6 +107,25 @@ def test_per_pu_routes_match(gpu, w, h, R, layout):
     want = d_out.cpu().numpy().view(xg.RESULT_DTYPE)
     assert got.tobytes() == want.tobytes()
     assert batched.tobytes() == want.tobytes()
+    sess.set_pus(pus[::-1])
+    stream = torch.cuda.Stream()
+    sess.set_stream(stream.cuda_stream)
+    lib.xavs2gpu_set_abort_on_error(0)
+    try:
+        assert lib.xavs2gpu_me_prepare(ctypes.c_void_p(sess.h), ctypes.byref(prm)) == 0
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream, capture_error_mode="thread_local"):
+            sess.run(prm)
+        assert lib.xavs2gpu_get_status() == 0, lib.xavs2gpu_get_error()
+        with torch.cuda.stream(stream):
+            g.replay()
+            g.replay()
+        captured = sess.results()
+    finally:
+        lib.xavs2gpu_clear_error()
+        lib.xavs2gpu_set_abort_on_error(1)
+    assert captured[::-1].tobytes() == want.tobytes()
+    sess.set_stream(None)
     sess.close()
 
 
